@@ -49,7 +49,9 @@ static TcShape tc_shape(int prec, int norbs) {
   t.ke = 128 / t.esize;
   t.kpad = (norbs + 63) / 64 * 64;
   t.npanels = (t.kpad + 255) / 256;
-  t.pw = ((t.kpad + t.npanels - 1) / t.npanels + 15) / 16 * 16;
+  // whole 32-column blocks: the epilogue reads a panel in blocks of 32 (panels of 208 or 240 columns,
+  // kpad = 704, 832, 960, 1152, lost their last 16)
+  t.pw = ((t.kpad + t.npanels - 1) / t.npanels + 31) / 32 * 32;
   t.nrows_b = t.npanels * t.pw;
   return t;
 }
