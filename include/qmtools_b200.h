@@ -110,15 +110,16 @@ qmt_status qmt_density(qmt_mol* mol, int nx, int ny, int nz, float step,
                        float ox, float oy, float oz, int subgrid, int precision,
                        int rescale, float* qube_dev, double* sum_out, void* stream);
 
-/* Selects the tensor-core density implementation (new; process-wide): 0 = automatic (fused
- * when the contraction is fp16/bf16 and N <= 320, staged otherwise; with the factored density
- * matrix when it has one), 1 = staged (basis values through HBM), 2 = fused (basis values
+/* Selects the tensor-core density implementation (new; process-wide): 0 = automatic (the
+ * factored density matrix when it has one; else fused when the contraction is fp16/bf16 and
+ * N <= 320, staged otherwise), 1 = staged (basis values through HBM), 2 = fused (basis values
  * stay in shared memory), 3 = the factored density matrix: P = L L^T from a pivoted Cholesky
- * factorisation (FP64, on the host, once per matrix) and rho = sum_k (Phi L)_k^2, which needs
- * rank(P) columns instead of N -- for a positive semi-definite P of rank at most min(128, N/2)
- * (an SCF density matrix has the rank of its occupied orbitals), on the fused path when N <= 320
- * and the rank <= 64, else on the staged path (fp16 / bf16); QMT_BAD_ARG when the factorisation
- * finds P indefinite or of higher rank.  What the factor leaves out is checked on
+ * factorisation (FP64, on the host, once per matrix; refined on the device) and
+ * rho = sum_k (Phi L)_k^2, which needs rank(P) columns instead of N -- for a positive
+ * semi-definite P of rank at most min(128, N/2) (an SCF density matrix has the rank of its
+ * occupied orbitals) and fp16 / bf16 contractions; QMT_BAD_ARG when the factorisation finds P
+ * indefinite or of higher rank.  (The automatic choice factors up to min(256, N/2) with fp16x3; bf16
+ * up to rank 64 when N <= 320, else min(128, N/2).)  What the factor leaves out is checked on
  * the device (max |P - L L^T| <= 2e-7 max |P|), which runs the unfactored kernel instead when the
  * check fails, without a host round trip. */
 qmt_status qmt_set_density_path(int mode);
@@ -129,13 +130,12 @@ qmt_status qmt_density_factor_rank(qmt_mol* mol, int* rank_out, void* stream);
 
 /* ---- batches of molecules (new; no reference counterpart) ---------------------------- */
 /* The reference evaluates one molecule per Compute_density call (qmtools/qmtools.py:2381-2430).
- * A batch evaluates the densities of many molecules together: the molecules whose contraction
- * takes the fused path share one persistent launch over all their tiles (one for those with a
- * factored density matrix, one for the others); the rest (N > 320 or tf32) get the staged path,
- * one molecule after another; then each grid is summed and, with rescale, scaled to its nuclear
+ * A batch evaluates the densities of many molecules together: those with a factored density
+ * matrix share one persistent launch over all their tiles, the others with N <= 320 another; the
+ * rest (N > 320 or tf32) get the staged path, one molecule after another; then each grid is summed and, with rescale, scaled to its nuclear
  * charge.  Inputs: shapes[3 i + (0,1,2)] = nx, ny, nz and geoms[4 i + (0,1,2,3)] = step, ox, oy,
  * oz (bohr) of molecule i; qube_devs[i] its grid (device, nx ny nz floats, x-fastest); paths[i]
- * 0 = automatic (fused or staged), 1 = staged, 2 = fused, 3 = fused or staged with the factored
+ * 0 = automatic (fused or staged), 1 = staged, 2 = fused, 3 = with the factored
  * density matrix when it has one that passes its check (as qmt_set_density_path mode 3), else
  * unfactored (NULL: automatic).  A factored molecule's factor is built at creation: refresh != 0
  * is refused for a batch that holds one.
@@ -152,8 +152,8 @@ qmt_status qmt_batch_density(qmt_batch* batch, int rescale, int refresh, void* s
 /* FP64 grid sums before rescaling, sums[nmol] (host); synchronous; reports and clears the kernels'
  * barrier-timeout flags (QMT_CUDA_ERR). */
 qmt_status qmt_batch_sums(qmt_batch* batch, double* sums, void* stream);
-/* Molecules of the batch on the fused launches, and those with a factored density matrix (fused
- * or staged) (-1 for NULL). */
+/* Molecules of the batch that fit the fused kernel (N <= 320, factored or not), and those with a
+ * factored density matrix (-1 for NULL). */
 int qmt_batch_fused_count(const qmt_batch* batch);
 int qmt_batch_factored_count(const qmt_batch* batch);
 qmt_status qmt_batch_destroy(qmt_batch* batch);

@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "density.cuh"
+#include "density_factored.cuh"
 #include "reduce.cuh"
 #include "sm100.cuh"
 
@@ -93,11 +94,9 @@ struct TcParams {
   float* qube;
   double* partials;
   double outscale;
-  const double* gsc;   // device {max, 2^g, 2^-g} of the split density matrix (factored: the
-                       // column scales 2^-2h_k of the squares)
+  const double* gsc;   // device {max, 2^g, 2^-g} of the split density matrix
   int* err;
   uint64_t wait_ns;    // limit of every bounded wait (a test shortens it)
-  int nb;              // factored: rank rounded up to 16 (B holds its hi rows, then its lo rows)
   const int* gate;     // when set, the launch runs only if *gate == gate_want (device-side check
   int gate_want;       // of the factor picks the factored or the unfactored launch)
 };
@@ -169,12 +168,7 @@ __device__ __forceinline__ void load_phi16(const TcParams& p, int64_t row, int c
   }
 }
 
-// FACT: B is the factored density matrix (one box of nb hi rows then nb lo rows per K-chunk, one
-// output panel); per K-step one MMA [A_hi B_hi | A_hi B_lo] into the buffer's first accumulator and
-// one [A_lo B_hi | A_lo B_lo] into its second; the epilogue adds the four column groups and sums
-// the squares with the column scales (no re-read of Phi').  TMEM buffers of 2 x N columns, two of
-// them when they fit in 512.
-template <int FMT, bool FACT>
+template <int FMT>
 __global__ void __launch_bounds__(192, 1)
     density_mma_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
                        const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo,
@@ -245,7 +239,7 @@ __global__ void __launch_bounds__(192, 1)
             if (p.nsplit == 2) tma_load_2d(st + p.a_bytes, &tmA_lo, &full_bar[s], x, t * 128);
             uint8_t* bst = st + p.nsplit * p.a_bytes;
             tma_load_2d(bst, &tmB_hi, &full_bar[s], x, pn * p.pw);
-            if (p.nsplit == 2 && !FACT) tma_load_2d(bst + p.b_bytes, &tmB_lo, &full_bar[s], x, pn * p.pw);
+            if (p.nsplit == 2) tma_load_2d(bst + p.b_bytes, &tmB_lo, &full_bar[s], x, pn * p.pw);
             last_par[s] = (int)ph;
           }
         }
@@ -260,18 +254,15 @@ __global__ void __launch_bounds__(192, 1)
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
       const int ksteps = 128 / (p.esize * (p.esize == 4 ? 8 : 16));  // 4 steps of 32 bytes
-      // factored: N = the factor's hi and lo rows, a buffer holds two accumulators of N
-      const uint32_t nfac = (uint32_t)(p.nsplit * p.nb), fbuf = (uint32_t)p.nsplit * nfac;
-      const uint32_t nbuf = FACT ? (fbuf <= 256u ? 2u : 1u) : 2u;
       for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
         for (int pn = 0; pn < p.npanels && ok; ++pn, ++acc_it) {
-          const uint32_t buf = nbuf == 2u ? (acc_it & 1u) : 0u, aph = ((nbuf == 2u ? acc_it >> 1 : acc_it)) & 1u;
+          const uint32_t buf = acc_it & 1u, aph = (acc_it >> 1) & 1u;
           if (!mbar_wait(&tempty[buf], aph ^ 1u, &abort_flag, p.wait_ns)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d = tmem + buf * (FACT ? 256u * (2u / nbuf) : 256u);
+          const uint32_t d = tmem + buf * 256u;
           for (int kc = 0; kc < p.kchunks; ++kc, ++it) {
             const int s = it % p.stages;
             const uint32_t ph = (it / p.stages) & 1u;
@@ -293,9 +284,6 @@ __global__ void __launch_bounds__(192, 1)
                   mma_tf32(d, sw128_kmajor_desc(a0 + off), sw128_kmajor_desc(b1 + off), p.idesc, 1u);
                   mma_tf32(d, sw128_kmajor_desc(a1 + off), sw128_kmajor_desc(b0 + off), p.idesc, 1u);
                 }
-              } else if (FACT) {
-                mma_f16(d, sw128_kmajor_desc(a0 + off), sw128_kmajor_desc(b0 + off), p.idesc, acc);
-                if (p.nsplit == 2) mma_f16(d + nfac, sw128_kmajor_desc(a1 + off), sw128_kmajor_desc(b0 + off), p.idesc, acc);
               } else {
                 mma_f16(d, sw128_kmajor_desc(a0 + off), sw128_kmajor_desc(b0 + off), p.idesc, acc);
                 if (p.nsplit == 2) {
@@ -320,13 +308,11 @@ __global__ void __launch_bounds__(192, 1)
     const int et = threadIdx.x - 64;
     uint32_t acc_it = 0;
     bool ok = true;
-    const uint32_t nfac = (uint32_t)(p.nsplit * p.nb), fbuf = (uint32_t)p.nsplit * nfac;
-    const uint32_t nbuf = FACT ? (fbuf <= 256u ? 2u : 1u) : 2u;
     for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
       double acc = 0.0;
       const int64_t grow = (int64_t)t * 128 + row;
       for (int pn = 0; pn < p.npanels; ++pn, ++acc_it) {
-        const uint32_t buf = nbuf == 2u ? (acc_it & 1u) : 0u, aph = ((nbuf == 2u ? acc_it >> 1 : acc_it)) & 1u;
+        const uint32_t buf = acc_it & 1u, aph = (acc_it >> 1) & 1u;
         // the four epilogue warps leave together: one of them giving up while the others go on
         // would leave those waiting at the next named barrier
         const bool got = mbar_wait(&tfull[buf], aph, &abort_flag, p.wait_ns);
@@ -335,45 +321,21 @@ __global__ void __launch_bounds__(192, 1)
           break;
         }
         tc_fence_after();
-        if (FACT) {
-          // T_k = the sum of the column groups (hi x hi, hi x lo, lo x hi, lo x lo), then
-          // rho = sum_k 2^-2h_k T_k^2
-          const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + buf * 256u * (2u / nbuf);
-          const int ng = p.nsplit == 2 ? 4 : 1;
-          for (int c = 0; c * 16 < p.nb; ++c) {
-            float tsum[16];
+        for (int c = 0; c < p.pw / 32; ++c) {
+          const int col = pn * p.pw + 32 * c;
+          if (col >= p.kpad) break;
+          float v[32], ph[32];
+          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + buf * 256u + 32u * c, v);
+          if constexpr (FMT == FMT_TF32) load_phi32(p, grow, col, ph);
+          else load_phi16<FMT>(p, grow, col, ph);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) tsum[e] = 0.f;
-            for (int gi = 0; gi < ng; ++gi) {
-              uint32_t tv[16];
-              tmem_ld16_issue(tb + (uint32_t)(gi * p.nb + c * 16), tv);
-              tmem_ld16_wait(tv);
-#pragma unroll
-              for (int e = 0; e < 16; ++e) tsum[e] += __uint_as_float(tv[e]);
-            }
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const double v = (double)tsum[e];
-              acc = fma(__ldg(p.gsc + c * 16 + e) * v, v, acc);
-            }
-          }
-        } else {
-          for (int c = 0; c < p.pw / 32; ++c) {
-            const int col = pn * p.pw + 32 * c;
-            if (col >= p.kpad) break;
-            float v[32], ph[32];
-            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + buf * 256u + 32u * c, v);
-            if constexpr (FMT == FMT_TF32) load_phi32(p, grow, col, ph);
-            else load_phi16<FMT>(p, grow, col, ph);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) acc = fma((double)ph[k], (double)v[k], acc);
-          }
+          for (int k = 0; k < 32; ++k) acc = fma((double)ph[k], (double)v[k], acc);
         }
         tc_fence_before();
         mbar_arrive(&tempty[buf]);
       }
       if (!ok) break;
-      rho_s[row] = FACT ? acc : acc * p.gsc[2];
+      rho_s[row] = acc * p.gsc[2];
       named_barrier(1, 128);
       double mysum = 0.0;
       if (et < p.pm.vpt) {
@@ -506,7 +468,7 @@ __global__ void split_exp_kernel(double* gsc) {
 // Column scales 2^s_j (fs, folded into the producer tables) and 2^-s_j (device, for the split)
 // and the producer tables: they depend on the basis only, so they are built once per molecule.
 static qmt_status ensure_mol_tables(qmt_mol* m, const std::vector<float>& fs, int K, cudaStream_t s);
-static qmt_status ensure_basis_operands(qmt_mol* m, int K, cudaStream_t s) {
+qmt_status ensure_basis_operands(qmt_mol* m, int K, cudaStream_t s) {
   if (m->basis_ops_ready) return QMT_OK;
   const int n = m->norbs;
   std::vector<float> fs(K, 0.f);
@@ -522,7 +484,7 @@ static qmt_status ensure_basis_operands(qmt_mol* m, int K, cudaStream_t s) {
   m->split_inv = inv;
   // pageable uploads return once the data is staged, so `inv` may go
   QMT_CUDA(cudaMemcpyAsync(m->d_split_scale.ptr, inv.data(), K * sizeof(double), cudaMemcpyHostToDevice, s));
-  if ((st = ensure_mol_tables(m, fs, K, s))) return st;
+  if ((st = ensure_mol_tables(m, fs, K, s)) || (st = ensure_unit_tables(m, fs, s))) return st;
   m->basis_ops_ready = true;
   return QMT_OK;
 }
@@ -587,8 +549,7 @@ struct FusedMol {
   int natoms, norbs;
   int n16;                 // functions rounded up to 16: K of the MMAs; the K-steps beyond it
                            // only hold zero padding and are skipped
-  int nb;                  // N of the MMAs (rows of a K-step block of B): n16 for the density
-                           // matrix, the rank rounded up to 16 for its factor
+  int nb;                  // N of the MMAs (rows of a K-step block of U): n16
   int ksteps, nchunks;     // n16 / 16 K-steps; ceil(n16 / 64) column chunks of A
   int tail0;               // n16 & ~63: first column of A's 32-byte swizzled tail blocks
   int u_rows;              // rows of one K-step block of U in HBM (kpad + 64)
@@ -622,19 +583,6 @@ struct FusedParams {
   const int* gate;         // when set, the launch runs only if *gate == gate_want (the device-side
   int gate_want;           // check of the factored matrix picks one of two launches)
 };
-
-// Factored path: a stage holds the factor's hi rows followed by its lo rows, so one MMA of
-// N = 2 nb gives [A_hi B_hi | A_hi B_lo] and, with two pieces, one more [A_lo B_hi | A_lo B_lo].
-// The first kind of the K-steps of the nchunks column chunks goes to fact_nacc(nchunks, nb, two)
-// TMEM accumulators of 2 nb columns (chunk c to accumulator c * na / nchunks), the second kind to
-// one more, and the epilogue adds them.  The accumulators' FP32 additions round with a bias
-// toward zero, which the squares of T would double into rho; few additions of large terms per
-// accumulator keep it small.  Two different accumulators alternate, so no MMA waits on the one
-// before it.
-__host__ __device__ __forceinline__ int fact_nacc(int nchunks, int nb, bool two) {
-  const int fit = 512 / (two ? 2 * nb : nb) - (two ? 1 : 0);
-  return nchunks < fit ? nchunks : fit;
-}
 
 // Arrival count of a column-chunk barrier: each tile pre-arrives CHUNK_COUNT - need, the
 // production items the rest, so that molecules with different atom counts share the barriers.
@@ -733,37 +681,13 @@ __device__ __forceinline__ void unpack8(uint4 a, float* out) {
   }
 }
 
-// Primitive exponentials exp(-alpha q), zero at and beyond the cut-off.  FAST producers (the fused
-// kernel with the factored density matrix) take 2^(-beta q), beta = alpha log2(e) formed once per
-// primitive, with a single ex2.approx in place of the longer expf sequence: Phi' about a sixth
-// faster, at a larger error (fp16x3 density against the FP64 path, relative L2: 4.1e-7 -> 5.4e-7
-// on a 24^3 grid at 0.8 bohr around the 30-atom molecule, 4.2e-7 -> 4.5e-7 on its 128^3 grid at
-// 0.15 bohr).  The unfactored contraction sits nearer its 1e-6 budget (9.7e-7 on the coarse grid)
-// and keeps expf.
-constexpr float kLog2e = 1.44269504f;
-constexpr float kExpCut2 = kExpCut * kLog2e;   // the cut-off in the base-2 scale
-
-template <bool FAST>
-__device__ __forceinline__ float exp_scale(float alpha) {
-  if constexpr (FAST) return alpha * kLog2e;
-  else return alpha;
-}
-
-template <bool FAST>
-__device__ __forceinline__ float exp_cut(float x) {   // x = exp_scale<FAST>(alpha) * q
-  if constexpr (FAST) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-x));
-    return x < kExpCut2 ? r : 0.f;
-  } else {
-    return x < kExpCut ? expf(-x) : 0.f;
-  }
-}
+// Primitive exponentials exp(-alpha q), zero at and beyond the cut-off.
+__device__ __forceinline__ float exp_cut(float x) { return x < kExpCut ? expf(-x) : 0.f; }
 
 // Contracted radial parts sum_k c_k exp(-alpha_k r^2) (zero beyond the cut-off) of NP primitives
 // (alpha, c) at two points, in primitive order.  When the next shell of the atom has the same
 // exponents (pn != nullptr) its radial parts are formed from the same exponentials.
-template <int NP, bool FAST>
+template <int NP>
 __device__ __forceinline__ void radial_np(const float2* pa, const float2* pn, float q0, float q1, float& r0,
                                           float& r1, float& n0, float& n1) {
   float2 ac[NP];
@@ -772,9 +696,9 @@ __device__ __forceinline__ void radial_np(const float2* pa, const float2* pn, fl
   float e0[NP], e1[NP];
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
-    const float b = exp_scale<FAST>(ac[k].x);
-    e0[k] = exp_cut<FAST>(b * q0);
-    e1[k] = exp_cut<FAST>(b * q1);
+    const float b = ac[k].x;
+    e0[k] = exp_cut(b * q0);
+    e1[k] = exp_cut(b * q1);
   }
   r0 = 0.f;
   r1 = 0.f;
@@ -802,7 +726,7 @@ __device__ __forceinline__ void radial_np(const float2* pa, const float2* pn, fl
 // same order as the generic loop, so the values are identical.
 enum { SHAPE_GENERIC = 0, SHAPE_S3S1P1 = 1, SHAPE_S8S8S1P3P1D1 = 2 };
 
-template <int NP, bool FAST>
+template <int NP>
 __device__ __forceinline__ void exps2(const float2* pa, float q0, float q1, float qmin, float (&e0)[NP],
                                       float (&e1)[NP], float (&c)[NP]) {
   float2 ac[NP];
@@ -814,9 +738,9 @@ __device__ __forceinline__ void exps2(const float2* pa, float q0, float q1, floa
     e0[k] = 0.f;
     e1[k] = 0.f;
     if (ac[k].x * qmin < kExpCut) {   // uniform over the warp: qmin is the item's minimum
-      const float b = exp_scale<FAST>(ac[k].x);
-      e0[k] = exp_cut<FAST>(b * q0);
-      e1[k] = exp_cut<FAST>(b * q1);
+      const float b = ac[k].x;
+      e0[k] = exp_cut(b * q0);
+      e1[k] = exp_cut(b * q1);
     }
   }
 }
@@ -965,9 +889,8 @@ struct WindowRowsOut {
 // in `pos`, 1e30 for rows without a point), handed to `out` shell by shell.  Tables as staged
 // by the kernels: shell records, (alpha, scaled coefficient) pairs in descending alpha order,
 // per-atom words (first shell | layout << 24), float nuclear coordinates.  The whole warp works
-// on the atom (lanes r0 = half * 32 + lane); FAST selects the exponentials of exp_cut.  Returns
-// the atom's last function.
-template <bool FAST, class Out>
+// on the atom (lanes r0 = half * 32 + lane).  Returns the atom's last function.
+template <class Out>
 __device__ __forceinline__ int atom_rows(const int4* sh_s, const float2* pr_s, const int* ash_s, const float* crd_s,
                                          int a, const double (*pos)[3], int r0, const Out& out) {
   const int as0 = ash_s[a];
@@ -996,15 +919,15 @@ __device__ __forceinline__ int atom_rows(const int4* sh_s, const float2* pr_s, c
     if (shape == SHAPE_S3S1P1) {
       {
         float e0[3], e1[3], c[3];
-        exps2<3, FAST>(pa, q0, q1, qmin, e0, e1, c);
+        exps2<3>(pa, q0, q1, qmin, e0, e1, c);
         contract2<3>(c, e0, e1, rA0, rA1);
       }
       float rB0, rB1, rC0, rC1;
       {
         float e0[1], e1[1], c[1];
-        exps2<1, FAST>(pa + 3, q0, q1, qmin, e0, e1, c);
+        exps2<1>(pa + 3, q0, q1, qmin, e0, e1, c);
         contract2<1>(c, e0, e1, rB0, rB1);
-        exps2<1, FAST>(pa + 4, q0, q1, qmin, e0, e1, c);
+        exps2<1>(pa + 4, q0, q1, qmin, e0, e1, c);
         contract2<1>(c, e0, e1, rC0, rC1);
       }
       if (!ok0) rA0 = rB0 = rC0 = 0.f;
@@ -1029,7 +952,7 @@ __device__ __forceinline__ int atom_rows(const int4* sh_s, const float2* pr_s, c
       float rB0, rB1;
       {
         float e0[8], e1[8], c[8], d[8];
-        exps2<8, FAST>(pa, q0, q1, qmin, e0, e1, c);
+        exps2<8>(pa, q0, q1, qmin, e0, e1, c);
         contract2<8>(c, e0, e1, rA0, rA1);
 #pragma unroll
         for (int k = 0; k < 8; ++k) d[k] = pa[8 + k].y;   // second s shell: same exponents
@@ -1038,19 +961,19 @@ __device__ __forceinline__ int atom_rows(const int4* sh_s, const float2* pr_s, c
       float rC0, rC1, rD0, rD1, rE0, rE1, rF0, rF1;
       {
         float e0[1], e1[1], c[1];
-        exps2<1, FAST>(pa + 16, q0, q1, qmin, e0, e1, c);
+        exps2<1>(pa + 16, q0, q1, qmin, e0, e1, c);
         contract2<1>(c, e0, e1, rC0, rC1);
       }
       {
         float e0[3], e1[3], c[3];
-        exps2<3, FAST>(pa + 17, q0, q1, qmin, e0, e1, c);
+        exps2<3>(pa + 17, q0, q1, qmin, e0, e1, c);
         contract2<3>(c, e0, e1, rD0, rD1);
       }
       {
         float e0[1], e1[1], c[1];
-        exps2<1, FAST>(pa + 20, q0, q1, qmin, e0, e1, c);
+        exps2<1>(pa + 20, q0, q1, qmin, e0, e1, c);
         contract2<1>(c, e0, e1, rE0, rE1);
-        exps2<1, FAST>(pa + 21, q0, q1, qmin, e0, e1, c);
+        exps2<1>(pa + 21, q0, q1, qmin, e0, e1, c);
         contract2<1>(c, e0, e1, rF0, rF1);
       }
       if (!ok0) rA0 = rB0 = rC0 = rD0 = rE0 = rF0 = 0.f;
@@ -1106,22 +1029,22 @@ __device__ __forceinline__ int atom_rows(const int4* sh_s, const float2* pr_s, c
           rad0 = rad1 = 0.f;
           nx0 = nx1 = 0.f;
           break;
-        case 1: radial_np<1, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 2: radial_np<2, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 3: radial_np<3, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 4: radial_np<4, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 5: radial_np<5, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 6: radial_np<6, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 7: radial_np<7, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
-        case 8: radial_np<8, FAST>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 1: radial_np<1>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 2: radial_np<2>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 3: radial_np<3>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 4: radial_np<4>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 5: radial_np<5>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 6: radial_np<6>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 7: radial_np<7>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
+        case 8: radial_np<8>(pa, pn, q0, q1, rad0, rad1, nx0, nx1); break;
         default:
           rad0 = 0.f;
           rad1 = 0.f;
           for (int k = 0; k < np_ - sk; ++k) {
             const float2 ac = pa[k];
-            const float b = exp_scale<FAST>(ac.x);
-            rad0 = fmaf(ac.y, exp_cut<FAST>(b * q0), rad0);
-            rad1 = fmaf(ac.y, exp_cut<FAST>(b * q1), rad1);
+            const float b = ac.x;
+            rad0 = fmaf(ac.y, exp_cut(b * q0), rad0);
+            rad1 = fmaf(ac.y, exp_cut(b * q1), rad1);
           }
       }
     }
@@ -1161,6 +1084,7 @@ struct StageParams {
   void* out_hi;
   void* out_lo;
   int two;
+  const int* gate;         // when set, the launch runs only if *gate is set
 };
 
 constexpr int STAGE_THREADS = 256;
@@ -1194,6 +1118,7 @@ __device__ __forceinline__ void split_store2(float x0, float x1, void* hi, void*
 template <int FMT>
 __global__ void __launch_bounds__(STAGE_THREADS, 2) basis_window_kernel(const StageParams p) {
   extern __shared__ __align__(16) uint8_t smem_dyn[];
+  if (p.gate && *p.gate == 0) return;
   __shared__ double pos[128][3];
   __shared__ int item_ctr;
   const int lane = threadIdx.x & 31;
@@ -1243,7 +1168,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, 2) basis_window_kernel(const St
         const int a = ar.x + (itm >> 1);
         if ((ash_s[a + 1] & 0xffffff) <= (ash_s[a] & 0xffffff)) continue;
         const int r0 = (itm & 1) * 32 + lane;
-        atom_rows<false>(sh_s, pr_s, ash_s, crd_s, a, pos, r0,
+        atom_rows(sh_s, pr_s, ash_s, crd_s, a, pos, r0,
                   WindowRowsOut{buf + r0 * STAGE_LD, buf + (r0 + 64) * STAGE_LD, c0, pos[r0][0] < 1e29,
                                 pos[r0 + 64][0] < 1e29});
       }
@@ -1380,127 +1305,7 @@ __device__ __forceinline__ void fused_issue_mma(const FusedParams* pp, uint32_t 
   mbar_wait_drain(drain_bar, 0u, 500000000ull);
 }
 
-// Factored path: a stage is one column chunk of the factor, its K-steps each [hi rows | lo rows]
-// (nb rows of 32 bytes apiece), one contiguous copy from HBM (ensure_factor's layout).
-__device__ __forceinline__ uint32_t fact_chunk_ksteps(int c, int ksteps) { return (uint32_t)min(4, ksteps - 4 * c); }
-
-template <bool MULTI>
-__device__ __forceinline__ void fact_produce(const FusedParams& p, uint8_t* stages, uint64_t* full_bar,
-                                             uint64_t* empty_bar, volatile int* abort_flag) {
-  int s = 0;
-  uint32_t ph = 0, issued = 0, par = 0;
-  bool ok = true;
-  for (int64_t t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
-    int m;
-    const FusedMol& M = fused_mol<MULTI>(p, t, m);
-    const int ksteps = M.ksteps, nchunks = M.nchunks;
-    const uint32_t kbytes = (uint32_t)p.nsplit * (uint32_t)M.nb * 32u;   // one K-step of the factor
-    const uint8_t* const src0 = M.u_hi;
-    for (int c = 0; c < nchunks; ++c) {
-      if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, p.wait_ns)) {
-        ok = false;
-        break;
-      }
-      const uint32_t bytes = fact_chunk_ksteps(c, ksteps) * kbytes;
-      mbar_expect_tx(&full_bar[s], bytes);
-      bulk_load(stages + (size_t)s * p.stage_bytes, src0 + (size_t)c * 4 * kbytes, bytes, &full_bar[s]);
-      issued |= 1u << s;
-      par = (par & ~(1u << s)) | (ph << s);
-      if (++s == p.stages) {
-        s = 0;
-        ph ^= 1u;
-      }
-    }
-  }
-  if (!ok)
-    for (int q = 0; q < p.stages; ++q)
-      if ((issued >> q) & 1u) mbar_wait_drain(&full_bar[q], (par >> q) & 1u, 100000000ull);
-}
-
-// Per chunk: wait for its columns of A and its stage, then per K-step one MMA of N = 2 nb
-// [A_hi B_hi | A_hi B_lo] into the chunk's accumulator and, with two pieces, [A_lo B_hi | A_lo B_lo]
-// into the last (fact_nacc); the stage is freed by one commit per chunk.
-template <bool MULTI>
-__device__ __forceinline__ void fact_issue(const FusedParams& p, uint32_t abase, uint32_t lbase, uint8_t* stages,
-                                           uint32_t tmem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* chunk_bar,
-                                           uint64_t* t_full, uint64_t* drain_bar, volatile int* abort_flag) {
-  const bool two = p.nsplit == 2;
-  int s = 0, cur_m = -1;
-  uint32_t ph = 0, cpar = 0;
-  int ksteps = 0, nb = 0, tail0 = 0, nchunks = 0;
-  uint32_t idesc = 0, kbytes = 0, dsmall = 0, firstmask = 0, need = 0;
-  uint32_t dmain[MAX_FUSED_CHUNKS];
-  bool ok = true;
-  for (int64_t t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
-    int m;
-    const FusedMol& M = fused_mol<MULTI>(p, t, m);
-    if (m != cur_m) {   // the molecule's shape of the contraction (once for a single molecule)
-      ksteps = M.ksteps;
-      nb = M.nb;
-      tail0 = M.tail0;
-      nchunks = M.nchunks;
-      const int nfull = two ? 2 * nb : nb;
-      const int na = fact_nacc(nchunks, nb, two);
-      idesc = make_idesc(p.fmt, 128, (uint32_t)nfull);
-      kbytes = (uint32_t)nfull * 32u;
-      dsmall = tmem + (uint32_t)(na * nfull);
-      firstmask = need = 0;
-#pragma unroll
-      for (int c = 0; c < MAX_FUSED_CHUNKS; ++c) {
-        const int a = c < nchunks ? c * na / nchunks : 0;
-        dmain[c] = tmem + (uint32_t)(a * nfull);
-        if (c < nchunks && (c == 0 || (c - 1) * na / nchunks != a)) firstmask |= 1u << c;
-        if (M.chunk_need[c] > 0) need |= 1u << c;
-      }
-      cur_m = m;
-    }
-#pragma unroll 1
-    for (int c = 0; c < nchunks; ++c) {
-      if ((need >> c) & 1u) {
-        if (!mbar_wait(&chunk_bar[c], (cpar >> c) & 1u, abort_flag, p.wait_ns)) {
-          ok = false;
-          break;
-        }
-        cpar ^= 1u << c;
-      }
-      if (!mbar_wait(&full_bar[s], ph, abort_flag, p.wait_ns)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t bst = smem_u32(stages + (size_t)s * p.stage_bytes);
-      const uint32_t kc = fact_chunk_ksteps(c, ksteps);
-      const uint32_t dm = dmain[c];
-      const bool first = (firstmask >> c) & 1u;
-      for (uint32_t kk = 0; kk < kc; ++kk) {
-        const int j0 = (4 * c + (int)kk) * 16;
-        uint64_t ahi, alo;
-        if (j0 < tail0) {
-          const uint32_t aoff = (uint32_t)(c * 16384 + kk * 32);
-          ahi = sw128_kmajor_desc(abase + aoff);
-          alo = sw128_kmajor_desc(lbase + aoff);
-        } else {
-          const uint32_t aoff = (uint32_t)(tail0 * 256 + ((j0 - tail0) >> 4) * 4096);
-          ahi = sw32_kmajor_desc(abase + aoff);
-          alo = sw32_kmajor_desc(lbase + aoff);
-        }
-        const uint64_t bd = sw32_kmajor_desc(bst + kk * kbytes);
-        mma_f16(dm, ahi, bd, idesc, (first && kk == 0) ? 0u : 1u);
-        if (two) mma_f16(dsmall, alo, bd, idesc, (c == 0 && kk == 0) ? 0u : 1u);
-      }
-      tc_commit(&empty_bar[s]);
-      if (++s == p.stages) {
-        s = 0;
-        ph ^= 1u;
-      }
-    }
-    if (ok) tc_commit(t_full);
-  }
-  tc_commit(drain_bar);
-  mbar_wait_drain(drain_bar, 0u, 500000000ull);
-}
-
-template <int FMT, bool MULTI, bool FACT>
+template <int FMT, bool MULTI>
 __global__ void __launch_bounds__(FUSED_THREADS, 1)
     density_fused_kernel(const __grid_constant__ FusedParams p) {
   extern __shared__ uint8_t smem_dyn[];
@@ -1562,14 +1367,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      if (FACT) fact_produce<MULTI>(p, stages, full_bar, empty_bar, &abort_flag);
-      else fused_produce_u<MULTI>(&p, stages, full_bar, empty_bar, &abort_flag);
+      fused_produce_u<MULTI>(&p, stages, full_bar, empty_bar, &abort_flag);
     }
   } else if (warp == 1) {
-    if (lane == 0 && FACT)
-      fact_issue<MULTI>(p, smem_u32(A_hi), smem_u32(A_lo), stages, tmem, full_bar, empty_bar, chunk_bar, &t_full,
-                        &drain_bar, &abort_flag);
-    else if (lane == 0)
+    if (lane == 0)
       fused_issue_mma<MULTI>(&p, smem_u32(A_hi), smem_u32(A_lo), stages, tmem, full_bar, empty_bar, chunk_bar, &t_full,
                       &drain_bar, &abort_flag);
   } else {
@@ -1638,7 +1439,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
         const int a = itm >> 1;
         const int s0 = ash_s[a] & 0xffffff;
         if ((ash_s[a + 1] & 0xffffff) <= s0) continue;
-        const int flast = atom_rows<FACT>(sh_s, pr_s, ash_s, crd_s, a, pos, (itm & 1) * 32 + lane,
+        const int flast = atom_rows(sh_s, pr_s, ash_s, crd_s, a, pos, (itm & 1) * 32 + lane,
                                     SwizzledRowsOut<FMT>{A_hi, A_lo, (itm & 1) * 32 + lane, two, tail0});
         // publish: generic-proxy writes of A become visible to the tensor core, then one arrival
         // per column chunk this atom wrote
@@ -1657,90 +1458,45 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
       tc_fence_after();
       double acc[2] = {0.0, 0.0};
       const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-      if (FACT) {
-        // T = the accumulators' sum (FP32, rounded), rho = sum_k (2^-h_k T_ik)^2 over this warp's
-        // column chunks; M.gsc holds the column scales (layout of ensure_factor)
-        // (each accumulator: nb columns of A_x B_hi, then with two pieces nb of A_x B_lo)
-        const int nb = M.nb, nfull = two ? 2 * nb : nb;
-        const int ngrp = (fact_nacc(M.nchunks, nb, two) + (two ? 1 : 0)) * (two ? 2 : 1);
-        for (int c = hh; c * 16 < nb; c += FUSED_NCW / 4) {
-          float tsum[16];
-#pragma unroll
-          for (int k = 0; k < 16; ++k) tsum[k] = 0.f;
-          for (int gi = 0; gi < ngrp; gi += 2) {   // column group gi: accumulator gi / 2, half gi % 2
-            uint32_t t0[16], t1[16];
-            const uint32_t c0 = (uint32_t)((two ? (gi >> 1) * nfull + (gi & 1) * nb : gi * nb) + c * 16);
-            const uint32_t c1 = (uint32_t)((two ? ((gi + 1) >> 1) * nfull + ((gi + 1) & 1) * nb : (gi + 1) * nb) + c * 16);
-            tmem_ld16_issue(trow + c0, t0);
-            if (gi + 1 < ngrp) tmem_ld16_issue(trow + c1, t1);
-            tmem_ld16_wait(t0);
-            if (gi + 1 < ngrp) {
-              tmem_ld16_wait(t1);
-#pragma unroll
-              for (int k = 0; k < 16; ++k) tsum[k] += __uint_as_float(t0[k]) + __uint_as_float(t1[k]);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) tsum[k] += __uint_as_float(t0[k]);
-            }
-          }
-          // (2^-h_k T_k)^2 with the FP32 scales after the FP64 ones: eight squares per FP32
-          // partial, the partials summed in FP64, as in the unfactored epilogue
-          const float4* hs = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(M.gsc + 2 * nb) + c * 16);
-          float a32[2] = {0.f, 0.f};
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const float4 h4 = __ldg(hs + k4);
-            const float hk[4] = {h4.x, h4.y, h4.z, h4.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float u = tsum[4 * k4 + e] * hk[e];
-              a32[e & 1] = fmaf(u, u, a32[e & 1]);
-            }
-          }
-          acc[0] += (double)a32[0];
-          acc[1] += (double)a32[1];
+      for (int c = hh; c * 16 < n16; c += FUSED_NCW / 4) {
+        const int col = c * 16;
+        // the TMEM load of T' is in flight while the row's Phi' units are read from shared memory
+        uint32_t tv[16];
+        tmem_ld16_issue(trow + (uint32_t)col, tv);
+        float ph[16];
+        // the row's two 16-byte units of columns col .. col + 15 (layout of a_offset)
+        uint32_t rbase, uo[2];
+        if (col < tail0) {
+          const int u0 = (col & 63) >> 3;
+          rbase = (uint32_t)((col >> 6) * 16384 + (row >> 3) * 1024 + (row & 7) * 128);
+          uo[0] = (uint32_t)((u0 ^ (row & 7)) * 16);
+          uo[1] = (uint32_t)(((u0 + 1) ^ (row & 7)) * 16);
+        } else {
+          rbase = (uint32_t)(tail0 * 256 + ((col - tail0) >> 4) * 4096 + row * 32);
+          uo[0] = (uint32_t)(((row >> 2) & 1) << 4);
+          uo[1] = 16u - uo[0];
         }
-      } else {
-        for (int c = hh; c * 16 < n16; c += FUSED_NCW / 4) {
-          const int col = c * 16;
-          // the TMEM load of T' is in flight while the row's Phi' units are read from shared memory
-          uint32_t tv[16];
-          tmem_ld16_issue(trow + (uint32_t)col, tv);
-          float ph[16];
-          // the row's two 16-byte units of columns col .. col + 15 (layout of a_offset)
-          uint32_t rbase, uo[2];
-          if (col < tail0) {
-            const int u0 = (col & 63) >> 3;
-            rbase = (uint32_t)((col >> 6) * 16384 + (row >> 3) * 1024 + (row & 7) * 128);
-            uo[0] = (uint32_t)((u0 ^ (row & 7)) * 16);
-            uo[1] = (uint32_t)(((u0 + 1) ^ (row & 7)) * 16);
-          } else {
-            rbase = (uint32_t)(tail0 * 256 + ((col - tail0) >> 4) * 4096 + row * 32);
-            uo[0] = (uint32_t)(((row >> 2) & 1) << 4);
-            uo[1] = 16u - uo[0];
+        const uint8_t* rb = A_hi + rbase;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) unpack8<FMT>(*reinterpret_cast<const uint4*>(rb + uo[u]), ph + 8 * u);
+        if (two) {
+          const uint8_t* rl = A_lo + rbase;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            float lo8[8];
+            unpack8<FMT>(*reinterpret_cast<const uint4*>(rl + uo[u]), lo8);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ph[8 * u + e] += lo8[e];
           }
-          const uint8_t* rb = A_hi + rbase;
-#pragma unroll
-          for (int u = 0; u < 2; ++u) unpack8<FMT>(*reinterpret_cast<const uint4*>(rb + uo[u]), ph + 8 * u);
-          if (two) {
-            const uint8_t* rl = A_lo + rbase;
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              float lo8[8];
-              unpack8<FMT>(*reinterpret_cast<const uint4*>(rl + uo[u]), lo8);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) ph[8 * u + e] += lo8[e];
-            }
-          }
-          tmem_ld16_wait(tv);
-          // eight products per FP32 partial, partials summed in FP64 (the FP32 partials add
-          // ~3e-8 relative error; converting every product to FP64 ties up the conversion pipe)
-          float a32[2] = {0.f, 0.f};
-#pragma unroll
-          for (int k = 0; k < 16; ++k) a32[k & 1] = fmaf(ph[k], __uint_as_float(tv[k]), a32[k & 1]);
-          acc[0] += (double)a32[0];
-          acc[1] += (double)a32[1];
         }
+        tmem_ld16_wait(tv);
+        // eight products per FP32 partial, partials summed in FP64 (the FP32 partials add
+        // ~3e-8 relative error; converting every product to FP64 ties up the conversion pipe)
+        float a32[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 16; ++k) a32[k & 1] = fmaf(ph[k], __uint_as_float(tv[k]), a32[k & 1]);
+        acc[0] += (double)a32[0];
+        acc[1] += (double)a32[1];
       }
       tc_fence_before();
       rho_part[hh][row] = acc[0] + acc[1];
@@ -1755,7 +1511,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
         }
         int64_t vox, ix, iy, iz;
         if (tile_voxel(M.pm, lt, ct, vox, ix, iy, iz)) {
-          const float qv = (float)(r * (FACT ? 1.0 : M.gsc[2]) * M.outscale);
+          const float qv = (float)(r * M.gsc[2] * M.outscale);
           M.qube[vox] = qv;
           mysum = qv;
         }
@@ -1889,218 +1645,6 @@ static qmt_status ensure_fused_operands(qmt_mol* m, int prec, const TcShape& sh,
   return QMT_OK;
 }
 
-// ---- factored density matrix -----------------------------------------------------------------
-// A density matrix of rank r (r = occupied orbitals for an SCF density, P = 2 C_occ C_occ^T) is
-// P = L L^T with L n x r, and then rho_i = sum_jk Phi_ij P_jk Phi_ik = sum_k (Phi L)_ik^2: the
-// contraction needs N = r columns instead of n.  L comes from a pivoted Cholesky factorisation in
-// FP64 (largest remaining diagonal first), stopped once every remaining diagonal element is at
-// most kFactorTol of the largest one; the factor is used when the matrix it leaves out is at most
-// kFactorResid of max |P| (float32 input rounding is ~6e-8) and the rank is at most half of n.
-// A matrix that is not positive semi-definite, or of high rank, takes the unfactored path.
-// Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds tol; L row i at L[i * ld].
-__global__ void fact_residual_kernel(const double* __restrict__ P, int np, const double* __restrict__ L, int n, int ld,
-                                     int r, double tol, int* bad) {
-  const int64_t tot = (int64_t)n * n;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < tot; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx / n), j = (int)(idx - (int64_t)i * n);
-    if (j > i) continue;
-    double v = P[(size_t)i * np + j];
-    const double* li = L + (size_t)i * ld;
-    const double* lj = L + (size_t)j * ld;
-    for (int q = 0; q < r; ++q) v -= li[q] * lj[q];
-    if (fabs(v) > tol) *bad = 1;
-  }
-}
-
-// The factor's stage layout (ensure_factor): element (j, q), j < n16, q < r16, of W = L_jq 2^-s_j
-// 2^h_q (zero outside j < n, q < r) split into hi + lo (fp16 or bf16, as split_host); K-step block j / 16 holds nsplit x r16 rows
-// of 32 bytes (hi rows, then lo rows), the two 16-byte units of a row exchanged when bit 2 of the
-// row is set.
-__global__ void fact_split_kernel(const double* __restrict__ L, int n, int ld, int r, int n16, int r16,
-                                  const double* __restrict__ inv_s, const double* __restrict__ two_h, int fmt,
-                                  int nsplit, uint8_t* __restrict__ out) {
-  const int64_t tot = (int64_t)n16 * r16;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(i / r16), q = (int)(i - (int64_t)j * r16);
-    const double w = (j < n && q < r) ? L[(size_t)j * ld + q] * inv_s[j] * two_h[q] : 0.0;
-    const int e = j & 15, pe = ((((e >> 3) ^ (q >> 2)) & 1) << 3) | (e & 7);
-    const size_t idx = (size_t)(j >> 4) * nsplit * r16 * 16 + (size_t)q * 16 + pe;
-    uint16_t hi, lo;
-    if (fmt == FMT_F16) {
-      const __half h = __float2half_rn((float)w);
-      hi = __half_as_ushort(h);
-      lo = __half_as_ushort(__float2half_rn((float)(w - (double)__half2float(h))));
-    } else {
-      const __nv_bfloat16 h = __float2bfloat16_rn((float)w);
-      hi = __bfloat16_as_ushort(h);
-      lo = __bfloat16_as_ushort(__float2bfloat16_rn((float)(w - (double)__bfloat162float(h))));
-    }
-    reinterpret_cast<uint16_t*>(out)[idx] = hi;
-    if (nsplit == 2) reinterpret_cast<uint16_t*>(out)[idx + (size_t)r16 * 16] = lo;
-  }
-}
-
-// The factor as the staged path's B operand: row q < r16 holds the hi piece of factor column q,
-// row r16 + q its lo piece (two pieces), each kpad elements of W_jq = L_jq 2^-s_j 2^h_q (zero
-// outside j < n, q < r), row-major; the tensor map gives the 128-byte swizzle.
-__global__ void fact_rows_kernel(const double* __restrict__ L, int n, int ld, int r, int kpad, int r16,
-                                 const double* __restrict__ inv_s, const double* __restrict__ two_h, int fmt,
-                                 int nsplit, uint16_t* __restrict__ out) {
-  const int64_t tot = (int64_t)r16 * kpad;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    const int q = (int)(i / kpad), j = (int)(i - (int64_t)q * kpad);
-    const double w = (j < n && q < r) ? L[(size_t)j * ld + q] * inv_s[j] * two_h[q] : 0.0;
-    uint16_t hi, lo;
-    if (fmt == FMT_F16) {
-      const __half h = __float2half_rn((float)w);
-      hi = __half_as_ushort(h);
-      lo = __half_as_ushort(__float2half_rn((float)(w - (double)__half2float(h))));
-    } else {
-      const __nv_bfloat16 h = __float2bfloat16_rn((float)w);
-      hi = __bfloat16_as_ushort(h);
-      lo = __bfloat16_as_ushort(__float2bfloat16_rn((float)(w - (double)__bfloat162float(h))));
-    }
-    out[(size_t)q * kpad + j] = hi;
-    if (nsplit == 2) out[(size_t)(r16 + q) * kpad + j] = lo;
-  }
-}
-
-constexpr double kFactorTol = 1e-7;
-constexpr double kFactorResid = 2e-7;
-constexpr int kFactorMaxRank = 128;   // N = 2 x 128 per MMA of the staged path's factored kernel
-constexpr int kFusedFactorMaxR16 = 64; // the fused factored kernel: N = 2 x 64, three main accumulators
-
-// The scaled factor W_jk = L_jk 2^(h_k - s_j) (so Phi' W = 2^h_k (Phi L)_k, each column scaled
-// to a maximum near 2^14) split into hi + lo pieces, as the fused kernel streams it: K-step block
-// j / 16 holds the r16 hi rows, then (two pieces) the r16 lo rows, one row per factor column k of
-// 32 bytes (functions j .. j + 15 of that column, the two 16-byte units exchanged when bit 2 of the
-// row is set), so that one MMA of N = 2 r16 takes both and four consecutive blocks are one
-// stage.  The column scales 2^-2h_k of the squares go to d_fact_scale.  Sets fact_rank = 0 when
-// the matrix is not factored.
-static qmt_status ensure_factor(qmt_mol* m, int prec, const TcShape& sh, cudaStream_t s) {
-  if (m->fact_prec == prec) return QMT_OK;
-  qmt_status st;
-  if ((st = ensure_basis_operands(m, sh.kpad, s))) return st;
-  const int n = m->norbs, np = m->npad, n16 = (n + 15) / 16 * 16;
-  m->fact_prec = prec;
-  m->fact_rank = 0;
-  const int rmax = std::min(kFactorMaxRank, n16 / 2);
-  // a density matrix of N_e electrons whose occupations are at most 2 has rank >= N_e / 2: with
-  // the nuclear charge for N_e (ions of up to 16 charges allowed for) a rank above rmax is known
-  // without the factorisation's host work (tens of milliseconds at a thousand functions)
-  if (0.5 * m->qtot > rmax + 8) return QMT_OK;
-  // P_ij from the lower triangle of the matrix as given (no symmetric host copy is built)
-  const float* dm = m->dm_host.data();
-  auto Pij = [&](int i, int j) -> double { return i >= j ? dm[(size_t)i * n + j] : dm[(size_t)j * n + i]; };
-  // the scale of the device check's tolerance: max |P_jk| <= max_j P_jj for a positive
-  // semi-definite P (for any other matrix the check is only the stricter and falls back to the
-  // unfactored one)
-  double dmax = 0.0;
-  for (int j = 0; j < n; ++j) dmax = std::max(dmax, Pij(j, j));
-  const double pmax = dmax;
-  // L row by row (row i at Lr[i * rmax]), so that the dot products run over contiguous memory;
-  // the host buffers are the handle's, reused (no fresh pages per density-matrix change)
-  std::vector<double>& Lr = m->fact_Lr_host;
-  std::vector<double>& d = m->fact_d_host;
-  Lr.assign((size_t)n * rmax, 0.0);
-  d.assign(n, 0.0);
-  for (int j = 0; j < n; ++j) d[j] = Pij(j, j);
-  int r = 0;
-  for (;;) {
-    int jp = 0;
-    for (int j = 1; j < n; ++j)
-      if (d[j] > d[jp]) jp = j;
-    if (!(d[jp] > kFactorTol * dmax)) break;
-    if (r == rmax) return QMT_OK;   // rank too high for the factored path to pay
-    const double piv = std::sqrt(d[jp]), ipiv = 1.0 / piv;
-    const double* lj = Lr.data() + (size_t)jp * rmax;
-    for (int i = 0; i < n; ++i) {
-      const double* li = Lr.data() + (size_t)i * rmax;
-      double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-      int q = 0;
-      for (; q + 4 <= r; q += 4) {
-        a0 += li[q] * lj[q];
-        a1 += li[q + 1] * lj[q + 1];
-        a2 += li[q + 2] * lj[q + 2];
-        a3 += li[q + 3] * lj[q + 3];
-      }
-      for (; q < r; ++q) a0 += li[q] * lj[q];
-      Lr[(size_t)i * rmax + r] = (Pij(i, jp) - ((a0 + a1) + (a2 + a3))) * ipiv;
-    }
-    Lr[(size_t)jp * rmax + r] = piv;
-    for (int i = 0; i < n; ++i) d[i] -= Lr[(size_t)i * rmax + r] * Lr[(size_t)i * rmax + r];
-    d[jp] = 0.0;
-    ++r;
-  }
-  // an indefinite matrix leaves clearly negative diagonal elements behind
-  for (int i = 0; i < n; ++i)
-    if (d[i] < -10.0 * kFactorTol * dmax) return QMT_OK;
-  // what the factor leaves out, max |P - L L^T|, is checked on the device (n^2 r products) into
-  // the gate flag, without a round trip: the factored launch runs when it is 0, the unfactored
-  // one when it is 1 (density_tc)
-  {
-    const size_t lbytes = (size_t)n * rmax * sizeof(double);
-    if ((st = m->d_fact_L.reserve(lbytes + 16))) return st;
-    int* flag = reinterpret_cast<int*>(m->d_fact_L.as<uint8_t>() + lbytes);
-    QMT_CUDA(cudaMemcpyAsync(m->d_fact_L.ptr, Lr.data(), lbytes, cudaMemcpyHostToDevice, s));
-    QMT_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
-    const int64_t tot = (int64_t)n * n;
-    const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
-    fact_residual_kernel<<<std::max(blocks, 1), 256, 0, s>>>(m->d_P64.as<double>(), np, m->d_fact_L.as<double>(), n,
-                                                             rmax, r, kFactorResid * pmax, flag);
-    QMT_CHECK_LAUNCH("fact_residual_kernel");
-    m->fact_gate = flag;
-  }
-  // column scales on the host -- 2^-2h_k (FP64, the staged path's squares), 2^h_k (FP64, the
-  // split), then 2^-h_k (FP32, the fused path's squares (2^-h_k T_k)^2: an exact scaling) -- and
-  // the scaled, split factor in its stage layout on the device
-  const int r16 = std::max(16, (r + 15) / 16 * 16);
-  std::vector<double> sc(2 * r16 + r16 / 2, 0.0);
-  float* scf = reinterpret_cast<float*>(sc.data() + 2 * r16);
-  for (int q = 0; q < r; ++q) {
-    double wmax = 0.0;
-    for (int j = 0; j < n; ++j) wmax = std::max(wmax, std::fabs(Lr[(size_t)j * rmax + q] * m->split_inv[j]));
-    int h = wmax > 0 ? (int)std::floor(std::log2(16000.0 / wmax)) : 0;
-    h = std::max(-100, std::min(100, h));
-    sc[q] = std::ldexp(1.0, -2 * h);
-    sc[r16 + q] = std::ldexp(1.0, h);
-    scf[q] = std::ldexp(1.0f, -h);
-  }
-  const size_t sc_bytes = sc.size() * sizeof(double);
-  const size_t total = (size_t)(n16 / 16) * sh.nsplit * r16 * 32;   // bytes
-  if ((st = m->d_fact_B.reserve(total)) || (st = m->d_fact_scale.reserve(sc_bytes))) return st;
-  QMT_CUDA(cudaMemcpyAsync(m->d_fact_scale.ptr, sc.data(), sc_bytes, cudaMemcpyHostToDevice, s));
-  const int64_t tot = (int64_t)n16 * r16;
-  const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
-  fact_split_kernel<<<std::max(blocks, 1), 256, 0, s>>>(m->d_fact_L.as<double>(), n, rmax, r, n16, r16,
-                                                         m->d_split_scale.as<double>(),
-                                                         m->d_fact_scale.as<double>() + r16, sh.fmt, sh.nsplit,
-                                                         m->d_fact_B.as<uint8_t>());
-  QMT_CHECK_LAUNCH("fact_split_kernel");
-  m->fact_rank = r;
-  m->fact_r16 = r16;
-  m->fact_rows_prec = -1;
-  return QMT_OK;
-}
-
-// The factor in the staged path's B layout (fact_rows_kernel), once per factor.
-static qmt_status ensure_factor_rows(qmt_mol* m, int prec, const TcShape& sh, cudaStream_t s) {
-  if (m->fact_rows_prec == prec) return QMT_OK;
-  const int r16 = m->fact_r16, n16 = (m->norbs + 15) / 16 * 16;
-  const int rmax = std::min(kFactorMaxRank, n16 / 2);
-  qmt_status st = m->d_fact_Bs.reserve((size_t)sh.nsplit * r16 * sh.kpad * 2);
-  if (st) return st;
-  const int64_t tot = (int64_t)r16 * sh.kpad;
-  const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
-  fact_rows_kernel<<<std::max(blocks, 1), 256, 0, s>>>(m->d_fact_L.as<double>(), m->norbs, rmax, m->fact_rank,
-                                                        sh.kpad, r16, m->d_split_scale.as<double>(),
-                                                        m->d_fact_scale.as<double>() + r16, sh.fmt, sh.nsplit,
-                                                        m->d_fact_Bs.as<uint16_t>());
-  QMT_CHECK_LAUNCH("fact_rows_kernel");
-  m->fact_rows_prec = prec;
-  return QMT_OK;
-}
-
 // Shared-memory bytes of the molecule tables staged by the fused kernel.
 static int fused_tab_bytes(const qmt_mol* m) {
   const int words = (int)(m->shells.size() + (m->alpha.size() + 1) / 2);
@@ -2114,30 +1658,27 @@ static uint32_t fused_a_bytes(int n16) { return 128u * (uint32_t)n16 * 2u; }
 static uint32_t fused_b_slot(int nb) { return (uint32_t)nb * 32u; }
 
 // U pipeline stages that fit beside A and the tables (below 2: the fused path does not fit).
-// Bytes of one stage: a K-step of B (nb rows per piece), or four for the factor.
-static long fused_stage_bytes(const TcShape& sh, int nb, bool fact) {
-  return (long)(fact ? 4 : 1) * sh.nsplit * fused_b_slot(nb);
-}
+// Bytes of one stage: a K-step of U (nb rows per piece).
+static long fused_stage_bytes(const TcShape& sh, int nb) { return (long)sh.nsplit * fused_b_slot(nb); }
 
 template <int FMT>
-static int fused_stages(const TcShape& sh, int n16, int nb, int tab_bytes, bool fact = false) {
+static int fused_stages(const TcShape& sh, int n16, int nb, int tab_bytes) {
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, density_fused_kernel<FMT, true, false>) != cudaSuccess) return 0;
-  const long a_bytes = fused_a_bytes(n16), stage_bytes = fused_stage_bytes(sh, nb, fact);
+  if (cudaFuncGetAttributes(&fa, density_fused_kernel<FMT, true>) != cudaSuccess) return 0;
+  const long a_bytes = fused_a_bytes(n16), stage_bytes = fused_stage_bytes(sh, nb);
   const long avail = (long)maxsm - (long)fa.sharedSizeBytes - 1024 - sh.nsplit * a_bytes - tab_bytes;
   return (int)std::max<long>(0, std::min<long>(MAX_STAGES, avail / stage_bytes));
 }
 
-// The descriptor of one molecule in a fused launch, its tiles starting at global tile `tile0`; B
-// is the scaled density matrix, or its factor (`fact`, built by ensure_factor).
+// The descriptor of one molecule in a fused launch, its tiles starting at global tile `tile0`.
 static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int64_t tile0, int64_t ntiles,
-                                 float* qube, double outscale, FusedMol& d, int& tab_bytes, bool fact = false) {
+                                 float* qube, double outscale, FusedMol& d, int& tab_bytes) {
   const int K = sh.kpad, n16 = fused_n16(m);
-  const size_t piece = fact ? 0 : (size_t)(K + 64) * K * 2;   // (the factor's pieces are interleaved)
-  const uint8_t* B = fact ? m->d_fact_B.as<uint8_t>() : m->d_fused_B.as<uint8_t>();
+  const size_t piece = (size_t)(K + 64) * K * 2;
+  const uint8_t* B = m->d_fused_B.as<uint8_t>();
   d = FusedMol{};
   d.pm = pm;
   d.tile0 = tile0;
@@ -2148,8 +1689,8 @@ static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& 
   d.ksteps = n16 / 16;
   d.nchunks = (n16 + 63) / 64;
   d.tail0 = n16 & ~63;
-  d.nb = fact ? m->fact_r16 : n16;
-  d.u_rows = fact ? m->fact_r16 : K + 64;
+  d.nb = n16;
+  d.u_rows = K + 64;
   d.u_hi = B;
   d.u_lo = B + piece;
   if (d.nchunks > MAX_FUSED_CHUNKS) return fail(QMT_BAD_ARG, "fused density path supports kpad <= 320");
@@ -2171,7 +1712,7 @@ static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& 
   d.qube = qube;
   d.partials = m->d_partials.as<double>();
   d.outscale = outscale;
-  d.gsc = fact ? m->d_fact_scale.as<double>() : m->d_gscale.as<double>();
+  d.gsc = m->d_gscale.as<double>();
   return QMT_OK;
 }
 
@@ -2179,16 +1720,15 @@ static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& 
 // p.mols); shared memory is sized for the largest operand, stage and table of the set.
 template <int FMT>
 static qmt_status launch_fused(FusedParams& p, const TcShape& sh_max, int n16_max, int nb_max, int tab_bytes_max,
-                               cudaStream_t s, bool fact = false) {
+                               cudaStream_t s) {
   p.nsplit = sh_max.nsplit;
   p.a_bytes = fused_a_bytes(n16_max);
   p.b_slot = fused_b_slot(nb_max);
-  p.stage_bytes = (uint32_t)fused_stage_bytes(sh_max, nb_max, fact);
+  p.stage_bytes = (uint32_t)fused_stage_bytes(sh_max, nb_max);
   p.fmt = (uint32_t)sh_max.fmt;
   p.wait_ns = wait_limit_ns();
-  auto kern = p.nmol > 1 ? (fact ? density_fused_kernel<FMT, true, true> : density_fused_kernel<FMT, true, false>)
-                         : (fact ? density_fused_kernel<FMT, false, true> : density_fused_kernel<FMT, false, false>);
-  const int stages = fused_stages<FMT>(sh_max, n16_max, nb_max, tab_bytes_max, fact);
+  auto kern = p.nmol > 1 ? density_fused_kernel<FMT, true> : density_fused_kernel<FMT, false>;
+  const int stages = fused_stages<FMT>(sh_max, n16_max, nb_max, tab_bytes_max);
   if (stages < 2) return fail(QMT_BAD_ARG, "fused density tile does not fit in shared memory");
   p.stages = stages;
   const size_t dyn = (size_t)p.nsplit * p.a_bytes + (size_t)stages * p.stage_bytes + tab_bytes_max + 1024;
@@ -2202,18 +1742,17 @@ static qmt_status launch_fused(FusedParams& p, const TcShape& sh_max, int n16_ma
 
 template <int FMT>
 static qmt_status run_fused(qmt_mol* m, const TcShape& sh, const PointMap& pm, int64_t ntiles, float* qube,
-                            double outscale, cudaStream_t s, bool fact = false, const int* gate = nullptr,
-                            int gate_want = 0) {
+                            double outscale, cudaStream_t s, const int* gate = nullptr, int gate_want = 0) {
   FusedParams p{};
   int tab_bytes = 0;
-  qmt_status st = fused_mol_desc(m, sh, pm, 0, ntiles, qube, outscale, p.one, tab_bytes, fact);
+  qmt_status st = fused_mol_desc(m, sh, pm, 0, ntiles, qube, outscale, p.one, tab_bytes);
   if (st) return st;
   p.gate = gate;
   p.gate_want = gate_want;
   p.nmol = 1;
   p.ntiles = ntiles;
   p.err = reinterpret_cast<int*>(m->d_scalars.as<double>() + 8);
-  return launch_fused<FMT>(p, sh, p.one.n16, p.one.nb, tab_bytes, s, fact);
+  return launch_fused<FMT>(p, sh, p.one.n16, p.one.nb, tab_bytes, s);
 }
 
 // Builds the scaled, split density matrix and the Phi column scales for `prec`.
@@ -2234,8 +1773,8 @@ static qmt_status ensure_tc_operands(qmt_mol* m, int prec, const TcShape& sh, cu
 template <int FMT>
 static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int64_t ntiles, int prec,
                          float* qube, double outscale, cudaStream_t s, DevBuf* phi_hi = nullptr,
-                         DevBuf* phi_lo = nullptr, size_t stage_bytes = (size_t)2 << 30, int fact = 0) {
-  // fact: 0 unfactored; 1 factored only; 2 both launches, gated by the device check of the factor
+                         DevBuf* phi_lo = nullptr, size_t stage_bytes = (size_t)2 << 30, const int* gate = nullptr) {
+  // gate: the launches run only if *gate is set (the device check refused the factor)
   qmt_status st;
   if (!phi_hi) {
     phi_hi = &m->d_Phi_hi;
@@ -2251,17 +1790,14 @@ static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int6
   if (sh.nsplit == 2 && (st = phi_lo->reserve(chunk * tile_bytes))) return st;
   void* lo_ptr = sh.nsplit == 2 ? phi_lo->ptr : phi_hi->ptr;
 
-  CUtensorMap tA_hi, tA_lo, tB_hi, tB_lo, tF;
+  CUtensorMap tA_hi, tA_lo, tB_hi, tB_lo;
   const uint8_t* Pb = m->d_tc_P.as<uint8_t>();
   const size_t piece = (size_t)sh.nrows_b * sh.kpad * sh.esize;
   if ((st = make_map(&tA_hi, phi_hi->ptr, sh.esize, sh.kpad, (uint64_t)chunk * 128, sh.ke, 128)) ||
       (st = make_map(&tA_lo, lo_ptr, sh.esize, sh.kpad, (uint64_t)chunk * 128, sh.ke, 128)))
     return st;
-  if (fact != 1 && ((st = make_map(&tB_hi, Pb, sh.esize, sh.kpad, sh.nrows_b, sh.ke, sh.pw)) ||
-                    (st = make_map(&tB_lo, Pb + piece, sh.esize, sh.kpad, sh.nrows_b, sh.ke, sh.pw))))
-    return st;
-  const int nfac = sh.nsplit * m->fact_r16;   // the factored launch's N: hi rows, then lo rows
-  if (fact && (st = make_map(&tF, m->d_fact_Bs.ptr, sh.esize, sh.kpad, (uint64_t)nfac, sh.ke, (uint32_t)nfac)))
+  if ((st = make_map(&tB_hi, Pb, sh.esize, sh.kpad, sh.nrows_b, sh.ke, sh.pw)) ||
+      (st = make_map(&tB_lo, Pb + piece, sh.esize, sh.kpad, sh.nrows_b, sh.ke, sh.pw)))
     return st;
 
   TcParams p{};
@@ -2285,22 +1821,8 @@ static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int6
   p.gsc = m->d_gscale.as<double>();
   p.err = reinterpret_cast<int*>(m->d_scalars.as<double>() + 8);
   p.wait_ns = wait_limit_ns();
-  if (fact == 2) {
-    p.gate = m->fact_gate;
-    p.gate_want = 1;
-  }
-  // the factored launch: one panel of N = nfac (the factor's hi and lo rows in one box)
-  TcParams pf = p;
-  pf.npanels = 1;
-  pf.pw = nfac;
-  pf.b_bytes = (uint32_t)nfac * 128u;
-  pf.stage_bytes = sh.nsplit * pf.a_bytes + pf.b_bytes;
-  pf.tx_bytes = pf.stage_bytes;
-  pf.idesc = make_idesc((uint32_t)sh.fmt, 128, (uint32_t)nfac);
-  pf.gsc = m->d_fact_scale.as<double>();
-  pf.nb = m->fact_r16;
-  pf.gate = fact == 2 ? m->fact_gate : nullptr;
-  pf.gate_want = 0;
+  p.gate = gate;
+  p.gate_want = 1;
 
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
@@ -2310,14 +1832,10 @@ static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int6
     q.stages = std::min((int)((maxsm - static_bytes - 1024) / q.stage_bytes), MAX_STAGES);
     return (size_t)q.stages * q.stage_bytes + 1024;
   };
-  const size_t dyn = plan(p), dynf = plan(pf);
-  if ((fact != 1 && p.stages < 2) || (fact && pf.stages < 2))
-    return fail(QMT_BAD_ARG, "tensor-core stage does not fit in shared memory");
-  constexpr int FF = FMT == FMT_TF32 ? FMT_F16 : FMT;   // (the factored kernel takes fp16 / bf16)
-  auto kern = density_mma_kernel<FMT, false>;
-  auto kernf = density_mma_kernel<FF, true>;
-  if (fact != 1) QMT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  if (fact) QMT_CUDA(cudaFuncSetAttribute(kernf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynf));
+  const size_t dyn = plan(p);
+  if (p.stages < 2) return fail(QMT_BAD_ARG, "tensor-core stage does not fit in shared memory");
+  auto kern = density_mma_kernel<FMT>;
+  QMT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
 
   // staging kernel: molecule tables in shared memory unless they would keep two CTAs off an SM
   const MolTabLayout lay = mol_tab_layout(m, sh.kpad);
@@ -2338,6 +1856,7 @@ static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int6
   sp.out_hi = phi_hi->ptr;
   sp.out_lo = lo_ptr;
   sp.two = sh.nsplit == 2;
+  sp.gate = gate;
   const int buf_bytes = 128 * STAGE_LD * 4;
   if (sp.tab_bytes + buf_bytes > (maxsm - 8192) / 2) sp.tab_bytes = 0;
   const size_t sdyn = (size_t)sp.tab_bytes + buf_bytes;
@@ -2354,23 +1873,28 @@ static qmt_status run_tc(qmt_mol* m, const TcShape& sh, const PointMap& pm, int6
     const int gb = (int)std::min<int64_t>(nt, (int64_t)nsm * stage_ctas);
     skern<<<gb, STAGE_THREADS, sdyn, s>>>(sp);
     QMT_CHECK_LAUNCH("basis_window_kernel");
-    p.tile0 = pf.tile0 = t0;
-    p.ntiles = pf.ntiles = nt;
+    p.tile0 = t0;
+    p.ntiles = nt;
     const int gm = (int)std::min<int64_t>(nt, nsm);
-    if (fact) {
-      kernf<<<gm, 192, dynf, s>>>(tA_hi, tA_lo, tF, tF, pf);
-      QMT_CHECK_LAUNCH("density_mma_kernel");
-    }
-    if (fact != 1) {
-      kern<<<gm, 192, dyn, s>>>(tA_hi, tA_lo, tB_hi, tB_lo, p);
-      QMT_CHECK_LAUNCH("density_mma_kernel");
-    }
+    kern<<<gm, 192, dyn, s>>>(tA_hi, tA_lo, tB_hi, tB_lo, p);
+    QMT_CHECK_LAUNCH("density_mma_kernel");
   }
   (void)prec;
   return QMT_OK;
 }
 
-static int g_density_path = 0;   // 0 auto, 1 staged, 2 fused, 3 fused with the factored matrix
+static int g_density_path = 0;   // 0 auto, 1 staged, 2 fused, 3 the factored matrix
+
+// Whether the molecule's contraction takes its factor: with fp16x3 whenever there is one (rank <= 256,
+// N / 2: the factored kernel needs 3 x rank MMA columns per K-step where the others need 3 x N and a row
+// dot; N = 1176, rank 238: 6.3 against 42.9 ms).  bf16 keeps the ranks that it was factored for before
+// (64 beside the fused kernel, 128 beyond it): its pieces carry 16 bits, so another operand split
+// would move its results by as much as their error (1e-5).
+constexpr int kFactorAskedRank = 128;    // path 3 asked for by name: at most this rank
+constexpr int kBf16FusedMaxR16 = 64;
+static bool takes_factor(const qmt_mol* m, const TcShape& sh, bool fused) {
+  return m->fact_rank > 0 && (sh.fmt == FMT_F16 || !fused || m->fact_r16 <= kBf16FusedMaxR16);
+}
 
 // The fused path takes fp16/bf16 contractions of up to 320 functions whose tile, stages and tables
 // fit in shared memory.
@@ -2395,35 +1919,34 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   const bool fused = g_density_path == 1 ? false : fusable;
   if (g_density_path == 2 && !fusable)
     return fail(QMT_BAD_ARG, "fused density path needs fp16/bf16, N <= 320 and molecule tables that fit in shared memory");
-  // the factored matrix when there is one (automatic, or asked for): fused (rank <= 64) or staged
-  // (rank <= 128, fp16 / bf16)
+  // the factored matrix when there is one (automatic, or asked for)
   bool fact = false;
   if (sh.fmt != FMT_TF32 && g_density_path != 1 && g_density_path != 2) {
-    if ((st = ensure_factor(mol, precision, sh, s))) return st;
-    fact = mol->fact_rank > 0 && (!fused || mol->fact_r16 <= kFusedFactorMaxR16);
-    if (g_density_path == 3 && !fact)
+    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, s))) return st;
+    fact = takes_factor(mol, sh, fused);
+    if (g_density_path == 3 && (!fact || mol->fact_rank > kFactorAskedRank))
       return fail(QMT_BAD_ARG, "factored density path needs a positive semi-definite density matrix of low rank");
   }
+  // with a factor, the device check of what it leaves out picks the launch (no host round trip)
+  const int* gate = fact ? mol->fact_gate : nullptr;
+  if (fact) {
+    FactMol d;
+    fact_mol_desc(mol, pm, 0, ntiles, qube, outscale, d);
+    if ((st = launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit,
+                              reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), gate, 0, s)))
+      return st;
+  }
   if (fused) {
-    // with a factor, the device check of what it leaves out picks the launch (no host round trip)
     if ((st = ensure_fused_operands(mol, precision, sh, s))) return st;
-    const int* gate = fact ? mol->fact_gate : nullptr;
-    if (sh.fmt == FMT_F16) {
-      if (fact) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, true, gate, 0);
-      if (!st) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, false, gate, 1);
-    } else {
-      if (fact) st = run_fused<FMT_BF16>(mol, sh, pm, ntiles, qube, outscale, s, true, gate, 0);
-      if (!st) st = run_fused<FMT_BF16>(mol, sh, pm, ntiles, qube, outscale, s, false, gate, 1);
-    }
+    if (sh.fmt == FMT_F16) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
+    else st = run_fused<FMT_BF16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
   } else {
     if ((st = ensure_tc_operands(mol, precision, sh, s))) return st;
-    if (fact && (st = ensure_factor_rows(mol, precision, sh, s))) return st;
-    const int fmode = fact ? 2 : 0;   // with a factor, the device check picks the launch
     if (sh.fmt == FMT_TF32) st = run_tc<FMT_TF32>(mol, sh, pm, ntiles, precision, qube, outscale, s);
     else if (sh.fmt == FMT_F16)
-      st = run_tc<FMT_F16>(mol, sh, pm, ntiles, precision, qube, outscale, s, nullptr, nullptr, (size_t)2 << 30, fmode);
+      st = run_tc<FMT_F16>(mol, sh, pm, ntiles, precision, qube, outscale, s, nullptr, nullptr, (size_t)2 << 30, gate);
     else
-      st = run_tc<FMT_BF16>(mol, sh, pm, ntiles, precision, qube, outscale, s, nullptr, nullptr, (size_t)2 << 30, fmode);
+      st = run_tc<FMT_BF16>(mol, sh, pm, ntiles, precision, qube, outscale, s, nullptr, nullptr, (size_t)2 << 30, gate);
   }
   if (st) return st;
   st = finish_density(mol, pm.nvox, ntiles, rescale, qube, sum_out, s);
@@ -2455,8 +1978,8 @@ struct BatchItem {
   int64_t ntiles;
   float* qube;
   double outscale;
-  bool fused;
-  bool fact;   // fused, with the factored density matrix
+  bool fused;  // N <= 320: the fused kernel takes it
+  bool fact;   // on the factored launch
 };
 
 }  // namespace qmt
@@ -2473,7 +1996,11 @@ struct qmt_batch_group {
 struct qmt_batch {
   int precision = 0, fmt = 0;
   std::vector<qmt::BatchItem> items;
-  qmt_batch_group fused, fact;        // unfactored and factored fused launches
+  qmt_batch_group fused;              // the unfactored fused launch
+  std::vector<qmt::FactMol> fact;     // the factored launch's molecules
+  int64_t fact_tiles = 0;
+  int nsplit = 2;
+  qmt::DevBuf d_fact;
   qmt::DevBuf d_err;
   qmt::DevBuf phi_hi, phi_lo;         // staged-path basis values, shared by the batch's molecules
 };
@@ -2485,7 +2012,7 @@ namespace qmt {
 static qmt_status batch_operands(const BatchItem& it, int prec, bool refresh, cudaStream_t s) {
   if (it.fact) {
     if (refresh) return fail(QMT_BAD_ARG, "a batch with factored molecules cannot re-derive their operands");
-    return it.fused ? QMT_OK : ensure_factor_rows(it.mol, prec, it.sh, s);
+    return QMT_OK;
   }
   if (refresh) {
     it.mol->fused_prec = -1;
@@ -2494,9 +2021,9 @@ static qmt_status batch_operands(const BatchItem& it, int prec, bool refresh, cu
   return it.fused ? ensure_fused_operands(it.mol, prec, it.sh, s) : ensure_tc_operands(it.mol, prec, it.sh, s);
 }
 
-// Descriptors of the fused molecules of one kind (factored or not) and the shared-memory plan of
-// their launch; `stages` < 2 when the plan does not fit, `largest` the molecule to move out then.
-static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, bool fact, int& stages, int& largest) {
+// Descriptors of the unfactored fused molecules and the shared-memory plan of their launch; `stages`
+// < 2 when the plan does not fit, `largest` the molecule to move out then.
+static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, int& stages, int& largest) {
   g.fdesc.clear();
   g.sh_max = TcShape{};
   g.n16_max = g.nb_max = g.tab_bytes_max = 0;
@@ -2505,10 +2032,10 @@ static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, bool fact, int& 
   stages = MAX_STAGES;
   for (size_t i = 0; i < b->items.size(); ++i) {
     BatchItem& it = b->items[i];
-    if (!it.fused || it.fact != fact) continue;
+    if (!it.fused || it.fact) continue;
     FusedMol d;
     int tb = 0;
-    qmt_status st = fused_mol_desc(it.mol, it.sh, it.pm, g.tiles, it.ntiles, it.qube, it.outscale, d, tb, fact);
+    qmt_status st = fused_mol_desc(it.mol, it.sh, it.pm, g.tiles, it.ntiles, it.qube, it.outscale, d, tb);
     if (st) return st;
     g.tiles += it.ntiles;
     g.fdesc.push_back(d);
@@ -2520,13 +2047,13 @@ static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, bool fact, int& 
       largest = (int)i;
   }
   if (!g.fdesc.empty())
-    stages = b->fmt == FMT_F16 ? fused_stages<FMT_F16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max, fact)
-                               : fused_stages<FMT_BF16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max, fact);
+    stages = b->fmt == FMT_F16 ? fused_stages<FMT_F16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max)
+                               : fused_stages<FMT_BF16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max);
   return QMT_OK;
 }
 
 template <int FMT>
-static qmt_status batch_launch(qmt_batch* b, const qmt_batch_group& g, bool fact, cudaStream_t s) {
+static qmt_status batch_launch(qmt_batch* b, const qmt_batch_group& g, cudaStream_t s) {
   if (g.fdesc.empty()) return QMT_OK;
   FusedParams p{};
   p.nmol = (int)g.fdesc.size();
@@ -2534,7 +2061,7 @@ static qmt_status batch_launch(qmt_batch* b, const qmt_batch_group& g, bool fact
   p.mols = g.d_fdesc.as<FusedMol>();
   p.ntiles = g.tiles;
   p.err = b->d_err.as<int>();
-  return launch_fused<FMT>(p, g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max, s, fact);
+  return launch_fused<FMT>(p, g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max, s);
 }
 
 template <int FMT>
@@ -2544,11 +2071,15 @@ static qmt_status batch_run(qmt_batch* b, int rescale, bool refresh, cudaStream_
     if ((st = batch_operands(it, b->precision, refresh, s))) return st;
   if (FMT != FMT_TF32) {
     constexpr int F = FMT == FMT_TF32 ? FMT_F16 : FMT;
-    if ((st = batch_launch<F>(b, b->fact, true, s)) || (st = batch_launch<F>(b, b->fused, false, s))) return st;
+    if (!b->fact.empty() &&
+        (st = launch_factored(b->fact.data(), b->d_fact.as<FactMol>(), (int)b->fact.size(), b->fact_tiles, F, b->nsplit,
+                              b->d_err.as<int>(), nullptr, 0, s)))
+      return st;
+    if ((st = batch_launch<F>(b, b->fused, s))) return st;
   }
   for (const BatchItem& it : b->items)
-    if (!it.fused && (st = run_tc<FMT>(it.mol, it.sh, it.pm, it.ntiles, b->precision, it.qube, it.outscale, s,
-                                       &b->phi_hi, &b->phi_lo, BATCH_STAGE_BYTES, it.fact ? 1 : 0)))
+    if (!it.fused && !it.fact && (st = run_tc<FMT>(it.mol, it.sh, it.pm, it.ntiles, b->precision, it.qube, it.outscale, s,
+                                       &b->phi_hi, &b->phi_lo, BATCH_STAGE_BYTES)))
       return st;
   for (const BatchItem& it : b->items)
     if ((st = finish_density(it.mol, it.pm.nvox, it.ntiles, rescale, it.qube, nullptr, s))) return st;
@@ -2602,7 +2133,7 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
     it.fact = false;
     if (path == 3 && it.sh.fmt != FMT_TF32) {   // factored when the matrix has a factor that passes the check
       int gate = 1;
-      if ((st = ensure_factor(m, precision, it.sh, s))) break;
+      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, s))) break;
       if (m->fact_rank > 0) {
         const cudaError_t e1 = cudaMemcpyAsync(&gate, m->fact_gate, sizeof(int), cudaMemcpyDeviceToHost, s);
         const cudaError_t e2 = cudaStreamSynchronize(s);
@@ -2611,7 +2142,7 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
           break;
         }
       }
-      it.fact = m->fact_rank > 0 && gate == 0 && (!it.fused || m->fact_r16 <= kFusedFactorMaxR16);
+      it.fact = gate == 0 && takes_factor(m, it.sh, it.fused);
     }
     if ((st = m->d_partials.reserve(it.ntiles * sizeof(double))) || (st = m->d_scalars.reserve(64 * sizeof(double))))
       break;
@@ -2619,28 +2150,32 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
     b->items.push_back(it);
   }
   b->fmt = tc_shape(precision, 1).fmt;
-  // fused molecules of each kind: one launch sized for the largest of them; drop the largest to
+  b->nsplit = tc_shape(precision, 1).nsplit;
+  // the unfactored fused molecules: one launch sized for the largest of them; drop the largest to
   // the staged path until the shared-memory plan of the set fits
-  for (int kind = 0; kind < 2 && !st; ++kind) {
-    qmt_batch_group& g = kind ? b->fact : b->fused;
-    for (;;) {
-      int stg = 0, largest = -1;
-      if ((st = batch_group(b, g, kind == 1, stg, largest))) break;
-      if (g.fdesc.empty() || stg >= 2) break;
-      b->items[largest].fused = false;   // (a factored molecule stays factored on the staged path)
-      if ((st = batch_operands(b->items[largest], precision, false, s))) break;
-    }
+  while (!st) {
+    int stg = 0, largest = -1;
+    if ((st = batch_group(b, b->fused, stg, largest)) || b->fused.fdesc.empty() || stg >= 2) break;
+    b->items[largest].fused = false;
+    st = batch_operands(b->items[largest], precision, false, s);
+  }
+  // the factored molecules: one launch over all their tiles
+  for (const BatchItem& it : b->items) {
+    if (!it.fact) continue;
+    FactMol d;
+    fact_mol_desc(it.mol, it.pm, b->fact_tiles, it.ntiles, it.qube, it.outscale, d);
+    b->fact_tiles += it.ntiles;
+    b->fact.push_back(d);
   }
   if (!st) st = b->d_err.reserve(256);
-  for (qmt_batch_group* g : {&b->fused, &b->fact}) {
-    if (st || g->fdesc.empty()) continue;
-    const size_t bytes = g->fdesc.size() * sizeof(FusedMol);
-    st = g->d_fdesc.reserve(bytes);
-    if (!st) {
-      const cudaError_t e1 = cudaMemcpyAsync(g->d_fdesc.ptr, g->fdesc.data(), bytes, cudaMemcpyHostToDevice, s);
-      if (e1 != cudaSuccess) st = cuda_fail(e1, "batch descriptors");
-    }
-  }
+  auto upload = [&](DevBuf& buf, const void* src, size_t bytes) {
+    if (st || !bytes) return;
+    if ((st = buf.reserve(bytes))) return;
+    const cudaError_t e1 = cudaMemcpyAsync(buf.ptr, src, bytes, cudaMemcpyHostToDevice, s);
+    if (e1 != cudaSuccess) st = cuda_fail(e1, "batch descriptors");
+  };
+  upload(b->fused.d_fdesc, b->fused.fdesc.data(), b->fused.fdesc.size() * sizeof(FusedMol));
+  upload(b->d_fact, b->fact.data(), b->fact.size() * sizeof(FactMol));
   if (!st) {
     const cudaError_t e2 = cudaMemsetAsync(b->d_err.ptr, 0, 256, s);
     const cudaError_t e3 = cudaStreamSynchronize(s);
@@ -2692,7 +2227,9 @@ qmt_status qmt_batch_sums(qmt_batch* b, double* sums, void* stream) {
 
 int qmt_batch_fused_count(const qmt_batch* b) {
   if (!b) return -1;
-  return (int)(b->fused.fdesc.size() + b->fact.fdesc.size());
+  int n = 0;
+  for (const BatchItem& it : b->items) n += it.fused ? 1 : 0;
+  return n;
 }
 
 int qmt_batch_factored_count(const qmt_batch* b) {
@@ -2706,7 +2243,7 @@ qmt_status qmt_batch_destroy(qmt_batch* b) {
   if (!b) return QMT_OK;
   cudaDeviceSynchronize();
   b->fused.d_fdesc.release();
-  b->fact.d_fdesc.release();
+  b->d_fact.release();
   b->d_err.release();
   b->phi_hi.release();
   b->phi_lo.release();

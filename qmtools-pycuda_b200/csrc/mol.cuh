@@ -49,13 +49,15 @@ struct qmt_mol {
   int fact_prec = -1;           // precision of the factored-path operands below (-1: not built)
   int fact_rank = 0;            // rank of the density-matrix factor P = L L^T (0: not factored)
   std::vector<double> fact_Lr_host, fact_d_host;   // host work buffers of the factorisation
+  std::vector<float> fact_L0_host;
   int fact_r16 = 0;             // the rank rounded up to 16 (the MMA N)
-  qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of fact_r16 rows (hi then lo)
-  qmt::DevBuf d_fact_L;         // the factor (FP64, row by row) and a flag, for the residual check
-  int fact_rows_prec = -1;      // precision of d_fact_Bs (-1: not built for the current factor)
-  qmt::DevBuf d_fact_Bs;        // the factor as the staged path's B operand (fact_rows_kernel)
+  qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of fact_r16 rows a piece
+  qmt::DevBuf d_fact_tab;       // unit and class tables, then the function of each column
+  int fact_units = 0;           // units of 16 columns
+  size_t fact_col_off = 0;      // byte offset of the column table
+  qmt::DevBuf d_fact_L;         // the factor (FP64, row by row), scratch of its refinement, the flag of the residual check
   const int* fact_gate = nullptr; // that flag: 0 when the factor reproduces P, 1 when it does not
-  qmt::DevBuf d_fact_scale;     // per factor column k: 2^-2h_k, 2^h_k (FP64), then 2^-h_k (FP32)
+  qmt::DevBuf d_fact_scale;     // per factor column k: 2^h_k (FP64), then 2^-h_k (FP32)
   qmt::DevBuf d_fused_tab;      // fused path: packed shell records, then (alpha, scaled coefficient) pairs
   qmt::DevBuf d_coords, d_types, d_shells, d_alpha, d_coeff, d_alpha64, d_coeff64;
   qmt::DevBuf d_P32, d_P64;

@@ -83,18 +83,65 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     *abort_flag = 1;
     return false;
   }
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  // the clock is read only after 64 polls: reading it costs more than a short wait
+  uint64_t t0 = 0;
   for (uint32_t i = 1;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > limit_ns) break;
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit_ns) break;
       __nanosleep(64);
     }
   }
   *abort_flag = 1;
   return false;
+}
+
+// The same wait for a whole converged warp, with a warp-uniform result: the polls of one round are a
+// loop inside one asm statement, so that the code around it stays free of divergent branches and its
+// operands can live in uniform registers (a single thread's MMA loop written with mbar_wait took
+// ~900 clocks per K-step of serial code; see density_factored.cu).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                               uint64_t limit_ns) {
+  const uint32_t addr = smem_u32(bar);
+  const uint32_t polls = limit_ns < 100000ull ? 1u : 64u;
+  uint64_t t0 = 0;
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n\t"
+        "WAIT_LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra WAIT_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 q, n, 0;\n\t"
+        "@q bra WAIT_LOOP;\n\t"
+        "WAIT_DONE:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity), "r"(polls)
+        : "memory");
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
+    const uint64_t now = globaltimer_ns();
+    if (t0 == 0) t0 = now;
+    const bool out = now - t0 > limit_ns;
+    if (out) *abort_flag = 1;
+    if (__any_sync(0xffffffffu, out || *abort_flag)) return false;
+  }
+}
+
+// One lane of a converged warp (always the same one).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b32 d;\n\t"
+      "elect.sync d|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(r));
+  return r != 0;
 }
 
 // Bounded wait used after an abort, for work this thread itself started (copies in flight, MMAs
