@@ -6,27 +6,23 @@
 // Dirichlet mode (new): V'(interior) = (sum of 6 neighbours + 4 pi h^2 rho) / 6, evaluated as an
 // increment of V, and the outer shell keeps its given values.
 //
-// One cooperative, persistent launch runs every sweep.  A work item is four consecutive x
-// points (float4 loads of the row, the four neighbouring rows and Q): the grids of the path
-// (three fields up to 192^3 = 85 MB) stay in the 126 MB L2 across sweeps, so the stencil is
-// limited by L2 latency and wants many independent loads in flight rather than on-chip reuse.
-// Sweeps are separated by a grid barrier of this file (bounded wait: it raises an error flag
-// after the library's wait limit, 2 s unless qmt_set_wait_limit_ns changed it).
+// Three kernels, all one launch for every sweep and all with the same update, so their results are
+// identical; they differ in where the field lives and who waits for whom:
+//   persistent  any grid: the field in L2 (three fields up to 192^3 = 85 MB stay there), a work item
+//               is four consecutive x points, a grid barrier between sweeps (persistent.cuh);
+//   plane       nz <= the SM count, planes of up to 16384 points: one CTA per plane, values in
+//               registers and shared memory, only z neighbours through L2, each CTA waiting for its two
+//               neighbours' publications;
+//   cluster     up to 4096 points a plane, 64 planes: one 16-CTA thread-block cluster, the field in
+//               the CTAs' shared memory, z neighbours through distributed shared memory, the hardware
+//               cluster barrier between sweeps (the best for the smallest grids).
 // V and its copy are rewritten by other CTAs between sweeps, so they are read through L2
 // (ld.global.cg), never through the non-coherent L1 paths.  On sweeps that feed a
-// convergence check each CTA sums |V' - V| in FP64 over its units; CTA 0 adds the CTA sums in
-// CTA order, so the residual is deterministic, and every CTA takes the same stop decision.
-//
-// Small grids (a plane of at most 4096 points, at most 4 planes per CTA of a 16-CTA cluster:
-// the 64^3 grid of the small-molecule configuration) can run as one thread-block cluster instead
-// (the automatic choice for the Dirichlet update):
-// the field lives in the CTAs' shared memory (two buffers of each CTA's z-slab), each thread
-// keeps its column of four-point groups and their charges in registers, neighbours come from
-// registers (z inside the slab), warp shuffles (x), shared memory (y, x across warps) and the
-// neighbouring CTAs' shared memory (z across slabs, distributed shared memory), and sweeps are
-// separated by the hardware cluster barrier -- no global-memory round trip and no software
-// grid barrier per sweep.  Both kernels apply jac_point, so their results are identical.
+// convergence check each CTA sums |V' - V| in FP64 over its points and the CTA sums are added in
+// CTA order, so the residual is deterministic, and every CTA takes the same stop decision.  Every wait is
+// bounded: it raises an error flag after the library's wait limit (2 s unless qmt_set_wait_limit_ns changed it).
 #include "mol.cuh"
+#include "persistent.cuh"
 #include "reduce.cuh"
 
 namespace qmt {
@@ -45,60 +41,12 @@ struct JacobiArgs {
   int max_sweeps, check_every;
   double tol;
   double* part;        // per-CTA partial sums
-  unsigned* bar;       // [0] arrivals, [1] generation
+  unsigned long long* bar;   // grid-barrier counter
+  unsigned long long* pub;   // plane kernel: sweeps published by each plane
   uint64_t wait_ns;    // limit of a grid-barrier wait before the solve gives up
   double* res;         // [0] residual of the last check
   int* out;            // [0] sweeps done, [1] status: 0 running/cap, 1 converged, 2 not finite, 3 barrier timeout
 };
-
-__device__ __forceinline__ uint64_t jac_timer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Sense-counting grid barrier for a cooperative launch (all CTAs co-resident).  Returns false
-// on every CTA once any CTA has waited more than `wait_ns` or raised the flag.  Arrivals are
-// acquire-release atomics on bar[0] (the CTA's writes are ordered before its arrival by the CTA
-// barrier); the last arrival resets the count and releases the generation bar[1], which the
-// others read with acquire loads: no full memory fences.
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ bool grid_barrier(unsigned* bar, int* flag, unsigned nblocks, uint64_t wait_ns) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    volatile int* vflag = flag;
-    const unsigned g = ld_acquire_gpu(bar + 1);
-    int ok = 1;
-    unsigned old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
-    if (old == nblocks - 1) {
-      asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(bar) : "memory");
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar + 1) : "memory");
-    } else {
-      const uint64_t t0 = jac_timer_ns();
-      while (ld_acquire_gpu(bar + 1) == g) {
-        if (*vflag) {
-          ok = 0;
-          break;
-        }
-        if (jac_timer_ns() - t0 > wait_ns) {
-          atomicExch(flag, 1);
-          ok = 0;
-          break;
-        }
-      }
-    }
-    ok_s = ok && !*vflag;
-  }
-  __syncthreads();
-  return ok_s != 0;
-}
 
 template <bool DIRICHLET>
 __device__ __forceinline__ float jac_source(float q, float h, float src_scale) {
@@ -129,33 +77,13 @@ __device__ __forceinline__ float jac_point(float xm, float xp, float yp, float y
   }
 }
 
-__device__ __forceinline__ float4 ldcg4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
-
-// A thread's work items in a sweep: the grid-stride sequence tid, tid + nthreads, ... over
-// the groups (or points), as grid coordinates of the first item and of the stride, advanced by
-// additions with carries -- no division per item (the stride is below nxq * ny * nz, so each
-// carry needs one subtraction).  Set up once per launch.
-struct JacWalk {
-  int x, y, z;      // first item: x group (vec4) or point
-  int sx, sy, sz;   // the stride
-};
-
-__device__ JacWalk jac_walk(const JacobiArgs& a) {
-  const uint32_t w = a.vec4 ? (uint32_t)(a.nx >> 2) : (uint32_t)a.nx;
-  const uint32_t ny = (uint32_t)a.ny;
-  const uint32_t nthreads = gridDim.x * JAC_THREADS;   // (the grid is a few CTAs per SM)
-  const uint32_t tid = blockIdx.x * JAC_THREADS + threadIdx.y * JX + threadIdx.x;
-  const uint32_t r = tid / w, rs = nthreads / w;
-  return JacWalk{(int)(tid - r * w), (int)(r % ny), (int)(r / ny), (int)(nthreads - rs * w), (int)(rs % ny),
-                 (int)(rs / ny)};
-}
 
 // One sweep src -> dst.  Work items are groups of four consecutive x points (float4 loads of
 // the row, the four neighbouring rows and Q, scalar loads of the two x halo values), spread over
 // all CTAs; every load of a group is independent, so many are in flight per thread.  Returns
 // this thread's FP64 sum |dst - src| when `resid` is set.
 template <bool DIRICHLET>
-__device__ double sweep(const JacobiArgs& a, const float* src, float* dst, bool resid, const JacWalk& wk) {
+__device__ double sweep(const JacobiArgs& a, const float* src, float* dst, bool resid, const GridWalk& wk) {
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const int64_t row = nx, plane = (int64_t)nx * ny;
   const int64_t nthreads = (int64_t)gridDim.x * JAC_THREADS;
@@ -165,7 +93,6 @@ __device__ double sweep(const JacobiArgs& a, const float* src, float* dst, bool 
     const int nxq = nx >> 2;
     const int64_t ngroups = (int64_t)nxq * ny * nz;
     int xq = wk.x, y = wk.y, z = wk.z;
-    const int sx = wk.sx, sy = wk.sy, sz = wk.sz;
     for (int64_t gi = tid; gi < ngroups; gi += nthreads) {
       const int x0 = xq * 4;
       const int64_t b = z * plane + (int64_t)y * row + x0;
@@ -192,22 +119,11 @@ __device__ double sweep(const JacobiArgs& a, const float* src, float* dst, bool 
       if (resid)
         dsum += (fabs((double)o.x - (double)c.x) + fabs((double)o.y - (double)c.y)) +
                 (fabs((double)o.z - (double)c.z) + fabs((double)o.w - (double)c.w));
-      xq += sx;
-      if (xq >= nxq) {
-        xq -= nxq;
-        ++y;
-      }
-      y += sy;
-      if (y >= ny) {
-        y -= ny;
-        ++z;
-      }
-      z += sz;
+      grid_step(wk, nxq, ny, xq, y, z);
     }
   } else {
     const int64_t n = plane * nz;
     int x = wk.x, y = wk.y, z = wk.z;
-    const int sx = wk.sx, sy = wk.sy, sz = wk.sz;
     for (int64_t g = tid; g < n; g += nthreads) {
       const float vc = __ldcg(src + g);
       const float xm = x > 0 ? __ldcg(src + g - 1) : 0.f;
@@ -221,17 +137,7 @@ __device__ double sweep(const JacobiArgs& a, const float* src, float* dst, bool 
           jac_point<DIRICHLET>(xm, xp, yp, ym, zp, zm, jac_source<DIRICHLET>(__ldg(a.Q + g), a.h, a.src_scale), vc, edge);
       __stcg(dst + g, o);
       if (resid) dsum += fabs((double)o - (double)vc);
-      x += sx;
-      if (x >= nx) {
-        x -= nx;
-        ++y;
-      }
-      y += sy;
-      if (y >= ny) {
-        y -= ny;
-        ++z;
-      }
-      z += sz;
+      grid_step(wk, nx, ny, x, y, z);
     }
   }
   return dsum;
@@ -245,19 +151,20 @@ __global__ void __launch_bounds__(JAC_THREADS, JAC_BLOCKS_PER_SM) jacobi_persist
   double delta = INFINITY;
   int sweeps = 0, pairs = 0, status = 0;
   const int lin = threadIdx.y * JX + threadIdx.x;
-  const JacWalk wk = jac_walk(a);
+  unsigned long long round = 0;
+  const GridWalk wk = grid_walk(a.vec4 ? a.nx >> 2 : a.nx, a.ny, gridDim.x * JAC_THREADS, blockIdx.x * JAC_THREADS + lin);
   while (sweeps + 2 <= a.max_sweeps) {
     ++pairs;
     const bool check = pairs % a.check_every == 0 || sweeps + 4 > a.max_sweeps;
     sweep<DIRICHLET>(a, a.V, a.T, false, wk);
-    if (!grid_barrier(a.bar, flag, nb, a.wait_ns)) {
+    if (!grid_barrier(a.bar, round, flag, nb, a.wait_ns)) {
       status = 3;
       break;
     }
     const double ds = sweep<DIRICHLET>(a, a.T, a.V, check, wk);
     sweeps += 2;
     if (!check) {
-      if (!grid_barrier(a.bar, flag, nb, a.wait_ns)) {
+      if (!grid_barrier(a.bar, round, flag, nb, a.wait_ns)) {
         status = 3;
         break;
       }
@@ -273,7 +180,7 @@ __global__ void __launch_bounds__(JAC_THREADS, JAC_BLOCKS_PER_SM) jacobi_persist
       for (int w = 0; w < JAC_THREADS / 32; ++w) r += sh[w];
       __stcg(a.part + blockIdx.x, r);
     }
-    if (!grid_barrier(a.bar, flag, nb, a.wait_ns)) {
+    if (!grid_barrier(a.bar, round, flag, nb, a.wait_ns)) {
       status = 3;
       break;
     }
@@ -282,7 +189,7 @@ __global__ void __launch_bounds__(JAC_THREADS, JAC_BLOCKS_PER_SM) jacobi_persist
       for (unsigned b = 0; b < nb; ++b) r += __ldcg(a.part + b);
       __stcg(a.res, r);
     }
-    if (!grid_barrier(a.bar, flag, nb, a.wait_ns)) {
+    if (!grid_barrier(a.bar, round, flag, nb, a.wait_ns)) {
       status = 3;
       break;
     }
@@ -297,6 +204,187 @@ __global__ void __launch_bounds__(JAC_THREADS, JAC_BLOCKS_PER_SM) jacobi_persist
     }
   }
   if (blockIdx.x == 0 && lin == 0) {
+    a.out[0] = sweeps;
+    a.out[1] = status;
+    __stcg(a.res + 1, delta);
+  }
+}
+
+// ---- plane kernel ------------------------------------------------------------------------------
+// One CTA per plane z (nz <= the SM count): the plane's values stay in its threads' registers and, for the
+// x and y neighbours, in shared memory; the charges stay in shared memory; only the planes themselves go
+// through L2, for the CTAs of z - 1 and z + 1.  No grid barrier: CTA z publishes the number of sweeps it
+// has stored, and starts the next one when its two neighbours have published as many (they have then
+// also read what the next store overwrites).  Per sweep 12 B per point of L2 traffic (two planes read,
+// one written) against 28 of the persistent kernel, and the waiting time of two neighbours against all
+// CTAs'.  The x and y part of the update is formed before the wait.
+constexpr int JAC_PLANE_THREADS = 1024;
+constexpr int JAC_PLANE_MAX_G = 4;   // groups of four points per thread: planes of up to 16384 points
+
+// The update in two parts: the x and y neighbours, then z and the source (jac_point's order).
+template <bool DIRICHLET>
+__device__ __forceinline__ float jac_xy(float xm, float xp, float yp, float ym, float vc) {
+  if constexpr (!DIRICHLET) return ((xm + xp) + yp) + ym;
+  else return ((xm - vc) + (xp - vc)) + ((yp - vc) + (ym - vc));
+}
+template <bool DIRICHLET>
+__device__ __forceinline__ float jac_z(float part, float zp, float zm, float src, float vc, bool edge) {
+  if constexpr (!DIRICHLET) {
+    const float s = ((part + zp) + zm) - src;
+    return edge ? 0.f : s / 6.0f;
+  } else {
+    const float s = part + ((zp - vc) + (zm - vc));
+    return edge ? vc : fmaf(__fadd_rn(s, src), 1.0f / 6.0f, vc);
+  }
+}
+
+template <bool DIRICHLET, int G>
+__global__ void __launch_bounds__(JAC_PLANE_THREADS, 1) jacobi_plane_kernel(JacobiArgs a) {
+  extern __shared__ float4 pbuf[];
+  __shared__ double red[JAC_PLANE_THREADS / 32];
+  __shared__ int ok_s;
+  const int nx = a.nx, ny = a.ny, nz = a.nz, nxq = nx >> 2, ng = nxq * ny;
+  const int t = threadIdx.x, lane = t & 31, z = blockIdx.x;
+  int* flag = a.out + 2;
+  float4* val = pbuf;         // the plane's values
+  float4* src = pbuf + ng;    // its source terms
+  const int64_t plane = (int64_t)nx * ny, base = z * plane;
+  float4 v[G];
+  uint32_t edges = 0;         // per group: bit 0 whole row is edge, bit 1 x low, bit 2 x high, bit 3 y low, bit 4 y high
+#pragma unroll
+  for (int k = 0; k < G; ++k) {
+    const int g = t + k * JAC_PLANE_THREADS;
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < ng) {
+      const int y = g / nxq, xq = g - y * nxq;
+      v[k] = __ldcg(reinterpret_cast<const float4*>(a.V + base) + g);
+      const float4 q4 = __ldg(reinterpret_cast<const float4*>(a.Q + base) + g);
+      src[g] = make_float4(jac_source<DIRICHLET>(q4.x, a.h, a.src_scale), jac_source<DIRICHLET>(q4.y, a.h, a.src_scale),
+                           jac_source<DIRICHLET>(q4.z, a.h, a.src_scale), jac_source<DIRICHLET>(q4.w, a.h, a.src_scale));
+      val[g] = v[k];
+      uint32_t e = 0;
+      if (y == 0 || y == ny - 1 || z == 0 || z == nz - 1) e |= 1u;
+      if (xq == 0) e |= 2u;
+      if (xq == nxq - 1) e |= 4u;
+      if (y == 0) e |= 8u;
+      if (y == ny - 1) e |= 16u;
+      edges |= e << (8 * k);
+    }
+  }
+  __syncthreads();
+  int sweeps = 0, pairs = 0, status = 0;
+  unsigned long long round = 0;
+  double delta = INFINITY;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  while (sweeps + 2 <= a.max_sweeps) {
+    ++pairs;
+    const bool check = pairs % a.check_every == 0 || sweeps + 4 > a.max_sweeps;
+    double ds = 0.0;
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      const float* from = half == 0 ? a.V : a.T;
+      float* to = half == 0 ? a.T : a.V;
+      const bool resid = check && half == 1;
+      // x and y neighbours from this CTA's plane
+      float4 p[G];
+#pragma unroll
+      for (int k = 0; k < G; ++k) {
+        const int g = t + k * JAC_PLANE_THREADS;
+        const uint32_t e = edges >> (8 * k);
+        const float4 c = v[k];
+        const float wl = __shfl_up_sync(0xffffffffu, c.w, 1), xr0 = __shfl_down_sync(0xffffffffu, c.x, 1);
+        if (g < ng) {
+          const float4 ym = e & 8u ? zero : val[g - nxq], yp = e & 16u ? zero : val[g + nxq];
+          const float xl = e & 2u ? 0.f : (lane == 0 ? val[g - 1].w : wl);
+          const float xr = e & 4u ? 0.f : (lane == 31 ? val[g + 1].x : xr0);
+          p[k].x = jac_xy<DIRICHLET>(xl, c.y, yp.x, ym.x, c.x);
+          p[k].y = jac_xy<DIRICHLET>(c.x, c.z, yp.y, ym.y, c.y);
+          p[k].z = jac_xy<DIRICHLET>(c.y, c.w, yp.z, ym.z, c.z);
+          p[k].w = jac_xy<DIRICHLET>(c.z, xr, yp.w, ym.w, c.w);
+        }
+      }
+      // the neighbouring planes have stored sweep `sweeps + half`
+      if (t == 0) ok_s = 1;
+      __syncthreads();
+      if (t < 2) {
+        const int zn = t == 0 ? z - 1 : z + 1;
+        if (zn >= 0 && zn < nz && !wait_count(a.pub + zn, (unsigned long long)(sweeps + half), flag, a.wait_ns)) {
+          atomicOr(a.pub + z, kGaveUp);   // passes it on
+          ok_s = 0;
+        }
+      }
+      __syncthreads();
+      if (!ok_s) {
+        status = 3;
+        break;
+      }
+#pragma unroll
+      for (int k = 0; k < G; ++k) {
+        const int g = t + k * JAC_PLANE_THREADS;
+        if (g < ng) {
+          const uint32_t e = edges >> (8 * k);
+          const float4 zm = z > 0 ? __ldcg(reinterpret_cast<const float4*>(from + base - plane) + g) : zero;
+          const float4 zp = z + 1 < nz ? __ldcg(reinterpret_cast<const float4*>(from + base + plane) + g) : zero;
+          const float4 s4 = src[g], c = v[k];
+          const bool er = e & 1u, elo = e & 2u, ehi = e & 4u;
+          float4 o;
+          o.x = jac_z<DIRICHLET>(p[k].x, zp.x, zm.x, s4.x, c.x, er || elo);
+          o.y = jac_z<DIRICHLET>(p[k].y, zp.y, zm.y, s4.y, c.y, er);
+          o.z = jac_z<DIRICHLET>(p[k].z, zp.z, zm.z, s4.z, c.z, er);
+          o.w = jac_z<DIRICHLET>(p[k].w, zp.w, zm.w, s4.w, c.w, er || ehi);
+          __stcg(reinterpret_cast<float4*>(to + base) + g, o);
+          val[g] = o;
+          v[k] = o;
+          if (resid)
+            ds += (fabs((double)o.x - (double)c.x) + fabs((double)o.y - (double)c.y)) +
+                  (fabs((double)o.z - (double)c.z) + fabs((double)o.w - (double)c.w));
+        }
+      }
+      __syncthreads();   // the plane's stores before its publication, its values before the next reads
+      if (t == 0)
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(a.pub + z) : "memory");
+    }
+    if (status) break;
+    sweeps += 2;
+    if (!check) continue;
+    // FP64 residual: warp tree, warps in order, planes in order; every CTA adds the same partials in
+    // the same order and takes the same decision
+    for (int o = 16; o > 0; o >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, o);
+    if (lane == 0) red[t >> 5] = ds;
+    __syncthreads();
+    if (t == 0) {
+      double r = 0.0;
+      for (int w = 0; w < JAC_PLANE_THREADS / 32; ++w) r += red[w];
+      __stcg(a.part + z, r);
+    }
+    if (!grid_barrier(a.bar, round, flag, gridDim.x, a.wait_ns)) {
+      status = 3;
+      break;
+    }
+    if (t < 32) {
+      double r = 0.0;
+      for (int b = t; b < nz; b += 32) r += __ldcg(a.part + b);
+      for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+      if (t == 0) red[0] = r;
+    }
+    __syncthreads();
+    delta = red[0];
+    // the partials may be overwritten only when every CTA has read them: the next check is at least one
+    // publication of the neighbours away, but not of all CTAs
+    if (!grid_barrier(a.bar, round, flag, gridDim.x, a.wait_ns)) {
+      status = 3;
+      break;
+    }
+    if (!isfinite(delta)) {
+      status = 2;
+      break;
+    }
+    if (delta <= a.tol) {
+      status = 1;
+      break;
+    }
+  }
+  if (z == 0 && t == 0) {
     a.out[0] = sweeps;
     a.out[1] = status;
     __stcg(a.res + 1, delta);
@@ -466,6 +554,42 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
   }
 }
 
+// Groups per thread of the plane kernel for this grid, or 0 where it does not apply or is not the faster
+// one: one CTA per plane, all resident at once.  Its sweep takes about 1.2 us + 1.05 us per group of
+// 1024 x 4 points of a plane, whatever nz; the grid-barrier kernel's 2.2 us + 2.3 us per million points
+// (Dirichlet, us per sweep, plane / grid barrier: 64^3 2.1 / 2.6, 120x56x56 2.8 / 3.2, 128x64x128 2.9 / 4.9,
+// 96x96x64 3.9 / 4.0, 96x128x120 4.5 / 5.9, 128^3 5.4 / 6.9, 128x120x88 5.2 / 5.7, 128x128x48 5.3 / 4.7).
+static int plane_groups(const JacobiArgs& a, int nsm) {
+  if (!a.vec4 || a.nz > nsm) return 0;
+  const int64_t ng = (int64_t)(a.nx / 4) * a.ny, n = 4 * ng * a.nz;
+  const int64_t g = (ng + JAC_PLANE_THREADS - 1) / JAC_PLANE_THREADS;
+  static const int64_t least[JAC_PLANE_MAX_G + 1] = {0, 0, 300000, 550000, 1300000};
+  return g <= JAC_PLANE_MAX_G && n >= least[g] ? (int)g : 0;
+}
+
+template <bool DIRICHLET, int G>
+static qmt_status launch_plane(JacobiArgs& a, cudaStream_t s, bool* launched) {
+  auto kern = jacobi_plane_kernel<DIRICHLET, G>;
+  const size_t smem = 2ull * (a.nx / 4) * a.ny * sizeof(float4);
+  QMT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  void* params[] = {&a};
+  QMT_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(a.nz), dim3(JAC_PLANE_THREADS), params, smem, s));
+  note_launches(1);
+  *launched = true;
+  return QMT_OK;
+}
+
+template <bool DIRICHLET>
+static qmt_status try_plane(JacobiArgs& a, int G, cudaStream_t s, bool* launched) {
+  switch (G) {
+    case 1: return launch_plane<DIRICHLET, 1>(a, s, launched);
+    case 2: return launch_plane<DIRICHLET, 2>(a, s, launched);
+    case 3: return launch_plane<DIRICHLET, 3>(a, s, launched);
+    case 4: return launch_plane<DIRICHLET, 4>(a, s, launched);
+    default: return QMT_OK;
+  }
+}
+
 static int g_jacobi_path = 0;   // 0 automatic, 1 grid barrier per sweep, 2 single cluster
 
 // Planes per CTA of the cluster kernel for this grid (1, 2 or 4), or 0 if it does not apply.
@@ -554,25 +678,30 @@ static qmt_status run_jacobi(int nx, int ny, int nz, float step, const float* rh
   const int64_t items = a.vec4 ? (int64_t)(nx / 4) * ny * nz : (int64_t)nx * ny * nz;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + JAC_THREADS - 1) / JAC_THREADS, capacity));
 
-  // scratch: CTA partial sums, barrier words, residuals, status words (grows, never freed)
+  // scratch: CTA partial sums, barrier words, residuals, status words, publications (grows, never freed)
   static thread_local DevBuf scratch;
-  const size_t part_bytes = ((size_t)grid * sizeof(double) + 255) / 256 * 256;
-  qmt_status st = scratch.reserve(part_bytes + 256);
+  const size_t part_bytes = ((size_t)std::max(grid, nsm) * sizeof(double) + 255) / 256 * 256;
+  const size_t word_bytes = 256 + (size_t)nsm * sizeof(unsigned long long);
+  qmt_status st = scratch.reserve(part_bytes + word_bytes);
   if (st) return st;
   uint8_t* base = scratch.as<uint8_t>();
   a.part = reinterpret_cast<double*>(base);
   a.res = reinterpret_cast<double*>(base + part_bytes);          // [0] check sum, [1] last residual
-  a.bar = reinterpret_cast<unsigned*>(base + part_bytes + 64);    // [0] arrivals, [1] generation
+  a.bar = reinterpret_cast<unsigned long long*>(base + part_bytes + 64);
+  a.pub = reinterpret_cast<unsigned long long*>(base + part_bytes + 256);
   a.out = reinterpret_cast<int*>(base + part_bytes + 128);        // [0] sweeps, [1] status, [2] flag
-  QMT_CUDA(cudaMemsetAsync(base + part_bytes, 0, 256, s));
+  QMT_CUDA(cudaMemsetAsync(base + part_bytes, 0, word_bytes, s));
   if (max_sweeps >= 2) {
     bool done = false;
-    // the cluster kernel where it applies: for the Dirichlet update (measured 3.8 against 4.2 us per
-    // 64^3 sweep); the reference update's IEEE division makes it issue-bound on its 16 SMs (4.5
-    // against 4.3 us), so automatic selection leaves that one on the grid-barrier kernel
-    const bool want_cluster = g_jacobi_path == 2 || (g_jacobi_path == 0 && DIRICHLET);
+    // automatic: the cluster kernel for grids of up to 32768 points (32^3: 1.4 us per sweep against 1.8 of
+    // the plane and 2.1 of the grid-barrier kernel; 40^3, four planes a CTA: 2.7, 1.9, 2.2), else the
+    // plane kernel where plane_groups has it, else the grid-barrier kernel
+    const bool small = (int64_t)nx * ny * nz <= 32768;
+    const bool want_cluster = g_jacobi_path == 2 || (g_jacobi_path == 0 && small);
     const int P = want_cluster ? cluster_planes(nx, ny, nz, rho, v) : 0;
-    if (!done && P > 0 && (st = try_cluster<DIRICHLET>(a, P, s, &done))) return st;
+    if (P > 0 && (st = try_cluster<DIRICHLET>(a, P, s, &done))) return st;
+    const int G = !done && g_jacobi_path == 0 ? plane_groups(a, nsm) : 0;
+    if (G && (st = try_plane<DIRICHLET>(a, G, s, &done))) return st;
     if (g_jacobi_path == 2 && !done)
       return fail(QMT_BAD_ARG, "the single-cluster Jacobi kernel does not apply to this grid or device");
     if (!done) {
