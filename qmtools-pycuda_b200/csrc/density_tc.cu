@@ -1949,19 +1949,22 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
       st = run_tc<FMT_BF16>(mol, sh, pm, ntiles, precision, qube, outscale, s, nullptr, nullptr, (size_t)2 << 30, gate);
   }
   if (st) return st;
-  st = finish_density(mol, pm.nvox, ntiles, rescale, qube, sum_out, s);
-  if (st) return st;
+  if ((st = finish_density(mol, pm.nvox, ntiles, rescale, qube, nullptr, s))) return st;
   // The kernels' barrier-timeout flag is sticky: a call that returns a host sum (and so
-  // synchronises anyway) reads and clears it; fully asynchronous calls leave it for the next
-  // synchronous call on this molecule.
+  // synchronises anyway) reads it beside the sum and clears it; fully asynchronous calls leave it for
+  // the next synchronous call on this molecule.
   if (sum_out) {
-    int err = 0;
-    QMT_CUDA(cudaMemcpyAsync(&err, mol->d_scalars.as<double>() + 8, sizeof(int), cudaMemcpyDeviceToHost, s));
+    double h[9];   // [0] sum, [8] flag
+    QMT_CUDA(cudaMemcpyAsync(h, mol->d_scalars.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     QMT_CUDA(cudaStreamSynchronize(s));
+    *sum_out = h[0];
+    int err = 0;
+    std::memcpy(&err, h + 8, sizeof(err));
     if (err) {
       QMT_CUDA(cudaMemsetAsync(mol->d_scalars.as<double>() + 8, 0, sizeof(int), s));
       return fail(QMT_CUDA_ERR, "tensor-core density kernel gave up waiting on a barrier");
     }
+    if (!std::isfinite(h[0])) return fail(QMT_NAN, "non-finite density sum");
   }
   return QMT_OK;
 }

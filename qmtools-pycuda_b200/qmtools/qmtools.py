@@ -256,7 +256,7 @@ class Grid:
         if not numpy.array_equal(grd, blk * 8):
             raise ValueError("shape for xyz have to be multiple of 8")
         self.GPUblocks = tuple([x.item() for x in blk])
-        self.qube = numpy.zeros(self.shape).astype(numpy.float32)
+        self.qube = numpy.zeros(self.shape, dtype=numpy.float32)   # (pages are touched only when used)
         self.npts = numpy.uint32(self.shape[1] * self.shape[2] * self.shape[3])
         self.nfields = numpy.uint32(self.shape[0])
         self.step = numpy.float32(step * ANG2BOR)
@@ -294,7 +294,7 @@ class Grid:
 
     def _download(self):
         if self._t is not None:
-            self.qube = self._t.cpu().numpy().reshape(self.shape).copy()
+            self.qube = self._t.cpu().numpy().reshape(self.shape)
 
     def CopyBack(self):
         self._download()
@@ -413,9 +413,15 @@ class Grid:
         return grid
 
 
-def _new_like(g, nfields=None):
+def _new_like(g, nfields=None, written=False):
+    """A grid like `g` with device storage, zero unless its one field is about to be `written` whole.
+
+    The storage is made on the device and the host array's pages stay untouched: making zeros on the host
+    and uploading them took 3.5 ms for 192^3 points."""
     out = Grid.emptyAs(g, nfields)
-    out.tensor()
+    N.ensure_device()
+    new = _torch().empty if written and out.shape[0] == 1 else _torch().zeros
+    out._t = new(int(numpy.prod(out.shape)), dtype=_torch().float32, device="cuda")
     return out
 
 
@@ -430,7 +436,7 @@ class QMTools:
                         rescale=True):
         import ctypes as C
         prec = QMTools.default_precision if precision is None else precision
-        cgrid = _new_like(grid)
+        cgrid = _new_like(grid, written=True)
         nx, ny, nz, h, ox, oy, oz = grid._geom()
         s = C.c_double()
         N.call("qmt_density", molecule.handle, nx, ny, nz, h, ox, oy, oz, int(subgrid), N.PREC[prec],
