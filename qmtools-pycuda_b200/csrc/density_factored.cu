@@ -877,6 +877,161 @@ UnitTables build_units(const qmt_mol* m, const std::vector<float>& fs) {
   return out;
 }
 
+// ---- pivoted Cholesky factorisation (FP64, one thread-block cluster) ----------------------------------
+// Largest remaining diagonal first (compared in FP32, lowest index on a tie: any pivot near the largest
+// serves), until it is at most tol times the first, or rmax columns are done.  Each CTA owns a block of
+// rows: their remaining diagonal and their rows of L in shared memory (of L2 when they do not fit).  A
+// column is a chain of latencies: the CTAs exchange their largest diagonals through distributed shared
+// memory (one cluster barrier; none with a single CTA), fetch the pivot's row of L from its owner while
+// P's row comes from L2, form their elements, eight lanes a row, and find their next largest diagonal.
+// info: [0] the rank, [1] set when it exceeds rmax or a remaining diagonal is negative beyond rounding
+// (the matrix is indefinite).
+constexpr int PIV_THREADS = 512;
+constexpr int PIV_MAX_CTAS = 16;
+constexpr int PIV_PRE = 2;                    // rows per thread whose element of P is fetched early
+struct PivotArgs {
+  const double* P;
+  int np, n, rmax, rows;      // rows per CTA
+  int rows_in_smem, ld;       // row stride of L in shared memory
+  double tol;
+  double* L;                  // n x rmax, FP64 (used when the rows do not fit in shared memory)
+  float* L0;                  // n x ld0, FP32, zero beyond the rank up to a multiple of 16
+  int ld0;
+  int* info;
+  double* dmax;               // the first pivot
+};
+
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ double cluster_load_f64(const double* p, uint32_t rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+
+struct PivotCand {
+  double d;
+  int at;
+  uint32_t key;   // FP32 bits of d (0 when it is not positive): ordered like the values
+};
+__device__ __forceinline__ uint32_t pivot_key(double d) { return d > 0.0 ? __float_as_uint((float)d) : 0u; }
+// The warp's best candidate, the lowest lane on a tie, on every lane.
+__device__ __forceinline__ PivotCand pivot_best(PivotCand c) {
+  const uint32_t mx = __reduce_max_sync(0xffffffffu, c.key);
+  const int w = __ffs(__ballot_sync(0xffffffffu, c.key == mx)) - 1;
+  PivotCand b;
+  b.key = mx;
+  b.d = __shfl_sync(0xffffffffu, c.d, w);
+  b.at = __shfl_sync(0xffffffffu, c.at, w);
+  return b;
+}
+
+__global__ void __launch_bounds__(PIV_THREADS, 1) fact_pivot_kernel(PivotArgs a) {
+  extern __shared__ double piv_s[];
+  __shared__ __align__(16) PivotCand cand[2][32];   // per column parity and CTA
+  __shared__ PivotCand wbest[PIV_THREADS / 32];
+  const uint32_t c = cluster_cta_rank(), ncta = gridDim.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = t & 7, r0 = (int)c * a.rows;
+  const int nr = max(0, min(a.rows, a.n - r0)), nr4 = (nr + 3) / 4 * 4;   // (whole warps in every round)
+  double* d = piv_s;                            // remaining diagonal of the rows
+  double* lj = d + a.rows;                      // the pivot's row of L
+  double* own = a.rows_in_smem ? lj + a.rmax : a.L + (size_t)r0 * a.rmax;
+  const int ld = a.rows_in_smem ? a.ld : a.rmax;
+  const PivotCand none{0.0, 0x7fffffff, 0u};
+  PivotCand best = none;                        // of this thread's rows (lanes with sub == 0)
+  for (int i = t >> 3; i < nr; i += PIV_THREADS / 8)
+    if (sub == 0) {
+      const double v = a.P[(size_t)(r0 + i) * a.np + r0 + i];
+      d[i] = v;
+      if (pivot_key(v) > best.key) best = PivotCand{v, r0 + i, pivot_key(v)};
+    }
+  if (t < 64) cand[t >> 5][t & 31] = none;
+  if (ncta > 1) cluster_barrier();              // every CTA's candidates are cleared before the first store
+  int q = 0;
+  bool high = false;
+  double dmax = 0.0;
+  for (;; ++q) {
+    best = pivot_best(best);
+    if (lane == 0) wbest[warp] = best;
+    __syncthreads();   // (also: this column's elements are in `own` and d)
+    if (warp == 0) {
+      best = pivot_best(lane < PIV_THREADS / 32 ? wbest[lane] : none);
+      if (lane < (int)ncta) {   // this CTA's candidate to every CTA
+        const uint32_t p = cluster_addr(&cand[q & 1][c], (uint32_t)lane);
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(p), "d"(best.d) : "memory");
+        asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(p + 8), "r"(best.at), "r"(best.key) : "memory");
+      }
+    }
+    if (ncta > 1) cluster_barrier();
+    else __syncthreads();
+    best = pivot_best(cand[q & 1][lane]);       // (CTAs in row order)
+    if (q == 0) dmax = best.d;
+    if (!(best.d > a.tol * dmax)) break;
+    if (q == a.rmax) {
+      high = true;
+      break;
+    }
+    const int jp = best.at;
+    double pij[PIV_PRE];
+#pragma unroll
+    for (int k = 0; k < PIV_PRE; ++k) {
+      const int i = (t >> 3) + k * (PIV_THREADS / 8);
+      pij[k] = sub == 0 && i < nr ? __ldg(a.P + (size_t)jp * a.np + r0 + i) : 0.0;
+    }
+    const uint32_t oc = (uint32_t)(jp / a.rows);
+    for (int k = t; k < q; k += PIV_THREADS)
+      lj[k] = a.rows_in_smem ? cluster_load_f64(own + (size_t)(jp - (int)oc * a.rows) * ld + k, oc)
+                             : __ldcg(a.L + (size_t)jp * a.rmax + k);
+    // 1 / sqrt of the pivot to ~1e-14: an FP32 estimate and one Newton step (the library's FP64 rsqrt is a
+    // long serial chain, and L0 is kept in FP32)
+    const double y0 = (double)rsqrtf((float)best.d);
+    const double ipiv = y0 * (1.5 - 0.5 * best.d * y0 * y0), piv = best.d * ipiv;
+    __syncthreads();
+    best = none;
+#pragma unroll 1
+    for (int i = t >> 3, k2 = 0; i < nr4; i += PIV_THREADS / 8, ++k2) {
+      double s = 0.0;
+      const bool in = i < nr;
+      const double* li = own + (size_t)(in ? i : 0) * ld;
+      for (int k = sub; k < q; k += 8) s = fma(a.rows_in_smem ? li[k] : __ldcg(li + k), lj[k], s);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (in && sub == 0) {
+        const bool isp = r0 + i == jp;
+        const double p = k2 == 0 ? pij[0] : (k2 == 1 ? pij[1] : __ldg(a.P + (size_t)jp * a.np + r0 + i));
+        const double x = isp ? piv : (p - s) * ipiv;
+        if (a.rows_in_smem) own[(size_t)i * ld + q] = x;
+        else __stcg(own + (size_t)i * ld + q, x);
+        a.L0[(size_t)(r0 + i) * a.ld0 + q] = (float)x;
+        const double dn = isp ? 0.0 : d[i] - x * x;
+        d[i] = dn;
+        if (pivot_key(dn) > best.key) best = PivotCand{dn, r0 + i, pivot_key(dn)};
+      }
+    }
+  }
+  bool bad = high;
+  for (int i = t; i < nr; i += PIV_THREADS) bad |= d[i] < -10.0 * a.tol * dmax;
+  if (__syncthreads_or(bad) && t == 0) atomicExch(a.info + 1, 1);
+  const int pad = max(16, (q + 15) / 16 * 16) - q;
+  for (int i = t; i < nr * pad; i += PIV_THREADS) a.L0[(size_t)(r0 + i / pad) * a.ld0 + q + i % pad] = 0.f;
+  if (c == 0 && t == 0) {
+    a.info[0] = q;
+    *a.dmax = dmax;
+  }
+  if (ncta > 1) cluster_barrier();   // no CTA leaves while another may still read its shared memory
+}
+
 // ---- refinement of the factor (FP64, device) ----------------------------------------------------
 // The float32 input matrix is L L^T only up to its rounding, and a pivoted Cholesky factor takes that
 // rounding from the pivot columns alone, amplified: 1.2e-6 relative L2 of the density at 30 atoms, of
@@ -884,7 +1039,7 @@ UnitTables build_units(const qmt_mol* m, const std::vector<float>& fs) {
 // L = Y C^-T is the Nystroem approximation of P on the range of Y (2e-7, as the truncated
 // eigendecomposition).  L0 only spans the space, so it comes as float32.
 __global__ void __launch_bounds__(256) fact_y_kernel(const double* __restrict__ P, int np, const float* __restrict__ L0,
-                                                     int n, int r16, double* __restrict__ Y) {
+                                                     int ld0, int n, int r16, double* __restrict__ Y) {
   __shared__ double ps[32][33];
   __shared__ float ls[32][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = blockIdx.x * 32, q = blockIdx.y * 32 + tx;
@@ -894,7 +1049,7 @@ __global__ void __launch_bounds__(256) fact_y_kernel(const double* __restrict__ 
     for (int k = 0; k < 4; ++k) {
       const int r = ty + 8 * k;
       ps[r][tx] = i0 + r < n && j0 + tx < n ? P[(size_t)(i0 + r) * np + j0 + tx] : 0.0;
-      ls[r][tx] = j0 + r < n && q < r16 ? L0[(size_t)(j0 + r) * r16 + q] : 0.f;
+      ls[r][tx] = j0 + r < n && q < r16 ? L0[(size_t)(j0 + r) * ld0 + q] : 0.f;
     }
     __syncthreads();
 #pragma unroll 8
@@ -911,8 +1066,8 @@ __global__ void __launch_bounds__(256) fact_y_kernel(const double* __restrict__ 
 }
 
 // M = L0^T Y, r16 x r16; one block per 16 x 16 tile.
-__global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L0, const double* __restrict__ Y, int n,
-                                                     int r16, double* __restrict__ M) {
+__global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L0, int ld0, const double* __restrict__ Y,
+                                                     int n, int r16, double* __restrict__ M) {
   __shared__ float ls[32][17];
   __shared__ double ys[32][17];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, a = blockIdx.x * 16, b = blockIdx.y * 16;
@@ -921,7 +1076,7 @@ __global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L
   for (int i0 = 0; i0 < n; i0 += 32) {
     for (int r = ty; r < 32; r += 16) {
       const bool in = i0 + r < n;
-      ls[r][tx] = in ? L0[(size_t)(i0 + r) * r16 + a + tx] : 0.f;
+      ls[r][tx] = in ? L0[(size_t)(i0 + r) * ld0 + a + tx] : 0.f;
       ys[r][tx] = in ? Y[(size_t)(i0 + r) * r16 + b + tx] : 0.0;
     }
     __syncthreads();
@@ -932,55 +1087,102 @@ __global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L
   M[(size_t)(a + ty) * r16 + b + tx] = acc;
 }
 
-// Lower Cholesky factor of the leading r x r block of M (one CTA; in shared memory when it was given
-// any), its transpose to CT (CT[k * r16 + i] = C_ik, i > k; 1 / C_kk for i = k).  A column whose pivot is
-// lost in rounding (1e-12 of its diagonal element: a pivot of L0 that was the input's rounding) is left
-// out, zero in CT; the residual check sees whether that mattered.
-// One barrier per column: the update a_ij -= a_ik a_jk / a_kk leaves the scaling to the end.
-__global__ void __launch_bounds__(1024) fact_chol_kernel(double* __restrict__ M, int r, int r16, int in_smem,
-                                                         double* __restrict__ CT) {
+// Lower Cholesky factor of the leading r x r block of M (one CTA), as its transpose in CT (CT[k * r16 + i] =
+// C_ik, i > k; 1 / C_kk for i = k).  Panels of CHOL_NB columns: thread i holds row i of the panel in
+// registers (one barrier a column), then all threads update what is right of it from the panel in shared
+// memory.  A column whose pivot is lost in rounding (1e-12 of its diagonal element: a pivot of L0 that was
+// the input's rounding) is left out, zero in CT; the residual check sees whether that mattered.
+constexpr int CHOL_NB = 16, CHOL_THREADS = 1024;
+__global__ void __launch_bounds__(CHOL_THREADS) fact_chol_kernel(double* __restrict__ M, int r, int r16, int in_smem,
+                                                                double* __restrict__ CT) {
   extern __shared__ double chol_s[];
-  __shared__ double least[kFactorMaxR16];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  __shared__ double prow[2][CHOL_NB];
+  __shared__ double pan[kFactorMaxR16][CHOL_NB + 1];   // the panel, scaled: C_ik
+  const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
   double* a = in_smem ? chol_s : M;
   const int ld = in_smem ? r16 + 1 : r16;
   if (in_smem)
     for (int i = ty; i < r; i += 32)
       for (int j = tx; j <= i; j += 32) a[i * ld + j] = M[(size_t)i * r16 + j];
+  double least = 0.0;   // thread i: the least pivot of column i
   __syncthreads();
-  if (threadIdx.x < r) least[threadIdx.x] = 1e-12 * a[threadIdx.x * ld + threadIdx.x];
+  if (t < r) least = 1e-12 * a[t * ld + t];
   __syncthreads();
-  for (int k = 0; k < r; ++k) {
-    const double p = a[k * ld + k];
-    const double inv = p > least[k] ? 1.0 / p : 0.0;
-    for (int i = k + 1 + ty; i < r; i += 32) {
-      const double f = a[i * ld + k] * inv;
-      for (int j = k + 1 + tx; j <= i; j += 32) a[i * ld + j] -= f * a[j * ld + k];
+  for (int k0 = 0; k0 < r; k0 += CHOL_NB) {
+    const int nb = min(CHOL_NB, r - k0);
+    double v[CHOL_NB];
+    const bool mine = t < r && t >= k0;
+#pragma unroll
+    for (int j = 0; j < CHOL_NB; ++j) v[j] = mine && j < nb && k0 + j <= t ? a[t * ld + k0 + j] : 0.0;
+#pragma unroll
+    for (int j = 0; j < CHOL_NB; ++j) {
+      if (j < nb) {
+        // row k0 + j has its final values of columns <= j: it publishes column j's C of the rows below
+        if (t == k0 + j) {
+          const double s = v[j] > least ? rsqrt(v[j]) : 0.0;
+          prow[j & 1][0] = s;
+        }
+        __syncthreads();
+        const double s = prow[j & 1][0];
+        if (mine && t >= k0 + j) {
+          v[j] = t == k0 + j ? s : v[j] * s;      // C_ij (the diagonal keeps 1 / C_jj)
+          pan[t][j] = v[j];
+        }
+        __syncthreads();
+        if (mine && t > k0 + j) {
+          // columns right of j in the panel: a_ic -= C_ij C_cj
+#pragma unroll
+          for (int c2 = j + 1; c2 < CHOL_NB; ++c2)
+            if (c2 < nb && k0 + c2 <= t) v[c2] = fma(-v[j], pan[k0 + c2][j], v[c2]);
+        }
+      }
+    }
+    __syncthreads();
+    if (mine) {
+      for (int j = 0; j < nb; ++j)
+        if (k0 + j <= t) CT[(size_t)(k0 + j) * r16 + t] = pan[t][j];
+    }
+    // what is right of the panel: a_ij -= sum_k C_ik C_jk (the panel's diagonal is above these rows)
+    const int k1 = k0 + nb;
+    for (int i = k1 + ty; i < r; i += 32) {
+      double ci[CHOL_NB];
+#pragma unroll
+      for (int k = 0; k < CHOL_NB; ++k) ci[k] = k < nb ? pan[i][k] : 0.0;
+      for (int j = k1 + tx; j <= i; j += 32) {
+        double x = a[i * ld + j];
+#pragma unroll
+        for (int k = 0; k < CHOL_NB; ++k) x = fma(-ci[k], k < nb ? pan[j][k] : 0.0, x);
+        a[i * ld + j] = x;
+      }
     }
     __syncthreads();
   }
-  for (int k = ty; k < r; k += 32) {
-    const double p = a[k * ld + k], s = p > least[k] ? rsqrt(p) : 0.0;
-    for (int i = k + tx; i < r; i += 32) CT[(size_t)k * r16 + i] = i == k ? s : a[i * ld + k] * s;
-  }
 }
 
-// L = Y C^-T row by row (a warp each; lane l holds columns l, l + 32, ...), in place, and the largest
-// |L_iq| 2^-s_i of each column (as ordered bits of a non-negative double).
-__global__ void __launch_bounds__(128) fact_solve_kernel(double* __restrict__ Y, const double* __restrict__ CT, int n,
-                                                         int r, int r16, const double* __restrict__ inv_s,
-                                                         unsigned long long* __restrict__ colmax) {
-  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= n) return;
+// L = Y C^-T row by row (a warp each; lane l holds columns l, l + 32, ...; 32 rows of C^T at a time in shared
+// memory), in place, and the largest |L_iq| 2^-s_i of each column (as ordered bits of a non-negative double).
+constexpr int SOLVE_WARPS = 8;
+__global__ void __launch_bounds__(32 * SOLVE_WARPS) fact_solve_kernel(double* __restrict__ Y,
+                                                                      const double* __restrict__ CT, int n, int r,
+                                                                      int r16, const double* __restrict__ inv_s,
+                                                                      unsigned long long* __restrict__ colmax) {
+  extern __shared__ double ct_s[];   // 32 x r16
+  const int row = blockIdx.x * SOLVE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const bool in = row < n;
   double y[kFactorMaxR16 / 32];
 #pragma unroll
-  for (int b = 0; b < kFactorMaxR16 / 32; ++b) y[b] = 32 * b + lane < r ? Y[(size_t)row * r16 + 32 * b + lane] : 0.0;
+  for (int b = 0; b < kFactorMaxR16 / 32; ++b)
+    y[b] = in && 32 * b + lane < r ? Y[(size_t)row * r16 + 32 * b + lane] : 0.0;
 #pragma unroll
   for (int b = 0; b < kFactorMaxR16 / 32; ++b) {
     if (32 * b >= r) break;
-    for (int e = 0; e < 32 && 32 * b + e < r; ++e) {
+    const int ne = min(32, r - 32 * b);
+    __syncthreads();
+    for (int i = threadIdx.x; i < ne * r16; i += 32 * SOLVE_WARPS) ct_s[i] = CT[(size_t)32 * b * r16 + i];
+    __syncthreads();
+    for (int e = 0; e < ne; ++e) {
       const int k = 32 * b + e;
-      const double* c = CT + (size_t)k * r16;
+      const double* c = ct_s + e * r16;
       const double x = __shfl_sync(0xffffffffu, y[b], e) * c[k];   // (the diagonal holds 1 / C_kk)
       if (lane == e) y[b] = x;
 #pragma unroll
@@ -988,6 +1190,7 @@ __global__ void __launch_bounds__(128) fact_solve_kernel(double* __restrict__ Y,
         if (b2 >= b && 32 * b2 + lane > k && 32 * b2 + lane < r) y[b2] = fma(-c[32 * b2 + lane], x, y[b2]);
     }
   }
+  if (!in) return;
   const double sc = inv_s[row];
 #pragma unroll
   for (int b = 0; b < kFactorMaxR16 / 32; ++b)
@@ -1010,18 +1213,37 @@ __global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax,
   hscale[q] = q < r ? ldexpf(1.0f, -h) : 0.f;
 }
 
-// Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds tol; L row i at L[i * ld].
-__global__ void fact_residual_kernel(const double* __restrict__ P, int np, const double* __restrict__ L, int n, int ld,
-                                     int r, double tol, int* bad) {
-  const int64_t tot = (int64_t)n * n;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < tot; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx / n), j = (int)(idx - (int64_t)i * n);
-    if (j > i) continue;
-    double v = P[(size_t)i * np + j];
-    const double* li = L + (size_t)i * ld;
-    const double* lj = L + (size_t)j * ld;
-    for (int q = 0; q < r; ++q) v -= li[q] * lj[q];
-    if (fabs(v) > tol) *bad = 1;
+// Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds rel * dmax; L row i at L[i * ld].  One block per
+// 32 x 32 tile on or below the diagonal.
+__global__ void __launch_bounds__(256) fact_residual_kernel(const double* __restrict__ P, int np,
+                                                            const double* __restrict__ L, int n, int ld, int r, double rel,
+                                                            const double* __restrict__ dmax, int* bad) {
+  __shared__ double li[32][33], lj[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  if (j0 > i0) return;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int q0 = 0; q0 < r; q0 += 32) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int x = ty + 8 * k;
+      const bool q = q0 + tx < r;
+      li[x][tx] = q && i0 + x < n ? L[(size_t)(i0 + x) * ld + q0 + tx] : 0.0;
+      lj[x][tx] = q && j0 + x < n ? L[(size_t)(j0 + x) * ld + q0 + tx] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+      const double b = lj[tx][q];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[k] = fma(li[ty + 8 * k][q], b, acc[k]);
+    }
+    __syncthreads();
+  }
+  const double tol = rel * *dmax;   // max |P_jk| <= max_j P_jj for a positive semi-definite P
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = i0 + ty + 8 * k, j = j0 + tx;
+    if (i < n && j <= i && !(fabs(P[(size_t)i * np + j] - acc[k]) <= tol)) *bad = 1;
   }
 }
 
@@ -1061,6 +1283,55 @@ constexpr double kFactorResid = 2e-7;
 
 }  // namespace
 
+static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double* L, float* L0, int* info, double* dmax,
+                               cudaStream_t s) {
+  int maxsm = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  QMT_CUDA(cudaFuncSetAttribute(fact_pivot_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (int ncta = n > 320 ? PIV_MAX_CTAS : (n > 128 ? 8 : 1); ncta >= 1; ncta /= 2) {
+    PivotArgs a{};
+    a.P = P;
+    a.np = np;
+    a.n = n;
+    a.rmax = rmax;
+    a.rows = (n + ncta - 1) / ncta;
+    a.ld = rmax + 8;   // (four rows of a warp on two sets of banks)
+    a.tol = kFactorTol;
+    a.L = L;
+    a.L0 = L0;
+    a.ld0 = rmax;
+    a.info = info;
+    a.dmax = dmax;
+    const size_t base = (size_t)(a.rows + rmax) * sizeof(double), rows = (size_t)a.rows * a.ld * sizeof(double);
+    if (base > (size_t)maxsm - 2048) continue;
+    a.rows_in_smem = base + rows <= (size_t)maxsm - 2048 ? 1 : 0;
+    const size_t smem = base + (a.rows_in_smem ? rows : 0);
+    QMT_CUDA(cudaFuncSetAttribute(fact_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ncta);
+    cfg.blockDim = dim3(PIV_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ncta;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int nclusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, fact_pivot_kernel, &cfg) != cudaSuccess || nclusters < 1) {
+      cudaGetLastError();   // a smaller cluster
+      continue;
+    }
+    QMT_CUDA(cudaLaunchKernelEx(&cfg, fact_pivot_kernel, a));
+    note_launches(1);
+    return QMT_OK;
+  }
+  return fail(QMT_BAD_ARG, "factorisation does not fit in shared memory");
+}
+
 qmt_status ensure_unit_tables(qmt_mol* m, const std::vector<float>& fs, cudaStream_t s) {
   const UnitTables t = build_units(m, fs);
   const size_t wb = t.words.size() * sizeof(int4), cb = t.column.size() * sizeof(int);
@@ -1074,116 +1345,84 @@ qmt_status ensure_unit_tables(qmt_mol* m, const std::vector<float>& fs, cudaStre
   return QMT_OK;
 }
 
+// Largest rank that is factored: half of n; with `any_rank` (fp16x3 and many sample points, see density_tc)
+// every rank of a matrix of up to 256 functions; bf16 as takes_factor says.
+static int factor_rmax(int n16, int fmt, bool any_rank) {
+  if (fmt != 0) return std::min(kBf16MaxRank, n16 / 2);
+  return any_rank && n16 <= kFactorMaxR16 ? n16 : std::min(kFactorMaxR16, n16 / 2);
+}
+
 // A density matrix of rank r (r = occupied orbitals for an SCF density, P = 2 C_occ C_occ^T) is
-// P = L L^T with L n x r.  L comes from a pivoted Cholesky factorisation in FP64 (largest remaining
-// diagonal first), stopped once every remaining diagonal element is at most kFactorTol of the largest
-// one; the factor is used when the matrix it leaves out is at most kFactorResid of max |P| (float32
-// input rounding is ~6e-8) and the rank is at most half of n.  A matrix that is not positive
-// semi-definite, or of high rank, takes the unfactored path.  The scaled factor W_jk =
-// L_jk 2^(h_k - s_j) (so Phi' W = 2^h_k (Phi L)_k, each column scaled to a maximum near 2^14) goes to
-// the blocks of fact_split_kernel.  Sets fact_rank = 0 when the matrix is not factored.
-qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, cudaStream_t s) {
-  if (m->fact_prec == prec) return QMT_OK;
+// P = L L^T with L n x r.  L comes from a pivoted Cholesky factorisation (fact_pivot_kernel), stopped
+// once every remaining diagonal element is at most kFactorTol of the largest one, and is refined; it is
+// used when the matrix it leaves out is at most kFactorResid of max |P| (float32 input rounding is
+// ~6e-8).  A matrix that is not positive semi-definite, or of high rank, takes the unfactored path.
+// The scaled factor W_jk = L_jk 2^(h_k - s_j) (so Phi' W = 2^h_k (Phi L)_k, each column scaled to a
+// maximum near 2^14) goes to the blocks of fact_split_kernel.  Sets fact_rank = 0 when the matrix is not
+// factored.  The host waits for the rank, once per matrix.
+qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, cudaStream_t s) {
+  // built for this precision, or refused by at least this rank limit
+  if (m->fact_prec == prec && (m->fact_rank > 0 || m->fact_any_rank || !any_rank)) return QMT_OK;
   qmt_status st;
   if ((st = ensure_basis_operands(m, kpad, s))) return st;
   const int n = m->norbs, np = m->npad, n16 = (n + 15) / 16 * 16;
   m->fact_prec = prec;
+  m->fact_any_rank = any_rank;
   m->fact_rank = 0;
-  const int rmax = std::min(fmt == 0 ? kFactorMaxR16 : kBf16MaxRank, n16 / 2);
+  const int rmax = std::max(16, factor_rmax(n16, fmt, any_rank));
   // a density matrix of N_e electrons whose occupations are at most 2 has rank >= N_e / 2: with
   // the nuclear charge for N_e (ions of up to 16 charges allowed for) a rank above rmax is known
-  // without the factorisation's host work (tens of milliseconds at a thousand functions)
+  // without factoring
   if (0.5 * m->qtot > rmax + 8) return QMT_OK;
-  // P_ij from the lower triangle of the matrix as given (no symmetric host copy is built)
-  const float* dm = m->dm_host.data();
-  auto Pij = [&](int i, int j) -> double { return i >= j ? dm[(size_t)i * n + j] : dm[(size_t)j * n + i]; };
-  // the scale of the device check's tolerance: max |P_jk| <= max_j P_jj for a positive
-  // semi-definite P (for any other matrix the check is only the stricter and falls back to the
-  // unfactored one)
-  double dmax = 0.0;
-  for (int j = 0; j < n; ++j) dmax = std::max(dmax, Pij(j, j));
-  const double pmax = dmax;
-  // L row by row (row i at Lr[i * rmax]), so that the dot products run over contiguous memory;
-  // the host buffers are the handle's, reused (no fresh pages per density-matrix change)
-  std::vector<double>& Lr = m->fact_Lr_host;
-  std::vector<double>& d = m->fact_d_host;
-  Lr.assign((size_t)n * rmax, 0.0);
-  d.assign(n, 0.0);
-  for (int j = 0; j < n; ++j) d[j] = Pij(j, j);
-  int r = 0;
-  for (;;) {
-    int jp = 0;
-    for (int j = 1; j < n; ++j)
-      if (d[j] > d[jp]) jp = j;
-    if (!(d[jp] > kFactorTol * dmax)) break;
-    if (r == rmax) return QMT_OK;   // rank too high for the factored path to pay
-    const double piv = std::sqrt(d[jp]), ipiv = 1.0 / piv;
-    const double* lj = Lr.data() + (size_t)jp * rmax;
-    for (int i = 0; i < n; ++i) {
-      const double* li = Lr.data() + (size_t)i * rmax;
-      double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-      int q = 0;
-      for (; q + 4 <= r; q += 4) {
-        a0 += li[q] * lj[q];
-        a1 += li[q + 1] * lj[q + 1];
-        a2 += li[q + 2] * lj[q + 2];
-        a3 += li[q + 3] * lj[q + 3];
-      }
-      for (; q < r; ++q) a0 += li[q] * lj[q];
-      Lr[(size_t)i * rmax + r] = (Pij(i, jp) - ((a0 + a1) + (a2 + a3))) * ipiv;
-    }
-    Lr[(size_t)jp * rmax + r] = piv;
-    for (int i = 0; i < n; ++i) d[i] -= Lr[(size_t)i * rmax + r] * Lr[(size_t)i * rmax + r];
-    d[jp] = 0.0;
-    ++r;
-  }
-  // an indefinite matrix leaves clearly negative diagonal elements behind
-  for (int i = 0; i < n; ++i)
-    if (d[i] < -10.0 * kFactorTol * dmax) return QMT_OK;
-  // refined on the device; what the factor then leaves out, max |P - L L^T|, is checked there too, into
-  // the gate flag and without a round trip: the factored launch runs when it is 0, the unfactored one
-  // when it is 1 (density_tc)
-  const int r16 = std::max(16, (r + 15) / 16 * 16);
-  std::vector<float>& L0 = m->fact_L0_host;
-  L0.assign((size_t)n * r16, 0.f);
-  for (int i = 0; i < n; ++i)
-    for (int q = 0; q < r; ++q) L0[(size_t)i * r16 + q] = (float)Lr[(size_t)i * rmax + q];
-  // device scratch: Y (then L), M, C^T, column maxima and flag, L0
-  const size_t nr = (size_t)n * r16, rr = (size_t)r16 * r16;
-  if ((st = m->d_fact_L.reserve((nr + 2 * rr + r16 + 2) * sizeof(double) + nr * sizeof(float))) ||
-      (st = m->d_fact_scale.reserve(r16 * (sizeof(double) + sizeof(float)))))
+  // device scratch for any rank: L (FP64), Y (then the refined L), M, C^T, column maxima, flag, info, L0
+  const size_t nr = (size_t)n * rmax, rr = (size_t)rmax * rmax;
+  if ((st = m->d_fact_L.reserve((2 * nr + 2 * rr + rmax + 8) * sizeof(double) + nr * sizeof(float))) ||
+      (st = m->d_fact_scale.reserve(rmax * (sizeof(double) + sizeof(float)))))
     return st;
-  double* Y = m->d_fact_L.as<double>();
+  double* Lp = m->d_fact_L.as<double>();
+  double* Y = Lp + nr;
   double* M = Y + nr;
   double* CT = M + rr;
   unsigned long long* colmax = reinterpret_cast<unsigned long long*>(CT + rr);
-  int* flag = reinterpret_cast<int*>(colmax + r16);
-  float* dL0 = reinterpret_cast<float*>(colmax + r16 + 2);
+  int* info = reinterpret_cast<int*>(colmax + rmax);
+  double* dmax = reinterpret_cast<double*>(colmax + rmax + 1);
+  int* flag = reinterpret_cast<int*>(m->d_scalars.as<double>() + 9);   // beside the sum and the give-up flag
+  float* L0 = reinterpret_cast<float*>(colmax + rmax + 8);
   double* two_h = m->d_fact_scale.as<double>();
   const double* P = m->d_P64.as<double>();
-  QMT_CUDA(cudaMemcpyAsync(dL0, L0.data(), nr * sizeof(float), cudaMemcpyHostToDevice, s));
-  QMT_CUDA(cudaMemsetAsync(colmax, 0, (r16 + 2) * sizeof(double), s));
-  fact_y_kernel<<<dim3((n + 31) / 32, (r16 + 31) / 32), 256, 0, s>>>(P, np, dL0, n, r16, Y);
+  QMT_CUDA(cudaMemsetAsync(colmax, 0, (rmax + 8) * sizeof(double), s));
+  QMT_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
+  if ((st = launch_pivot(P, np, n, rmax, Lp, L0, info, dmax, s))) return st;
+  int got[2] = {0, 0};
+  QMT_CUDA(cudaMemcpyAsync(got, info, sizeof(got), cudaMemcpyDeviceToHost, s));
+  QMT_CUDA(cudaStreamSynchronize(s));
+  if (got[1] || got[0] <= 0 || got[0] > factor_rmax(n16, fmt, any_rank)) return QMT_OK;   // rank too high to pay, or indefinite
+  const int r = got[0], r16 = std::max(16, (r + 15) / 16 * 16);
+  // refined on the device; what the factor then leaves out, max |P - L L^T|, is checked there too, into
+  // the gate flag and without a round trip: the factored launch runs when it is 0, the unfactored one
+  // when it is 1 (density_tc)
+  fact_y_kernel<<<dim3((n + 31) / 32, (r16 + 31) / 32), 256, 0, s>>>(P, np, L0, rmax, n, r16, Y);
   QMT_CHECK_LAUNCH("fact_y_kernel");
-  fact_m_kernel<<<dim3(r16 / 16, r16 / 16), 256, 0, s>>>(dL0, Y, n, r16, M);
+  fact_m_kernel<<<dim3(r16 / 16, r16 / 16), 256, 0, s>>>(L0, rmax, Y, n, r16, M);
   QMT_CHECK_LAUNCH("fact_m_kernel");
   const size_t csm = (size_t)r * (r16 + 1) * sizeof(double);
-  const int in_smem = csm <= 200u * 1024u ? 1 : 0;
+  const int in_smem = csm <= 180u * 1024u ? 1 : 0;   // (beside the panel)
   if (in_smem)
-    QMT_CUDA(cudaFuncSetAttribute(fact_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  fact_chol_kernel<<<1, 1024, in_smem ? csm : 0, s>>>(M, r, r16, in_smem, CT);
+    QMT_CUDA(cudaFuncSetAttribute(fact_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024));
+  fact_chol_kernel<<<1, CHOL_THREADS, in_smem ? csm : 0, s>>>(M, r, r16, in_smem, CT);
   QMT_CHECK_LAUNCH("fact_chol_kernel");
-  fact_solve_kernel<<<(n + 3) / 4, 128, 0, s>>>(Y, CT, n, r, r16, m->d_split_scale.as<double>(), colmax);
+  const size_t ssm = (size_t)32 * r16 * sizeof(double);
+  QMT_CUDA(cudaFuncSetAttribute(fact_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                32 * kFactorMaxR16 * (int)sizeof(double)));
+  fact_solve_kernel<<<(n + SOLVE_WARPS - 1) / SOLVE_WARPS, 32 * SOLVE_WARPS, ssm, s>>>(
+      Y, CT, n, r, r16, m->d_split_scale.as<double>(), colmax);
   QMT_CHECK_LAUNCH("fact_solve_kernel");
   fact_scale_kernel<<<1, kFactorMaxR16, 0, s>>>(colmax, r, r16, two_h, reinterpret_cast<float*>(two_h + r16));
   QMT_CHECK_LAUNCH("fact_scale_kernel");
-  {
-    const int64_t tot = (int64_t)n * n;
-    const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
-    fact_residual_kernel<<<std::max(blocks, 1), 256, 0, s>>>(P, np, Y, n, r16, r, kFactorResid * pmax, flag);
-    QMT_CHECK_LAUNCH("fact_residual_kernel");
-    m->fact_gate = flag;
-  }
+  fact_residual_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), 256, 0, s>>>(P, np, Y, n, r16, r, kFactorResid, dmax, flag);
+  QMT_CHECK_LAUNCH("fact_residual_kernel");
+  m->fact_gate = flag;
+  m->fact_ok = -1;
   const size_t total = (size_t)m->fact_units * nsplit * r16 * 32;   // bytes
   if ((st = m->d_fact_B.reserve(total))) return st;
   const int64_t tot = (int64_t)m->fact_units * 16 * r16;

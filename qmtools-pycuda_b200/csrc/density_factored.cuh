@@ -29,8 +29,8 @@ constexpr int kFactorMaxR16 = 256;   // [H0 | S] of the rank's columns fill the 
 
 // Unit tables of the molecule's basis (fs: column scales 2^s_j), once per basis.
 qmt_status ensure_unit_tables(qmt_mol* m, const std::vector<float>& fs, cudaStream_t s);
-// P = L L^T on the host and the split factor on the device; m->fact_rank = 0 when there is none.
-qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, cudaStream_t s);
+// P = L L^T and the split factor (any_rank: of a full-rank matrix too); m->fact_rank = 0 when there is none.
+qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, cudaStream_t s);
 // Descriptor of the molecule in a launch, its tiles starting at global tile `tile0`.
 void fact_mol_desc(const qmt_mol* m, const PointMap& pm, int64_t tile0, int64_t ntiles, float* qube, double outscale,
                    FactMol& d);

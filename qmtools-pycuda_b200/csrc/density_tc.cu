@@ -481,7 +481,6 @@ qmt_status ensure_basis_operands(qmt_mol* m, int K, cudaStream_t s) {
   }
   qmt_status st = m->d_split_scale.reserve(K * sizeof(double));
   if (st) return st;
-  m->split_inv = inv;
   // pageable uploads return once the data is staged, so `inv` may go
   QMT_CUDA(cudaMemcpyAsync(m->d_split_scale.ptr, inv.data(), K * sizeof(double), cudaMemcpyHostToDevice, s));
   if ((st = ensure_mol_tables(m, fs, K, s)) || (st = ensure_unit_tables(m, fs, s))) return st;
@@ -1892,8 +1891,16 @@ static int g_density_path = 0;   // 0 auto, 1 staged, 2 fused, 3 the factored ma
 // would move its results by as much as their error (1e-5).
 constexpr int kFactorAskedRank = 128;    // path 3 asked for by name: at most this rank
 constexpr int kBf16FusedMaxR16 = 64;
-static bool takes_factor(const qmt_mol* m, const TcShape& sh, bool fused) {
-  return m->fact_rank > 0 && (sh.fmt == FMT_F16 || !fused || m->fact_r16 <= kBf16FusedMaxR16);
+// A full-rank matrix (a correlated density) of up to 256 functions is factored too when there are this many
+// tiles of 128 sample points: factoring it costs 0.25 ms more than the split of P (N = 97 to 140), and 148
+// tiles then take 4.3 instead of 9.8 us.  The tile count of the call decides, not what was built before, so
+// that equal calls give equal results.
+constexpr int64_t kAnyRankTiles = 8192;
+static bool any_rank_pays(const TcShape& sh, int64_t ntiles) { return sh.fmt == FMT_F16 && ntiles >= kAnyRankTiles; }
+static bool takes_factor(const qmt_mol* m, const TcShape& sh, bool fused, int64_t ntiles) {
+  if (m->fact_rank <= 0) return false;
+  if (sh.fmt != FMT_F16) return !fused || m->fact_r16 <= kBf16FusedMaxR16;
+  return any_rank_pays(sh, ntiles) || m->fact_rank <= (m->norbs + 15) / 16 * 8;
 }
 
 // The fused path takes fp16/bf16 contractions of up to 320 functions whose tile, stages and tables
@@ -1922,13 +1929,18 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   // the factored matrix when there is one (automatic, or asked for)
   bool fact = false;
   if (sh.fmt != FMT_TF32 && g_density_path != 1 && g_density_path != 2) {
-    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, s))) return st;
-    fact = takes_factor(mol, sh, fused);
-    if (g_density_path == 3 && (!fact || mol->fact_rank > kFactorAskedRank))
+    const bool any = g_density_path == 0 && any_rank_pays(sh, ntiles);
+    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, s))) return st;
+    fact = takes_factor(mol, sh, fused, ntiles);
+    if (g_density_path == 3 && (!fact || mol->fact_rank > std::min(kFactorAskedRank, fused_n16(mol) / 2)))
       return fail(QMT_BAD_ARG, "factored density path needs a positive semi-definite density matrix of low rank");
   }
-  // with a factor, the device check of what it leaves out picks the launch (no host round trip)
-  const int* gate = fact ? mol->fact_gate : nullptr;
+  // The device checks what a factor leaves out.  Once the host has read the check it decides; a call that
+  // returns a sum reads it afterwards and comes back for the unfactored kernel should it have failed; an
+  // asynchronous call before that launches both, and the check picks one on the device.
+  if (fact && mol->fact_ok == 0) fact = false;
+  const bool known = fact && mol->fact_ok == 1, pair = fact && !known && !sum_out;
+  const int* gate = fact && !known ? mol->fact_gate : nullptr;
   if (fact) {
     FactMol d;
     fact_mol_desc(mol, pm, 0, ntiles, qube, outscale, d);
@@ -1936,7 +1948,8 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
                               reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), gate, 0, s)))
       return st;
   }
-  if (fused) {
+  if (fact && !pair) {
+  } else if (fused) {
     if ((st = ensure_fused_operands(mol, precision, sh, s))) return st;
     if (sh.fmt == FMT_F16) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
     else st = run_fused<FMT_BF16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
@@ -1954,7 +1967,7 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   // synchronises anyway) reads it beside the sum and clears it; fully asynchronous calls leave it for
   // the next synchronous call on this molecule.
   if (sum_out) {
-    double h[9];   // [0] sum, [8] flag
+    double h[10];   // [0] sum, [8] give-up flag, [9] the factor's check
     QMT_CUDA(cudaMemcpyAsync(h, mol->d_scalars.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     QMT_CUDA(cudaStreamSynchronize(s));
     *sum_out = h[0];
@@ -1963,6 +1976,13 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
     if (err) {
       QMT_CUDA(cudaMemsetAsync(mol->d_scalars.as<double>() + 8, 0, sizeof(int), s));
       return fail(QMT_CUDA_ERR, "tensor-core density kernel gave up waiting on a barrier");
+    }
+    if (fact && !known) {
+      int refused = 0;
+      std::memcpy(&refused, h + 9, sizeof(refused));
+      mol->fact_ok = refused ? 0 : 1;
+      if (refused)
+        return density_tc(mol, nx, ny, nz, step, ox, oy, oz, subgrid, precision, rescale, qube, sum_out, s);
     }
     if (!std::isfinite(h[0])) return fail(QMT_NAN, "non-finite density sum");
   }
@@ -2136,7 +2156,7 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
     it.fact = false;
     if (path == 3 && it.sh.fmt != FMT_TF32) {   // factored when the matrix has a factor that passes the check
       int gate = 1;
-      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, s))) break;
+      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, any_rank_pays(it.sh, it.ntiles), s))) break;
       if (m->fact_rank > 0) {
         const cudaError_t e1 = cudaMemcpyAsync(&gate, m->fact_gate, sizeof(int), cudaMemcpyDeviceToHost, s);
         const cudaError_t e2 = cudaStreamSynchronize(s);
@@ -2145,7 +2165,8 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
           break;
         }
       }
-      it.fact = gate == 0 && takes_factor(m, it.sh, it.fused);
+      m->fact_ok = m->fact_rank > 0 ? gate == 0 : -1;
+      it.fact = gate == 0 && takes_factor(m, it.sh, it.fused, it.ntiles);
     }
     if ((st = m->d_partials.reserve(it.ntiles * sizeof(double))) || (st = m->d_scalars.reserve(64 * sizeof(double))))
       break;

@@ -45,18 +45,17 @@ struct qmt_mol {
   int fused_prec = -1;          // precision of the fused-path operands below
   qmt::DevBuf d_fused_B;        // scaled density matrix pieces for the fused path (hi then lo)
   qmt::DevBuf d_split_scale;    // 2^-s_j per function for the device split of the density matrix
-  std::vector<double> split_inv; // the same on the host
   int fact_prec = -1;           // precision of the factored-path operands below (-1: not built)
+  bool fact_any_rank = false;   // the rank limit they were built (or refused) with
   int fact_rank = 0;            // rank of the density-matrix factor P = L L^T (0: not factored)
-  std::vector<double> fact_Lr_host, fact_d_host;   // host work buffers of the factorisation
-  std::vector<float> fact_L0_host;
   int fact_r16 = 0;             // the rank rounded up to 16 (the MMA N)
   qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of fact_r16 rows a piece
   qmt::DevBuf d_fact_tab;       // unit and class tables, then the function of each column
   int fact_units = 0;           // units of 16 columns
   size_t fact_col_off = 0;      // byte offset of the column table
-  qmt::DevBuf d_fact_L;         // the factor (FP64, row by row), scratch of its refinement, the flag of the residual check
-  const int* fact_gate = nullptr; // that flag: 0 when the factor reproduces P, 1 when it does not
+  qmt::DevBuf d_fact_L;         // factorisation scratch: the factor (FP64), its refinement, the flag of the residual check
+  const int* fact_gate = nullptr; // device flag: 0 when the factor reproduces P, 1 when it does not
+  int fact_ok = -1;             // the same as last read by the host (1: it does, 0: it does not, -1: not read)
   qmt::DevBuf d_fact_scale;     // per factor column k: 2^h_k (FP64), then 2^-h_k (FP32)
   qmt::DevBuf d_fused_tab;      // fused path: packed shell records, then (alpha, scaled coefficient) pairs
   qmt::DevBuf d_coords, d_types, d_shells, d_alpha, d_coeff, d_alpha64, d_coeff64;
