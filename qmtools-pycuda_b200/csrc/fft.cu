@@ -12,10 +12,11 @@
 //   factors 2, 3, 5, 7), G(0) = voxel-cube average of 1/|r|; G_hat is real and even, so only
 //   its octant [0, M/2]^3 is stored, cached per (M, h, device).
 //
-// 1D transforms are mixed-radix Stockham (self-sorting) FFTs of batches of lines in shared
-// memory, twiddles from a per-length table computed in FP64 on the host; 256- and 128-point
-// lines (the padded axes of 128- and 64-voxel boxes) take register kernels instead (16 x 16 and
-// 16 x 8 four-step, one shared-memory exchange per transform).  A solve is five passes over an
+// 1D transforms are mixed-radix FFTs of batches of lines in shared memory, twiddles from a
+// per-length table computed in FP64 on the host: in place with one butterfly of up to 10 points per
+// thread where the length has no prime above 7, Stockham stages (self-sorting) for the others; 256- and
+// 128-point lines (the padded axes of 128- and 64-voxel boxes) take register kernels instead (16 x 16
+// and 16 x 8 four-step, one shared-memory exchange per transform).  A solve is five passes over an
 // x-fastest complex work grid:
 //   1. x forward, with the RHS assembled on the fly from q and the nuclei (only lines and
 //      elements inside the physical box are non-zero: y < ny, z < nz, x < nx);
@@ -44,6 +45,15 @@ constexpr double PI = 3.14159265358979323846;
 constexpr int FFT_MAXFAC = 16;
 constexpr int FFT_MAXLEN = 2048;
 
+// Plan of the in-place line kernel: radices, and per stage the distance of a butterfly's elements (L over the
+// radices up to and including this one) with its exact multiply-high divisor (as in Plan1D below).
+constexpr int LINE_MAXFAC = 5;
+struct LinePlan {
+  int nfac;               // 0: the length has a prime factor above 7
+  int fac[LINE_MAXFAC], sub[LINE_MAXFAC];
+  unsigned m_sub[LINE_MAXFAC];
+};
+
 struct Plan1D {
   int L;
   int nfac;
@@ -54,9 +64,8 @@ struct Plan1D {
   int ns[FFT_MAXFAC];
   unsigned m_nbf[FFT_MAXFAC], m_ns[FFT_MAXFAC];
   unsigned m_len;   // ceil(2^32 / L)
+  LinePlan lp;
 };
-
-constexpr int FFT_CAND = 24;   // nuclei listed per x line for the right-hand side
 
 __device__ __forceinline__ unsigned fdiv(unsigned n, unsigned m) { return __umulhi(n, m); }
 
@@ -236,6 +245,60 @@ __device__ __forceinline__ float2 load_elem(const PassArgs& a, int64_t base, int
   }
 }
 
+template <int N>
+struct Int { static constexpr int value = N; };
+// ---- right-hand side of an x line (y, z) ----
+__device__ __forceinline__ void load_atoms(const PassArgs& a, float* sat) {
+  for (int i = threadIdx.x; i < a.mol.natoms; i += blockDim.x) {
+    sat[4 * i] = a.mol.coords[3 * i] * (float)R_BOHR;
+    sat[4 * i + 1] = a.mol.coords[3 * i + 1] * (float)R_BOHR;
+    sat[4 * i + 2] = a.mol.coords[3 * i + 2] * (float)R_BOHR;
+    sat[4 * i + 3] = (float)a.mol.types[i];
+  }
+}
+
+__device__ __forceinline__ float electrons_at(const PassArgs& a, int x, int y, int z) {
+  return a.q[x + (int64_t)y * a.nx + (int64_t)z * a.nx * a.ny] / (-a.h_ang * a.h_ang * a.h_ang);
+}
+
+// Adds the Gaussian nuclei to the charge densities rho(line, x) of nb staged lines (y, z).  A warp per line, a
+// nucleus per lane for the (y, z) distance, then the lanes over the voxels within the cut-off in x; an element
+// stays with one lane and the nuclei come in their order.  With every voxel's thread running over a list of its line's
+// nuclei, and a thread per line making that list, the nuclei were half of this pass (20 of them, 168^3: 35 of 93 us).
+template <class Rho>
+__device__ __forceinline__ void add_nuclei(const PassArgs& a, const float* sat, int nb, const int* ly, const int* lz,
+                                           Rho rho) {
+  const int lane = threadIdx.x & 31;
+  const float cut = sqrtf(a.cut2) * 1.0001f;
+  for (int b = threadIdx.x >> 5; b < nb; b += blockDim.x >> 5) {
+    const float py = a.oy + (ly[b] + 0.5f) * a.h_ang, pz = a.oz + (lz[b] + 0.5f) * a.h_ang;
+    for (int at0 = 0; at0 < a.mol.natoms; at0 += 32) {
+      const int mine = at0 + lane;
+      bool near = false;
+      if (mine < a.mol.natoms) {
+        const float cy = py - sat[4 * mine + 1], cz = pz - sat[4 * mine + 2];
+        near = cy * cy + cz * cz <= a.cut2 * 1.0001f;   // superset of the per-voxel test below
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, near); m; m &= m - 1) {
+        const float* c = sat + 4 * (at0 + __ffs(m) - 1);
+        const float cy = py - c[1], cz = pz - c[2], mid = (c[0] - a.ox) / a.h_ang - 0.5f, half = cut / a.h_ang + 1.f;
+        const int lo = (int)fminf(fmaxf(floorf(mid - half), 0.f), (float)a.nx);
+        const int hi = (int)fmaxf(fminf(ceilf(mid + half), (float)(a.nx - 1)), -1.f);
+        for (int x = (lo & ~31) + lane; x <= hi; x += 32) {
+          const float cx = a.ox + (x + 0.5f) * a.h_ang - c[0];
+          const float r2 = cx * cx + cy * cy + cz * cz;
+          if (x >= lo && r2 <= a.cut2) rho(b, x) += c[3] * a.norm * expf(-r2 * a.i2s2);
+        }
+      }
+    }
+  }
+}
+
+// Charge density to the right-hand side that is transformed.
+__device__ __forceinline__ float rhs_of(const PassArgs& a, float rho) {
+  return a.periodic ? (float)(-(double)rho / EPS0) : rho * a.h_ang * a.h_ang * a.h_ang;
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
   extern __shared__ float2 fsm[];
@@ -246,12 +309,7 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
   float* sat = reinterpret_cast<float*>(b1 + (size_t)a.B * L);   // atoms (PASS_X_RHS)
   for (int i = threadIdx.x; i < L; i += blockDim.x) tw[i] = a.tw[i];
   if constexpr (MODE == PASS_X_RHS) {
-    for (int i = threadIdx.x; i < a.mol.natoms; i += blockDim.x) {
-      sat[4 * i] = a.mol.coords[3 * i] * (float)R_BOHR;
-      sat[4 * i + 1] = a.mol.coords[3 * i + 1] * (float)R_BOHR;
-      sat[4 * i + 2] = a.mol.coords[3 * i + 2] * (float)R_BOHR;
-      sat[4 * i + 3] = (float)a.mol.types[i];
-    }
+    load_atoms(a, sat);
   }
   const int64_t l0 = (int64_t)blockIdx.x * a.B;
   const int64_t rem = a.nlines - l0;
@@ -260,8 +318,6 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
   // per-line data, computed once per CTA (B <= 16 lines)
   __shared__ int64_t lbase[16];          // element 0 of the line in the work grid / output
   __shared__ int lx[16], ly[16];         // the line's two grid coordinates (RHS, multiply, output)
-  __shared__ int ncand[16];              // RHS: nuclei within the cut-off of the line, or -1 for all
-  __shared__ int cand[16][FFT_CAND];
   __syncthreads();   // twiddles and nuclei are in shared memory
   if (threadIdx.x < nb) {
     const int b = threadIdx.x;
@@ -270,19 +326,6 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
     lx[b] = c0;
     ly[b] = c1;
     lbase[b] = (int64_t)c0 * a.s1 + (int64_t)c1 * a.s2;
-    if constexpr (MODE == PASS_X_RHS) {
-      // line (y = c0, z = c1) along x: keep the nuclei whose (y, z) distance passes the cut-off
-      const float py = a.oy + (c0 + 0.5f) * a.h_ang, pz = a.oz + (c1 + 0.5f) * a.h_ang;
-      int cnt = 0;
-      for (int at = 0; at < a.mol.natoms; ++at) {
-        const float cy = py - sat[4 * at + 1], cz = pz - sat[4 * at + 2];
-        if (cy * cy + cz * cz <= a.cut2 * 1.0001f) {   // superset of the per-point test below
-          if (cnt < FFT_CAND) cand[b][cnt] = at;
-          ++cnt;
-        }
-      }
-      ncand[b] = cnt <= FFT_CAND ? cnt : -1;
-    }
   }
   __syncthreads();
   // ---- load ----
@@ -290,19 +333,7 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
     float2 v = make_float2(0.f, 0.f);
     if (e < a.lload) {
       if constexpr (MODE == PASS_X_RHS) {
-        const int y = lx[b], z = ly[b], x = e;
-        const float px = a.ox + (x + 0.5f) * a.h_ang, py = a.oy + (y + 0.5f) * a.h_ang,
-                    pz = a.oz + (z + 0.5f) * a.h_ang;
-        float rho = a.q[x + (int64_t)y * a.nx + (int64_t)z * a.nx * a.ny] / (-a.h_ang * a.h_ang * a.h_ang);
-        const int nc = ncand[b];
-        const int cnt = nc < 0 ? a.mol.natoms : nc;
-        for (int c = 0; c < cnt; ++c) {
-          const int at = nc < 0 ? c : cand[b][c];
-          const float cx = px - sat[4 * at], cy = py - sat[4 * at + 1], cz = pz - sat[4 * at + 2];
-          const float r2 = cx * cx + cy * cy + cz * cz;
-          if (r2 <= a.cut2) rho += sat[4 * at + 3] * a.norm * expf(-r2 * a.i2s2);
-        }
-        v.x = a.periodic ? (float)(-(double)rho / EPS0) : rho * a.h_ang * a.h_ang * a.h_ang;
+        v.x = electrons_at(a, e, lx[b], ly[b]);
       } else {
         v = load_elem<MODE>(a, lbase[b], e);
       }
@@ -319,6 +350,12 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
       for (int e = threadIdx.x; e < L; e += blockDim.x) load_one(b, e);
   }
   __syncthreads();
+  if constexpr (MODE == PASS_X_RHS) {
+    add_nuclei(a, sat, nb, lx, ly, [&](int b, int x) -> float& { return b0[b * L + x].x; });
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb * L; i += blockDim.x) b0[i].x = rhs_of(a, b0[i].x);
+    __syncthreads();
+  }
   float2* res;
   fft_lines_smem(b0, b1, a.plan, nb, tw, a.inv != 0, &res);
   if constexpr (MODE == PASS_Z_MUL) {
@@ -357,6 +394,305 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const PassArgs a) {
   } else {
     for (int b = 0; b < nb; ++b)
       for (int e = threadIdx.x; e < a.lstore; e += blockDim.x) store_one(b, e);
+  }
+}
+
+// ---- lines in place, one butterfly per thread ------------------------------------------------
+//
+// Lengths whose primes are 2, 3, 5 and 7 (every padded axis).  B = 16 lines per CTA (4 above 704 points, so that
+// an SM holds two blocks), stored element by element with the lines side by side, B + 1 float2 apart: a half-warp
+// reads one element of 16 lines, so global rows are 128 bytes, shared memory has no bank conflicts, a twiddle is
+// one broadcast and the butterfly index needs no division by B.  The radices go up to 10 (12 and 16 save some
+// lengths a stage, but their registers cost a block per SM: 100^3 padded 115 -> 137 us), a length takes two or three
+// stages, and the stages are decimation in frequency in place: one buffer and one barrier each.  The first stage
+// reads its elements from the grid and the last writes to it at the digit-reversed frequency; the z pass multiplies
+// by the kernel in the registers of the last stage, which are the inputs of the first stage back (the transposed
+// algorithm, frequencies in the same digit-reversed places), so a three-stage line crosses shared memory four times
+// there and back instead of fourteen.  Inverse transforms swap the two components on the way in and out.
+// Bound by issue (57 % of the slots in the z pass) and by the latency of the first loads.  Padded solves, kernels
+// alone, before and after: 88 x 104 x 96 182 -> 85 us, 168^3 1021 -> 334 us, 48^3 64 -> 44 us.
+template <int N>
+struct Roots {   // cos and sin of 2 pi k / N
+  float c[N], s[N];
+  __host__ __device__ constexpr Roots() : c{}, s{} {
+    for (int k = 0; k < N; ++k) {
+      // series at an angle folded to [-pi, pi]
+      const double x = 2 * PI * (2 * k > N ? k - N : k) / N;
+      double t = 1, cs = 0, sn = 0;
+      for (int i = 0; i < 40; i += 2) {
+        cs += t;
+        sn += t * x / (i + 1);
+        t *= -x * x / ((i + 1) * (i + 2));
+      }
+      c[k] = (float)cs;
+      s[k] = (float)sn;
+    }
+  }
+};
+
+template <int R>
+__device__ __forceinline__ void dft(float2 (&v)[R]);
+
+// R = N1 N2 points as N2 transforms of N1 points and N1 of N2.
+template <int N1, int N2>
+__device__ __forceinline__ void dft_split(float2 (&v)[N1 * N2]) {
+  constexpr int R = N1 * N2;
+  constexpr Roots<R> w;
+  float2 u[N2][N1];
+#pragma unroll
+  for (int b = 0; b < N2; ++b) {
+#pragma unroll
+    for (int i = 0; i < N1; ++i) u[b][i] = v[N2 * i + b];
+    dft<N1>(u[b]);
+#pragma unroll
+    for (int k = 1; k < N1; ++k) {
+      if (b * k == 0) continue;
+      if (4 * b * k == R) u[b][k] = make_float2(u[b][k].y, -u[b][k].x);
+      else u[b][k] = cmul(u[b][k], make_float2(w.c[b * k % R], -w.s[b * k % R]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < N1; ++k) {
+    float2 z[N2];
+#pragma unroll
+    for (int b = 0; b < N2; ++b) z[b] = u[b][k];
+    dft<N2>(z);
+#pragma unroll
+    for (int b = 0; b < N2; ++b) v[k + N1 * b] = z[b];
+  }
+}
+
+// Forward R-point DFT in registers, natural order.
+template <int R>
+__device__ __forceinline__ void dft(float2 (&v)[R]) {
+  if constexpr (R == 2) {
+    const float2 t = v[0];
+    v[0] = cadd(t, v[1]);
+    v[1] = csub(t, v[1]);
+  } else if constexpr (R == 4) {
+    const float2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]), t2 = cadd(v[1], v[3]), t3 = csub(v[1], v[3]);
+    v[0] = cadd(t0, t2);
+    v[2] = csub(t0, t2);
+    v[1] = make_float2(t1.x + t3.y, t1.y - t3.x);
+    v[3] = make_float2(t1.x - t3.y, t1.y + t3.x);
+  } else if constexpr (R == 3 || R == 5 || R == 7) {
+    // elements k and R - k share their cosines and their sines up to the sign
+    constexpr Roots<R> w;
+    constexpr int H = (R - 1) / 2;
+    float2 t[H], d[H], x0 = v[0];
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      t[k] = cadd(v[k + 1], v[R - 1 - k]);
+      d[k] = csub(v[k + 1], v[R - 1 - k]);
+      v[0] = cadd(v[0], t[k]);
+    }
+#pragma unroll
+    for (int q = 1; q <= H; ++q) {
+      float2 e = x0, o = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+        const float c = w.c[(k + 1) * q % R], sn = w.s[(k + 1) * q % R];
+        e = make_float2(e.x + c * t[k].x, e.y + c * t[k].y);
+        o = make_float2(o.x + sn * d[k].x, o.y + sn * d[k].y);
+      }
+      v[q] = make_float2(e.x + o.y, e.y - o.x);
+      v[R - q] = make_float2(e.x - o.y, e.y + o.x);
+    }
+  } else if constexpr (R == 6) dft_split<3, 2>(v);
+  else if constexpr (R == 8) dft_split<4, 2>(v);
+  else if constexpr (R == 9) dft_split<3, 3>(v);
+  else if constexpr (R == 10) dft_split<5, 2>(v);
+}
+
+__device__ __forceinline__ float2 swapped(float2 v) { return make_float2(v.y, v.x); }
+
+template <int MODE, int B>
+__global__ void __launch_bounds__(256, 4) fft_line_kernel(const PassArgs a) {
+  extern __shared__ float2 fsm[];
+  constexpr int P = B + 1, lb = B == 16 ? 4 : 2;
+  const int L = a.plan.L, T = blockDim.x, nf = a.plan.lp.nfac;
+  const int Rl = a.plan.lp.fac[nf - 1], Nl = L / Rl;
+  float2* const tw = fsm;
+  float2* const buf = fsm + L;
+  unsigned short* const rev = reinterpret_cast<unsigned short*>(buf + (size_t)L * P);   // frequency of block p
+  unsigned short* const place = rev + L;   // where frequency e stands in the buffer
+  float* const sat = reinterpret_cast<float*>(place + L);   // atoms (PASS_X_RHS); 2 L shorts before it
+  for (int i = threadIdx.x; i < L; i += T) tw[i] = a.tw[i];
+  if constexpr (MODE == PASS_X_RHS) load_atoms(a, sat);
+  for (int p = threadIdx.x; p < Nl; p += T) {
+    int k = 0, w = 1, pos = p * Rl;
+    for (int i = 0; i < nf - 1; ++i) {
+      const int d = (int)fdiv((unsigned)pos, a.plan.lp.m_sub[i]);
+      pos -= d * a.plan.lp.sub[i];
+      k += d * w;
+      w *= a.plan.lp.fac[i];
+    }
+    rev[p] = (unsigned short)k;
+    if constexpr (MODE == PASS_PLAIN || MODE == PASS_X_RHS)
+      for (int m = 0; m < Rl; ++m) place[k + m * Nl] = (unsigned short)(p * Rl + m);
+  }
+  const unsigned l0 = blockIdx.x * B, rem = (unsigned)a.nlines - l0;   // at most 2048^2 lines
+  const int nb = rem < B ? (int)rem : B;
+  __shared__ int64_t lbase[B];          // element 0 of the line in the work grid
+  __shared__ int lx[B], ly[B];          // the line's two grid coordinates
+  if (threadIdx.x < nb) {
+    const int i = threadIdx.x;
+    const unsigned l = l0 + i, c1 = l / (unsigned)a.n1, c0 = l - c1 * (unsigned)a.n1;
+    lx[i] = (int)c0;
+    ly[i] = (int)c1;
+    lbase[i] = (int64_t)c0 * a.s1 + (int64_t)c1 * a.s2;
+  }
+  __syncthreads();
+  const bool inv = a.inv != 0;
+  const bool adjacent = a.s1 == 1;
+  const int b = threadIdx.x & (B - 1);   // the blocks are multiples of 32 threads
+  const bool live = b < nb;
+  float2* const line = MODE == PASS_X_RHS ? nullptr : a.data + (live ? lbase[b] : 0);
+
+  // a stage of radix R: Load(element) and Store(element, butterfly, digit, value)
+  auto stage = [&](auto rc, int i, bool down, auto load, auto store) {
+    constexpr int R = decltype(rc)::value;
+    const int sub = a.plan.lp.sub[i], ts = L / (sub * R), items = (L / R) << lb;
+    const unsigned msub = a.plan.lp.m_sub[i];
+    for (int w = threadIdx.x; w < items; w += T) {
+      const int it = w >> lb, p = sub == 1 ? it : (int)fdiv((unsigned)it, msub), j = it - p * sub;
+      const int base = p * sub * R + j;
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = load(base + q * sub);
+      if (!down && sub > 1) {
+#pragma unroll
+        for (int q = 1; q < R; ++q) v[q] = cmul(v[q], tw[j * q * ts]);
+      }
+      dft<R>(v);
+      if (down && sub > 1) {
+#pragma unroll
+        for (int q = 1; q < R; ++q) v[q] = cmul(v[q], tw[j * q * ts]);
+      }
+#pragma unroll
+      for (int q = 0; q < R; ++q) store(base + q * sub, it, q, v[q]);
+    }
+  };
+  auto with_radix = [&](int i, auto f) {
+    switch (a.plan.lp.fac[i]) {
+      case 2: f(Int<2>()); break;
+      case 3: f(Int<3>()); break;
+      case 4: f(Int<4>()); break;
+      case 5: f(Int<5>()); break;
+      case 6: f(Int<6>()); break;
+      case 7: f(Int<7>()); break;
+      case 8: f(Int<8>()); break;
+      case 9: f(Int<9>()); break;
+      default: f(Int<10>()); break;
+    }
+    __syncthreads();
+  };
+  auto from_buf = [&](int e) { return buf[e * P + b]; };
+  auto to_buf = [&](int e, int, int, float2 v) { buf[e * P + b] = v; };
+
+  // ---- first stage, or the lines into the buffer where they are not side by side in the grid ----
+  int i0 = 0;   // first stage still to do
+  if (MODE == PASS_X_RHS || !adjacent) {
+    auto put = [&](int bb, int e, float2 v) { buf[e * P + bb] = inv ? swapped(v) : v; };
+    const float2 zero = make_float2(0.f, 0.f);
+    constexpr int AHEAD = B < 8 ? B : 8;   // reads in flight per thread
+    for (int e = threadIdx.x; e < L; e += T)
+      for (int b0 = 0; b0 < B; b0 += AHEAD) {
+        float2 v[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+          v[u] = zero;
+          if (b0 + u < nb && e < a.lload) {
+            if constexpr (MODE == PASS_X_RHS) v[u].x = electrons_at(a, e, lx[b0 + u], ly[b0 + u]);
+            else v[u] = load_elem<MODE>(a, lbase[b0 + u], e);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) put(b0 + u, e, v[u]);
+      }
+    __syncthreads();
+    if constexpr (MODE == PASS_X_RHS) {
+      add_nuclei(a, sat, nb, lx, ly, [&](int bb, int x) -> float& { return buf[x * P + bb].x; });
+      __syncthreads();
+      auto from_rho = [&](int e) { return make_float2(rhs_of(a, buf[e * P + b].x), 0.f); };
+      with_radix(0, [&](auto rc) { stage(rc, 0, true, from_rho, to_buf); });
+      i0 = 1;
+    }
+  } else if constexpr (MODE == PASS_PLAIN || MODE == PASS_Z_MUL) {
+    auto from_grid = [&](int e) {
+      float2 v = make_float2(0.f, 0.f);
+      if (live && e < a.lload) v = line[(int64_t)e * a.se];
+      return inv ? swapped(v) : v;
+    };
+    with_radix(0, [&](auto rc) { stage(rc, 0, true, from_grid, to_buf); });
+    i0 = 1;
+  }
+  const bool staged_out = MODE == PASS_X_RHS || (MODE == PASS_PLAIN && !adjacent);
+  for (int i = i0; i < nf - (staged_out ? 0 : 1); ++i)
+    with_radix(i, [&](auto rc) { stage(rc, i, true, from_buf, to_buf); });
+
+  auto to_grid = [&](int e, float2 v) {
+    if (inv) v = swapped(v);
+    if (live && e < a.lstore) line[(int64_t)e * a.se] = make_float2(v.x * a.scale, v.y * a.scale);
+  };
+  if constexpr (MODE == PASS_X_RHS || MODE == PASS_PLAIN) {
+    if (staged_out) {
+      for (int bb = 0; bb < nb; ++bb)
+        for (int e = threadIdx.x; e < a.lstore; e += T) {
+          float2 v = buf[place[e] * P + bb];
+          if (inv) v = swapped(v);
+          a.data[lbase[bb] + (int64_t)e * a.se] = make_float2(v.x * a.scale, v.y * a.scale);
+        }
+      return;
+    }
+  }
+  if constexpr (MODE == PASS_PLAIN) {
+    with_radix(nf - 1, [&](auto rc) {
+      stage(rc, nf - 1, true, from_buf, [&](int, int it, int q, float2 v) { to_grid(rev[it] + q * Nl, v); });
+    });
+  } else if constexpr (MODE == PASS_X_OUT) {
+    // line (z = lx, y = ly) along x into the C-order output: adjacent lines are adjacent in z
+    const int64_t row = (int64_t)a.ny * a.nz;
+    float* const out = a.out + (live ? (int64_t)ly[b] * a.nz + lx[b] : 0);
+    with_radix(nf - 1, [&](auto rc) {
+      stage(rc, nf - 1, true, from_buf, [&](int, int it, int q, float2 v) {
+        const int e = rev[it] + q * Nl;
+        if (live && e < a.lstore) out[e * row] = (inv ? v.y : v.x) * a.scale;
+      });
+    });
+  } else if constexpr (MODE == PASS_Z_MUL) {
+    const int hx = a.Mx / 2 + 1, hy = a.My / 2 + 1;
+    const int x = live ? lx[b] : 0, y = live ? ly[b] : 0;
+    const float* const g =
+        a.periodic ? nullptr : a.gsym + min(x, a.Mx - x) + (int64_t)hx * min(y, a.My - y);
+    const int64_t gz = (int64_t)hx * hy;
+    with_radix(nf - 1, [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      for (int w = threadIdx.x; w < Nl << lb; w += T) {
+        const int it = w >> lb, k0 = rev[it];
+        float2 v[R];
+        float f[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          const int kz = k0 + q * Nl;
+          f[q] = a.periodic ? periodic_factor(a, x, y, kz) : __ldg(g + gz * min(kz, L - kz));
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = from_buf(it * R + q);
+        dft<R>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = make_float2(v[q].y * f[q], v[q].x * f[q]);   // swapped for the way back
+        dft<R>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) to_buf(it * R + q, 0, 0, v[q]);
+      }
+    });
+    for (int i = nf - 2; i > 0; --i)
+      with_radix(i, [&](auto rc) { stage(rc, i, false, from_buf, to_buf); });
+    auto back = [&](int e, float2 v) { to_grid(e, swapped(v)); };
+    with_radix(0, [&](auto rc) {
+      stage(rc, 0, false, from_buf, [&](int e, int, int, float2 v) { back(e, v); });
+    });
   }
 }
 
@@ -490,20 +826,13 @@ __global__ void __launch_bounds__(256) fft_reg_pass_kernel(const PassArgs a) {
   float* sat = reinterpret_cast<float*>(buf + LINES * RegFft<L>::S_MAX);   // atoms (PASS_X_RHS)
   for (int i = threadIdx.x; i < L; i += blockDim.x) tw[i] = a.tw[i];
   if constexpr (MODE == PASS_X_RHS) {
-    for (int i = threadIdx.x; i < a.mol.natoms; i += blockDim.x) {
-      sat[4 * i] = a.mol.coords[3 * i] * (float)R_BOHR;
-      sat[4 * i + 1] = a.mol.coords[3 * i + 1] * (float)R_BOHR;
-      sat[4 * i + 2] = a.mol.coords[3 * i + 2] * (float)R_BOHR;
-      sat[4 * i + 3] = (float)a.mol.types[i];
-    }
+    load_atoms(a, sat);
   }
   const int64_t l0 = (int64_t)blockIdx.x * LINES;
   const int64_t rem = a.nlines - l0;
   const int nb = rem < LINES ? (int)rem : LINES;
   __shared__ int64_t lbase[LINES];
   __shared__ int lx[LINES], ly[LINES];
-  __shared__ int ncand[LINES];
-  __shared__ int cand[LINES][FFT_CAND];
   __syncthreads();
   if (threadIdx.x < nb) {
     const int bb = threadIdx.x;
@@ -512,18 +841,6 @@ __global__ void __launch_bounds__(256) fft_reg_pass_kernel(const PassArgs a) {
     lx[bb] = c0;
     ly[bb] = c1;
     lbase[bb] = (int64_t)c0 * a.s1 + (int64_t)c1 * a.s2;
-    if constexpr (MODE == PASS_X_RHS) {
-      const float py = a.oy + (c0 + 0.5f) * a.h_ang, pz = a.oz + (c1 + 0.5f) * a.h_ang;
-      int cnt = 0;
-      for (int at = 0; at < a.mol.natoms; ++at) {
-        const float cy = py - sat[4 * at + 1], cz = pz - sat[4 * at + 2];
-        if (cy * cy + cz * cz <= a.cut2 * 1.0001f) {
-          if (cnt < FFT_CAND) cand[bb][cnt] = at;
-          ++cnt;
-        }
-      }
-      ncand[bb] = cnt <= FFT_CAND ? cnt : -1;
-    }
   }
   __syncthreads();
   // lines adjacent in memory: a half-warp spans 16 lines at one element; lines contiguous: it
@@ -534,30 +851,24 @@ __global__ void __launch_bounds__(256) fft_reg_pass_kernel(const PassArgs a) {
   const int S = RegFft<L>::S(bfast);
   const bool live = b < nb;
   float2 x[16];
+  if constexpr (MODE == PASS_X_RHS) {
+    float* const rho = reinterpret_cast<float*>(buf);   // line b, voxel e at b (L + 1) + e
 #pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const int e = t + TPL * m;
-    float2 v = make_float2(0.f, 0.f);
-    if (live && e < a.lload) {
-      if constexpr (MODE == PASS_X_RHS) {
-        const int y = lx[b], z = ly[b], xx = e;
-        const float px = a.ox + (xx + 0.5f) * a.h_ang, py = a.oy + (y + 0.5f) * a.h_ang,
-                    pz = a.oz + (z + 0.5f) * a.h_ang;
-        float rho = a.q[xx + (int64_t)y * a.nx + (int64_t)z * a.nx * a.ny] / (-a.h_ang * a.h_ang * a.h_ang);
-        const int nc = ncand[b];
-        const int cnt = nc < 0 ? a.mol.natoms : nc;
-        for (int c = 0; c < cnt; ++c) {
-          const int at = nc < 0 ? c : cand[b][c];
-          const float cx = px - sat[4 * at], cy = py - sat[4 * at + 1], cz = pz - sat[4 * at + 2];
-          const float r2 = cx * cx + cy * cy + cz * cz;
-          if (r2 <= a.cut2) rho += sat[4 * at + 3] * a.norm * expf(-r2 * a.i2s2);
-        }
-        v.x = a.periodic ? (float)(-(double)rho / EPS0) : rho * a.h_ang * a.h_ang * a.h_ang;
-      } else {
-        v = load_elem<MODE>(a, lbase[b], e);
-      }
+    for (int m = 0; m < 16; ++m) {
+      const int e = t + TPL * m;
+      rho[b * (L + 1) + e] = live && e < a.lload ? electrons_at(a, e, lx[b], ly[b]) : 0.f;
     }
-    x[m] = v;
+    __syncthreads();
+    add_nuclei(a, sat, nb, lx, ly, [&](int bb, int e) -> float& { return rho[bb * (L + 1) + e]; });
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; ++m) x[m] = make_float2(rhs_of(a, rho[b * (L + 1) + t + TPL * m]), 0.f);
+  } else {
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int e = t + TPL * m;
+      x[m] = live && e < a.lload ? load_elem<MODE>(a, lbase[b], e) : make_float2(0.f, 0.f);
+    }
   }
   fft_regs<L>(x, tw, buf, b, t, S, a.inv != 0);
   if constexpr (MODE == PASS_Z_MUL) {
@@ -715,14 +1026,56 @@ static qmt_status launch_pass_reg(int mode, PassArgs a, cudaStream_t s) {
   }
 }
 
+template <int MODE, int B>
+static qmt_status launch_mode_lines(const PassArgs& a, unsigned blocks, int threads, size_t smem, cudaStream_t s) {
+  QMT_CUDA(cudaFuncSetAttribute(fft_line_kernel<MODE, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fft_line_kernel<MODE, B><<<blocks, threads, smem, s>>>(a);
+  QMT_CHECK_LAUNCH("fft_line_kernel");
+  return QMT_OK;
+}
+
+template <int B>
+static qmt_status launch_pass_lines(int mode, const PassArgs& a, cudaStream_t s) {
+  const int L = a.plan.L;
+  size_t smem = (size_t)L * ((2 + B) * sizeof(float2) + 2 * sizeof(unsigned short));
+  if (mode == PASS_X_RHS) smem += 16 * (size_t)a.mol.natoms;
+  const unsigned blocks = (unsigned)((a.nlines + B - 1) / B);
+  if (blocks == 0) return QMT_OK;
+  // the block size that leaves the fewest threads idle in the last round of each stage; four blocks of at least
+  // 192 (with 128 and fewer idle threads a 336-point solve took 393 us, with these 334)
+  int threads = 256, best = 1 << 30;
+  for (int t = 256; t >= 192; t -= 32) {
+    int cost = 0;
+    for (int i = 0; i < a.plan.lp.nfac; ++i) {
+      const int items = L / a.plan.lp.fac[i] * B;
+      cost += (items + t - 1) / t * t * a.plan.lp.fac[i];
+    }
+    if (cost < best) {
+      best = cost;
+      threads = t;
+    }
+  }
+  switch (mode) {
+    case PASS_PLAIN: return launch_mode_lines<PASS_PLAIN, B>(a, blocks, threads, smem, s);
+    case PASS_X_RHS: return launch_mode_lines<PASS_X_RHS, B>(a, blocks, threads, smem, s);
+    case PASS_Z_MUL: return launch_mode_lines<PASS_Z_MUL, B>(a, blocks, threads, smem, s);
+    default: return launch_mode_lines<PASS_X_OUT, B>(a, blocks, threads, smem, s);
+  }
+}
+
 static qmt_status launch_pass(int mode, PassArgs a, cudaStream_t s) {
   a.B = std::max(1, std::min(16, 12288 / a.plan.L));
   const float2* tw;
   qmt_status st = twiddles(a.plan.L, &tw);
   if (st) return st;
   a.tw = tw;
-  if (a.plan.L == 256) return launch_pass_reg<256>(mode, a, s);   // register kernels
+  // Register kernels for their two lengths (128^3 padded 125 us; the in-place kernel takes 190).  The in-place
+  // kernel where there are two stages to take (88 x 104 x 96 padded: 181 us by the kernel below, 85 by it); a single
+  // radix, up to 10 points, gains nothing there (3 x 2 x 2: 19 us below, 26), and other primes need it.
+  if (a.plan.L == 256) return launch_pass_reg<256>(mode, a, s);
   if (a.plan.L == 128) return launch_pass_reg<128>(mode, a, s);
+  if (a.plan.lp.nfac > 1)
+    return a.plan.L <= 704 ? launch_pass_lines<16>(mode, a, s) : launch_pass_lines<4>(mode, a, s);
   size_t smem = ((size_t)a.plan.L * (1 + 2 * a.B)) * sizeof(float2);
   if (mode == PASS_X_RHS) smem += 16 * (size_t)a.mol.natoms;
   const unsigned blocks = (unsigned)((a.nlines + a.B - 1) / a.B);
@@ -733,6 +1086,39 @@ static qmt_status launch_pass(int mode, PassArgs a, cudaStream_t s) {
     case PASS_Z_MUL: return launch_mode<PASS_Z_MUL>(a, blocks, smem, s);
     default: return launch_mode<PASS_X_OUT>(a, blocks, smem, s);
   }
+}
+
+// Fewest stages of radices up to 10, then the smallest sum of the radices (work per element); larger radices
+// first.  No plan (nfac 0) if the length has another prime.
+static LinePlan line_plan(int L) {
+  constexpr int radices[] = {10, 9, 8, 7, 6, 5, 4, 3, 2};
+  LinePlan best{};
+  int best_sum = 0, pick[LINE_MAXFAC];
+  auto search = [&](auto&& self, int left, int depth, int first, int sum) -> void {
+    if (left == 1) {
+      if (best.nfac == 0 || depth < best.nfac || sum < best_sum) {
+        best.nfac = depth;
+        best_sum = sum;
+        std::copy(pick, pick + depth, best.fac);
+      }
+      return;
+    }
+    const int limit = best.nfac ? best.nfac : LINE_MAXFAC;
+    if (depth == limit) return;
+    for (int i = first; i < (int)(sizeof(radices) / sizeof(int)); ++i)
+      if (left % radices[i] == 0) {
+        pick[depth] = radices[i];
+        self(self, left / radices[i], depth + 1, i, sum + radices[i]);
+      }
+  };
+  search(search, L, 0, 0, 0);
+  int n = L;
+  for (int i = 0; i < best.nfac; ++i) {
+    n /= best.fac[i];
+    best.sub[i] = n;
+    best.m_sub[i] = n > 1 ? (unsigned)(((1ull << 32) + (uint64_t)n - 1) / (uint64_t)n) : 0u;
+  }
+  return best;
 }
 
 static qmt_status plan_of(int L, Plan1D& p) {
@@ -748,6 +1134,7 @@ static qmt_status plan_of(int L, Plan1D& p) {
     p.m_ns[i] = ns > 1 ? (unsigned)(((1ull << 32) + (uint64_t)ns - 1) / (uint64_t)ns) : 0u;
     ns *= p.fac[i];
   }
+  p.lp = line_plan(L);
   return QMT_OK;
 }
 

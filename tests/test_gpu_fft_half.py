@@ -1,4 +1,4 @@
-"""The half-spectrum FFT Poisson solve on odd and ragged lengths, against numpy.fft restatements.
+"""The half-spectrum FFT Poisson solve on odd, ragged and long lengths, against numpy.fft restatements.
 
 The x spectrum of a real right-hand side is kept up to Mx / 2.  That leans on the k-space factor being even,
 which the reference's frequency rule (kernel_fft.cu:90-104) is not on odd axes: it takes (N - 1) / 2 as a negative
@@ -60,3 +60,10 @@ def test_periodic_odd_lengths(basis, shape):
 def test_padded_ragged_lengths(basis, shape):
     """2 * 37 = 74 is padded to 75, an odd length; the rest mixes the radices 2, 3, 5 and 7."""
     assert rel_l2(*_solve(basis, shape, True)) < TOL
+
+
+@pytest.mark.parametrize("shape", [(4, 6, 10), (11, 22, 13), (12, 14, 15), (49, 5, 81), (704, 4, 12), (12, 720, 4),
+                                   (4, 12, 1715), (1875, 2, 12), (2, 2048, 17), (40, 36, 127)])
+def test_periodic_line_plans(basis, shape):
+    """One stage to five, every radix, 16 and 4 lines per block, remainders of lines, and lengths with other primes."""
+    assert rel_l2(*_solve(basis, shape, False)) < TOL
