@@ -19,19 +19,20 @@
 //     warps run the epilogue of the previous tile from TMEM meanwhile.
 //
 // Split products: T = A_hi L_hi (main, "H") + A_hi L_lo + A_lo L_hi (small, "S"; with bf16 pieces also
-// A_lo L_lo, 2^-16 of the main term), in two accumulators: the tensor core's FP32 additions round toward
-// zero by 2^-24 of the accumulator, so the small terms stay out of the large one's way.
+// A_lo L_lo, 2^-16 of the main term), in separate accumulators: the tensor core's FP32 additions round toward
+// zero by 2^-24 of the accumulator, so the small terms stay out of the large one's way, and the large ones take
+// turns on up to three (fact_mol_desc): without rescaling N = 294 is 4e-7 off FP64 with three, 7e-7 with one, for
+// 0.02 of 0.53 ms.
 //
 // Bound: the hand-over of K-steps (waits, commits, the issuing threads' serial code: ~420 clocks per
 // unit with the MMAs, ~340 without production, ~370 without MMAs) and the producers' issue slots; DRAM
 // idle, tensor pipe 20-45% busy.  Measured (B200, fp16x3, one call, before -> now; before: a resident
 // Phi' tile per CTA for N <= 320 and rank <= 64, Phi' through HBM beyond, no factor past rank 128):
-//   N = 294,  rank 59,  128^3 points:  1.48 -> 0.51 ms
-//   N = 588,  rank 119, 192^3 points:  11.2 -> 3.8 ms
+//   N = 294,  rank 59,  128^3 points:  1.48 -> 0.53 ms
+//   N = 588,  rank 119, 192^3 points:  11.2 -> 4.0 ms
 //   N = 1176, rank 238, 168^3 points:  42.9 -> 6.3 ms (the factor's 1.3 MB per tile from L2: 7.5 TB/s)
 // Tried and dropped: pairing hi and lo factor rows in one MMA of N = 2 r16 (overlapping accumulators,
-// +8%); one MMA-issuing lane outside a converged warp (~900 clocks per K-step); K-steps of a tile over
-// three H accumulators (no gain in error once the factor is refined, half the TMEM buffering); 16
+// +8%); one MMA-issuing lane outside a converged warp (~900 clocks per K-step); 16
 // producer warps of 80 registers (same); 128-byte swizzled A reads (same).
 //
 // Replaces the per-voxel pair loop of gpu_densityqube_shmem_subgrid (kernel_density.cu:74-140).
@@ -438,10 +439,10 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
     if (!ok) break;
     last_sets = sets;
     tc_fence_after();
-    const uint32_t S = d0 + r16;
+    const uint32_t na = (uint32_t)M.na, S = d0 + na * r16;
     const uint32_t idesc = make_idesc(p.fmt, 128, r16);
     const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * r16 * 32u, half = r16 * 32u;
-    uint32_t acc = 0;
+    uint32_t acc = 0, ha = 0;   // accumulated before; H accumulator of the next unit (in turn)
     uint32_t bres = smem_u32(res);
     for (int u0 = 0; u0 < nunits; u0 += GROUP) {
       ok = (ready || mbar_wait_warp(&B.a_full[s], ph, &B.abort_flag, p.wait_ns)) &&
@@ -458,7 +459,7 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
         if (u0 + k < nunits) {
           const uint64_t ahi = sw32_desc(a), bhi = sw32_desc(b);
           if (MAIN) {
-            if (leader) mma_f16(d0, ahi, bhi, idesc, acc);
+            if (leader) mma_f16(d0 + ha * r16, ahi, bhi, idesc, acc);
           } else {
             const uint64_t alo = sw32_desc(a + PIECE), blo = sw32_desc(b + half);
             if (leader) {
@@ -467,7 +468,10 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
               if (FMT == 1) mma_f16(S, alo, blo, idesc, 1u);
             }
           }
-          acc = 1u;
+          if (!MAIN || ++ha == na) {
+            acc = 1u;
+            ha = 0;
+          }
           a += UNIT_A;
           b += blk;
         }
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
       uint32_t ha[16], la[16], hb[16], lb[16];
       auto load = [&](int c, uint32_t(&h)[16], uint32_t(&l)[16]) {
         tmem_ld16_issue(base + (uint32_t)c, h);
-        if (TWO) tmem_ld16_issue(base + (uint32_t)(r16 + c), l);
+        if (TWO) tmem_ld16_issue(base + (uint32_t)(M.na * r16 + c), l);
       };
       auto square = [&](int c, uint32_t(&h)[16], uint32_t(&l)[16]) {
         f2 sq = 0ull;
@@ -653,16 +657,36 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
         tmem_ld16_wait(h);
         if (TWO) tmem_ld16_wait(l);
       };
-      load(0, ha, la);
+      if (M.na > 1) {
+        // several H accumulators: their sum takes the registers of the second block of columns
 #pragma unroll 1
-      for (int c = 0; c < r16; c += 32) {
-        arrived(ha, la);
-        if (c + 16 < r16) load(c + 16, hb, lb);
-        square(c, ha, la);
-        if (c + 16 < r16) {
-          arrived(hb, lb);
-          if (c + 32 < r16) load(c + 32, ha, la);
-          square(c + 16, hb, lb);
+        for (int c = 0; c < r16; c += 16) {
+          load(c, ha, la);
+          tmem_ld16_issue(base + (uint32_t)(r16 + c), hb);
+          if (M.na > 2) tmem_ld16_issue(base + (uint32_t)(2 * r16 + c), lb);
+          arrived(ha, la);
+          tmem_ld16_wait(hb);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) ha[j] = __float_as_uint(__uint_as_float(ha[j]) + __uint_as_float(hb[j]));
+          if (M.na > 2) {
+            tmem_ld16_wait(lb);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) ha[j] = __float_as_uint(__uint_as_float(ha[j]) + __uint_as_float(lb[j]));
+          }
+          square(c, ha, la);
+        }
+      } else {
+        load(0, ha, la);
+#pragma unroll 1
+        for (int c = 0; c < r16; c += 32) {
+          arrived(ha, la);
+          if (c + 16 < r16) load(c + 16, hb, lb);
+          square(c, ha, la);
+          if (c + 16 < r16) {
+            arrived(hb, lb);
+            if (c + 32 < r16) load(c + 32, ha, la);
+            square(c + 16, hb, lb);
+          }
         }
       }
       tc_fence_before();
@@ -1446,6 +1470,10 @@ void fact_mol_desc(const qmt_mol* m, const PointMap& pm, int64_t tile0, int64_t 
   d.nunits = m->fact_units;
   d.r16 = m->fact_r16;
   d.sets = 2 * d.r16 <= 256 ? 2 : 1;
+  // The tensor core's additions truncate, so every K-step takes about 2^-24 of T away and the squares double that:
+  // a uniform loss, which only rescaling hides.  Units in turn on up to three accumulators divide it by as many where
+  // two buffers hold them (a third buffer's worth of TMEM is not given up for it).
+  d.na = d.sets == 2 ? std::clamp(256 / d.r16 - 1, 1, std::min(3, d.nunits)) : 1;
   d.B = m->d_fact_B.as<uint8_t>();
   d.units = m->d_fact_tab.as<int4>();
   d.coords = m->d_coords.as<float>();

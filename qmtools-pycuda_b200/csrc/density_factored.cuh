@@ -15,7 +15,8 @@ struct FactMol {
   int64_t tile0, ntiles;
   int nunits;              // K-steps (units of 16 columns)
   int r16;                 // rank rounded up to 16
-  int sets;                // TMEM buffers of [H | S]: two (2 r16 <= 256 columns each) or one
+  int sets;                // TMEM buffers of [H.. | S]: two (2 r16 <= 256 columns each) or one
+  int na;                  // H accumulators: up to three where two buffers hold them, else one
   const uint8_t* B;        // factor blocks (fact_split_kernel)
   const int4* units;       // unit and class tables
   const float* coords;
