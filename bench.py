@@ -29,8 +29,8 @@ Beside the headline step, rank 0 also reports (not part of `value`):
   * `c2_sweep`: the large molecule (60 atoms, N = 588) on 192^3 at 0.12 bohr, the density in
     every precision, and an FP32 Jacobi solve to a relative FP64 residual of 1e-8;
   * `batched`: 64 molecules of 5-60 atoms (grids = bounding box + 3 bohr per side at
-    0.15 bohr) in one CUDA graph (one persistent fused density launch for the molecules with
-    N <= 320, autotuned paths and FFT lengths), against the plain FP32 single-molecule path;
+    0.15 bohr) in one CUDA graph (one persistent density launch for the factored molecules,
+    autotuned paths for the others and FFT lengths), against the plain FP32 single-molecule path;
   * `serving`: Poisson request streams at 50, 200 and 800 req/s (atoms log-uniform 3-120)
     through the engine with p50/p99 latency, against serial plain FP32;
   * `cpu_baseline`: the FP64 NumPy/SciPy evaluation on a bounded sample;
@@ -44,9 +44,9 @@ total and rescale, periodic cuFFT Poisson route), plus its analytic potential
 (gpu_hartree_GTO) and Jacobi sweeps (gpu_hartree_iteration) on the small molecule's 64^3
 grid.  Without those builds the FP64 CPU port of its algorithm is timed instead.
 
-`--ncu-import CSV` turns an ncu metrics capture of the fused density kernel
+`--ncu-import CSV` turns an ncu metrics capture of the factored density kernel
 (`--metrics dram__bytes_read.sum,dram__bytes_write.sum --csv`) into
-profiles/density_fused_kernel_c1.traffic.json, which the bench reads for `roofline.traffic`.
+profiles/density_factored_kernel_c1.traffic.json, which the bench reads for `roofline.traffic`.
 """
 import argparse
 import json
@@ -335,8 +335,8 @@ def _engine_run(serving, reqs, slots, precision, realtime):
 
 def batched(basis, qmtools, N, precision, reps=5):
     """The batch workload (64 molecules, 5-60 atoms, grids = bounding box + 3 bohr per side at
-    0.15 bohr) through BatchEvaluator, all in one CUDA graph: fused density launches for the
-    molecules with N <= 320, the staged path for the rest, Hockney solves with tuned padding;
+    0.15 bohr) through BatchEvaluator, all in one CUDA graph: one density launch for the factored
+    molecules, the fused and staged paths for the rest, Hockney solves with tuned padding;
     against the plain FP32 single-molecule path (SIMT FP32 density + Hockney solve per molecule,
     handles built beforehand).  Device time with CUDA events.  Two graphs: `value` with every
     molecule's factored density matrix (factors built and checked when the batch is created,
@@ -432,7 +432,7 @@ def batched(basis, qmtools, N, precision, reps=5):
                     "h2d_bytes": int(sum(d.numel() * 4 for d in dms)), "d2h_bytes": int(v_host.numel() * 4)},
             "serial_plain_fp32": {"value": pts / (ms32 / 1e3), "ms": ms32},
             "speedup_vs_serial_plain_fp32": ms32 / ms, "speedup_e2e_vs_serial_plain_fp32": ms32 / ms_e2e,
-            "design": f"one CUDA graph per batch: persistent fused density launches over the tiles of "
+            "design": f"one CUDA graph per batch: persistent density launches over the tiles of "
                       f"{fact_info['fused_molecules']} molecules (factored density matrices), the staged "
                       f"path for the other {len(bm) - fact_info['fused_molecules']} "
                       f"({fact_info['factored_molecules']} of 64 factored in all), rescale, 64 Hockney "
@@ -728,14 +728,15 @@ def run_ours(args, world, rank, local, pg):
     frank = int(frank.value)
     r16 = max(16, (frank + 15) // 16 * 16)
     out["roofline"] = {"bound": "tensor",
-                       "kernel": "density_fused_kernel (basis values in shared memory + tcgen05 contraction)",
+                       "kernel": ("density_factored_kernel" if frank else "density_fused_kernel") +
+                                 " (basis values in shared memory + tcgen05 contraction)",
                        "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s", "frac": achieved / peak_tf,
                        "peak_source": f"bf16_tflops burst, {kind}", "density_ms": dens_ms,
                        "algorithmic_flop_per_launch": flops,
                        "algorithmic_flop_definition": "npts (2 N^2 + 2 N): Phi P plus the row-dot",
                        "contraction": (f"factored density matrix P = L L^T, rank {frank}: rho = sum_k (Phi L)_k^2, "
-                                       f"MMA N = {2 * r16} (hi and lo rows of L) x 2 products, "
-                                       f"{npts * 2.0 * nb * 2 * r16 * 2:.3e} tensor flop per launch"
+                                       f"MMA N = {r16} x 3 products (large and small in two accumulators), "
+                                       f"{npts * 2.0 * nb * r16 * 3:.3e} tensor flop per launch"
                                        if frank else "unfactored: Phi P (N columns) x 3 products, row-dot with Phi"),
                        "traffic": traffic["bytes_per_launch"] if traffic else None,
                        "traffic_unit": "DRAM bytes per launch (ncu, dram__bytes_read.sum + dram__bytes_write.sum)",
@@ -918,11 +919,11 @@ def gto_boundary(basis, qmtools, N, s, reps=3):
             "achieved_tflops": flops / (ms / 1e3) / 1e12}
 
 
-TRAFFIC_JSON = ROOT / "profiles" / "density_fused_kernel_c1.traffic.json"
+TRAFFIC_JSON = ROOT / "profiles" / "density_factored_kernel_c1.traffic.json"
 
 
 def profiled_traffic():
-    """DRAM bytes (read + write) per launch of the fused density kernel at the bench size, from
+    """DRAM bytes (read + write) per launch of the factored density kernel at the bench size, from
     the machine-written summary of an ncu metrics capture (`--ncu-import`), or None."""
     if not TRAFFIC_JSON.exists():
         return None
@@ -939,7 +940,7 @@ def ncu_import(csv_path, command):
     scale = {"byte": 1, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "KB": 1e3, "MB": 1e6, "GB": 1e9}
     per = {}
     for r in rows:
-        if "density_fused_kernel" not in r["Kernel Name"]:
+        if "density_factored_kernel" not in r["Kernel Name"]:
             continue
         if r["Metric Name"] not in ("dram__bytes_read.sum", "dram__bytes_write.sum"):
             continue
@@ -947,10 +948,10 @@ def ncu_import(csv_path, command):
         per.setdefault(r["ID"], {})[r["Metric Name"]] = v
     launches = [d for d in per.values() if len(d) == 2]
     if not launches:
-        raise SystemExit("no density_fused_kernel launch with both DRAM metrics in " + str(csv_path))
+        raise SystemExit("no density_factored_kernel launch with both DRAM metrics in " + str(csv_path))
     rd = float(np.mean([d["dram__bytes_read.sum"] for d in launches]))
     wr = float(np.mean([d["dram__bytes_write.sum"] for d in launches]))
-    out = {"kernel": "density_fused_kernel", "launches": len(launches), "dram_bytes_read": rd,
+    out = {"kernel": "density_factored_kernel", "launches": len(launches), "dram_bytes_read": rd,
            "dram_bytes_write": wr, "bytes_per_launch": rd + wr, "command": command}
     TRAFFIC_JSON.write_text(json.dumps(out, indent=1) + "\n")
     print(json.dumps(out))
@@ -1146,7 +1147,7 @@ def main():
     ap.add_argument("--quick", action="store_true", help="headline step only (no plain-FP32, batch, serving)")
     ap.add_argument("--grid", type=int, default=0, help="cube edge of a smaller grid for the same molecule")
     ap.add_argument("--only", default="", choices=["", "jacobi", "gto"], help="run one kernel family alone (profiling)")
-    ap.add_argument("--ncu-import", default="", help="ncu --csv metrics capture of the fused density kernel "
+    ap.add_argument("--ncu-import", default="", help="ncu --csv metrics capture of the factored density kernel "
                                                      "to summarise into profiles/ (no GPU needed)")
     ap.add_argument("--ncu-command", default="", help="the command line of that capture (recorded beside it)")
     args = ap.parse_args()

@@ -5,10 +5,9 @@ reference evaluates one molecule per facade call, qmtools/qmtools.py:2381-2639).
 
 * keeps every molecule's operands, its density grid and its potential grid on the device (one
   flat buffer each, 256-byte aligned slices);
-* evaluates all densities through `qmt_batch_density`: the molecules whose contraction takes the
-  fused path share persistent launches over all their tiles (one for those whose density matrix
-  has a low-rank factor, one for the others), the rest take the staged path; every grid is then
-  scaled to its nuclear charge;
+* evaluates all densities through `qmt_batch_density`: the molecules whose density matrix has a
+  low-rank factor share one persistent launch over all their tiles, the others with N <= 320 a second
+  one, the rest take the staged path; every grid is then scaled to its nuclear charge;
 * solves the free-space (Hockney) FFT Poisson problem of every molecule with the padded lengths
   the autotuner picked (`qmtools.autotune`);
 * captures all of it into one CUDA graph after a first eager run (which builds every operand,
@@ -50,9 +49,8 @@ class BatchEvaluator:
         total = int(self.offsets[-1])
         self.q = torch.zeros(total, dtype=torch.float32, device="cuda")
         self.v = torch.zeros(total, dtype=torch.float32, device="cuda") if hartree else None
-        # tuned choices; every molecule takes its factored density matrix when it has one, on the
-        # fused path when it fits (a batch that re-derives its operands in the graph keeps the
-        # unfactored matrices)
+        # tuned choices; every molecule takes its factored density matrix when it has one (a batch
+        # that re-derives its operands in the graph keeps the unfactored matrices)
         from .autotune import PATH_FACTORED
         self.paths = [self.tuner.density_path(m, n, precision) for m, n in zip(self.molecules, self.npts)]
         if not self.refresh and not precision.startswith("tf32"):
