@@ -920,7 +920,7 @@ struct PivotArgs {
   double tol;
   double* L;                  // n x rmax, FP64 (used when the rows do not fit in shared memory)
   float* L0;                  // n x ld0, FP32, zero beyond the rank up to a multiple of 16
-  int ld0;
+  int ld0;                    // (at least rmax rounded up to 16)
   int* info;
   double* dmax;               // the first pivot
 };
@@ -1307,8 +1307,8 @@ constexpr double kFactorResid = 2e-7;
 
 }  // namespace
 
-static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double* L, float* L0, int* info, double* dmax,
-                               cudaStream_t s) {
+static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double* L, float* L0, int ld0, int* info,
+                               double* dmax, cudaStream_t s) {
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1324,7 +1324,7 @@ static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double*
     a.tol = kFactorTol;
     a.L = L;
     a.L0 = L0;
-    a.ld0 = rmax;
+    a.ld0 = ld0;
     a.info = info;
     a.dmax = dmax;
     const size_t base = (size_t)(a.rows + rmax) * sizeof(double), rows = (size_t)a.rows * a.ld * sizeof(double);
@@ -1398,36 +1398,40 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   // the nuclear charge for N_e (ions of up to 16 charges allowed for) a rank above rmax is known
   // without factoring
   if (0.5 * m->qtot > rmax + 8) return QMT_OK;
-  // device scratch for any rank: L (FP64), Y (then the refined L), M, C^T, column maxima, flag, info, L0
-  const size_t nr = (size_t)n * rmax, rr = (size_t)rmax * rmax;
-  if ((st = m->d_fact_L.reserve((2 * nr + 2 * rr + rmax + 8) * sizeof(double) + nr * sizeof(float))) ||
-      (st = m->d_fact_scale.reserve(rmax * (sizeof(double) + sizeof(float)))))
+  // device scratch for any rank: L (FP64), Y (then the refined L), M, C^T, column maxima, flag, info, L0.  The
+  // kernels work on whole blocks of 16 columns, so it is sized by the rank limit rounded up to them (n16 / 2 is an
+  // odd multiple of 8 for every second n16).
+  const int rbuf = (rmax + 15) / 16 * 16;
+  const size_t nr = (size_t)n * rbuf, rr = (size_t)rbuf * rbuf;
+  if ((st = m->d_fact_L.reserve((2 * nr + 2 * rr + rbuf + 8) * sizeof(double) + nr * sizeof(float))) ||
+      (st = m->d_fact_scale.reserve(rbuf * (sizeof(double) + sizeof(float)))))
     return st;
   double* Lp = m->d_fact_L.as<double>();
   double* Y = Lp + nr;
   double* M = Y + nr;
   double* CT = M + rr;
   unsigned long long* colmax = reinterpret_cast<unsigned long long*>(CT + rr);
-  int* info = reinterpret_cast<int*>(colmax + rmax);
-  double* dmax = reinterpret_cast<double*>(colmax + rmax + 1);
+  int* info = reinterpret_cast<int*>(colmax + rbuf);
+  double* dmax = reinterpret_cast<double*>(colmax + rbuf + 1);
   int* flag = reinterpret_cast<int*>(m->d_scalars.as<double>() + 9);   // beside the sum and the give-up flag
-  float* L0 = reinterpret_cast<float*>(colmax + rmax + 8);
+  float* L0 = reinterpret_cast<float*>(colmax + rbuf + 8);
   double* two_h = m->d_fact_scale.as<double>();
   const double* P = m->d_P64.as<double>();
-  QMT_CUDA(cudaMemsetAsync(colmax, 0, (rmax + 8) * sizeof(double), s));
+  QMT_CUDA(cudaMemsetAsync(colmax, 0, (rbuf + 8) * sizeof(double), s));
   QMT_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
-  if ((st = launch_pivot(P, np, n, rmax, Lp, L0, info, dmax, s))) return st;
+  if ((st = launch_pivot(P, np, n, rmax, Lp, L0, rbuf, info, dmax, s))) return st;
   int got[2] = {0, 0};
   QMT_CUDA(cudaMemcpyAsync(got, info, sizeof(got), cudaMemcpyDeviceToHost, s));
   QMT_CUDA(cudaStreamSynchronize(s));
   if (got[1] || got[0] <= 0 || got[0] > factor_rmax(n16, fmt, any_rank)) return QMT_OK;   // rank too high to pay, or indefinite
   const int r = got[0], r16 = std::max(16, (r + 15) / 16 * 16);
+  if (r16 > rbuf) return fail(QMT_BAD_ARG, "factor rank beyond its workspace");
   // refined on the device; what the factor then leaves out, max |P - L L^T|, is checked there too, into
   // the gate flag and without a round trip: the factored launch runs when it is 0, the unfactored one
   // when it is 1 (density_tc)
-  fact_y_kernel<<<dim3((n + 31) / 32, (r16 + 31) / 32), 256, 0, s>>>(P, np, L0, rmax, n, r16, Y);
+  fact_y_kernel<<<dim3((n + 31) / 32, (r16 + 31) / 32), 256, 0, s>>>(P, np, L0, rbuf, n, r16, Y);
   QMT_CHECK_LAUNCH("fact_y_kernel");
-  fact_m_kernel<<<dim3(r16 / 16, r16 / 16), 256, 0, s>>>(L0, rmax, Y, n, r16, M);
+  fact_m_kernel<<<dim3(r16 / 16, r16 / 16), 256, 0, s>>>(L0, rbuf, Y, n, r16, M);
   QMT_CHECK_LAUNCH("fact_m_kernel");
   const size_t csm = (size_t)r * (r16 + 1) * sizeof(double);
   const int in_smem = csm <= 180u * 1024u ? 1 : 0;   // (beside the panel)
