@@ -1124,7 +1124,7 @@ def run_reference(args, world, rank, local, pg):
     for _ in range(args.warmup):
         cpu_baseline_c1(sm, basis, qmtools)
     for _ in range(args.steps):
-        samples.append(cpu_baseline_c1(sm, basis, qmtools))
+        samples.append(cpu_baseline_c1(sm, basis, qmtools)[0])
     v = float(np.median([s["value"] for s in samples]))
     cb = dict(samples[0])
     cb["value"] = v
