@@ -1900,7 +1900,10 @@ static bool any_rank_pays(const TcShape& sh, int64_t ntiles) { return sh.fmt == 
 static bool takes_factor(const qmt_mol* m, const TcShape& sh, bool fused, int64_t ntiles) {
   if (m->fact_rank <= 0) return false;
   if (sh.fmt != FMT_F16) return !fused || m->fact_r16 <= kBf16FusedMaxR16;
-  return any_rank_pays(sh, ntiles) || m->fact_rank <= (m->norbs + 15) / 16 * 8;
+  // (a call on a small grid does not factor a molecule whose charge rules out a rank of half of N, and so leaves alone
+  // what a call on a large one has factored)
+  const int half = (m->norbs + 15) / 16 * 8;
+  return any_rank_pays(sh, ntiles) || (m->fact_rank <= half && 0.5 * m->qtot <= std::max(16, half) + 8);
 }
 
 // The fused path takes fp16/bf16 contractions of up to 320 functions whose tile, stages and tables

@@ -1,0 +1,54 @@
+"""Densities whose matrix is factored because of the size of the grid: from 8192 tiles of 128 sample points on, any
+positive semi-definite matrix of up to 256 functions."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import qmtools
+from qmtools import _native as N
+
+pytestmark = pytest.mark.gpu
+
+SMALL, LARGE = (24, 16, 16), (104, 104, 104)     # 48 and 8788 tiles
+
+
+def _molecule(basis, zs, matrix, seed=0):
+    """`matrix`(n, generator) -> the density matrix."""
+    rng = np.random.default_rng(seed)
+    k = int(np.ceil(len(zs) ** (1 / 3)))
+    pos = np.array([(x, y, z) for x in range(k) for y in range(k) for z in range(k)][:len(zs)]) * 1.4
+    rows = [[int(z), *(float(v) for v in p)] for z, p in zip(zs, pos + rng.uniform(-0.1, 0.1, pos.shape))]
+    n = sum(sum(2 * L + 1 for L, _, _ in basis.shells64[z]) for z in zs)
+    return qmtools.Molecule(rows, matrix(n, rng), basis)
+
+
+def _low_rank(rank):
+    def m(n, rng):
+        c = np.linalg.qr(rng.standard_normal((n, rank)))[0]
+        return c @ c.T
+    return m
+
+
+def _density(mol, shape, prec, subgrid=1):
+    import torch
+    span = float(np.ptp(np.asarray(mol.coords), axis=0).max()) + 6.0
+    h = span / max(shape)
+    org = [float(o) for o in np.asarray(mol.coords).mean(axis=0) - np.array(shape) * h / 2]
+    q = torch.empty(int(np.prod(shape)), device="cuda")
+    s = C.c_double()
+    N.ensure_device()
+    N.call("qmt_density", mol.handle, *shape, h, *org, subgrid, N.PREC[prec], 0, C.c_void_p(q.data_ptr()), C.byref(s),
+           N.stream_handle())
+    return q
+
+
+def test_equal_calls_give_equal_results(basis):
+    """A molecule whose charge rules out a rank of half of N (nine bromine atoms: 157 electron pairs, 243 functions) with
+    a matrix of low rank all the same: a small grid's result does not depend on a large one's call before it."""
+    import torch
+    mol = _molecule(basis, [35] * 9, _low_rank(40))
+    before = _density(mol, SMALL, "fp16x3")
+    _density(mol, LARGE, "fp16x3")
+    assert torch.equal(_density(mol, SMALL, "fp16x3"), before)
+    mol.release()
