@@ -114,14 +114,16 @@ qmt_status qmt_density(qmt_mol* mol, int nx, int ny, int nz, float step,
  * factored density matrix when it has one; else fused when the contraction is fp16/bf16 and
  * N <= 320, staged otherwise), 1 = staged (basis values through HBM), 2 = fused (basis values
  * stay in shared memory), 3 = the factored density matrix: P = L L^T from a pivoted Cholesky
- * factorisation (FP64, on the host, once per matrix; refined on the device) and
- * rho = sum_k (Phi L)_k^2, which needs rank(P) columns instead of N -- for a positive
- * semi-definite P of rank at most min(128, N/2) (an SCF density matrix has the rank of its
- * occupied orbitals) and fp16 / bf16 contractions; QMT_BAD_ARG when the factorisation finds P
- * indefinite or of higher rank.  (The automatic choice factors up to min(256, N/2) with fp16x3; bf16
- * up to rank 64 when N <= 320, else min(128, N/2).)  What the factor leaves out is checked on
- * the device (max |P - L L^T| <= 2e-7 max |P|), which runs the unfactored kernel instead when the
- * check fails, without a host round trip. */
+ * factorisation (FP64, on the device, once per matrix) and rho = sum_k (Phi L)_k^2, which needs
+ * rank(P) columns instead of N -- for a positive semi-definite P of rank at most min(128, N/2) (an
+ * SCF density matrix has the rank of its occupied orbitals) and fp16 / bf16 contractions;
+ * QMT_BAD_ARG when the factorisation finds P indefinite or of higher rank, for which the first call
+ * with a matrix waits.  The automatic choice factors up to rank min(256, N/2) with fp16x3 and fp16,
+ * and any rank of up to 256 functions from 8192 tiles of 128 sample points on; bf16 up to rank 64
+ * when N <= 320, else min(128, N/2).  What the factor leaves out is checked on the device
+ * (max |P - L L^T| <= 2e-7 max |P|).  The automatic choice never waits for the rank or the check: a
+ * call that returns a sum reads both, and an asynchronous one that finds them undecided launches
+ * both kernels, of which the device's decision runs one. */
 qmt_status qmt_set_density_path(int mode);
 
 /* Rank of the factor the last density call on `mol` contracted with (new): 0 when it ran the

@@ -14,9 +14,9 @@
 //     third of the production time);
 //   * items are numbered across tiles and taken from one counter: the warps run ahead into the next
 //     tiles as far as the ring and the positions allow, with no barrier among them;
-//   * one thread issues the MMAs unit by unit, one thread streams the factor's K-step blocks (or loads
-//     them once when they fit beside the ring), two warps compute the tiles' sample positions, and four
-//     warps run the epilogue of the previous tile from TMEM meanwhile.
+//   * one thread streams the factor's K-step blocks (or loads them once when they fit beside the ring), two
+//     warps issue the MMAs unit by unit (the large products and the small ones), one warp computes the tiles'
+//     sample positions, and four warps run the epilogue of the previous tile from TMEM meanwhile.
 //
 // Split products: T = A_hi L_hi (main, "H") + A_hi L_lo + A_lo L_hi (small, "S"; with bf16 pieces also
 // A_lo L_lo, 2^-16 of the main term), in separate accumulators: the tensor core's FP32 additions round toward
@@ -50,10 +50,12 @@ using namespace sm100;
 
 namespace {
 
+// Whose tiles a launch walks: one molecule's, several molecules', or one's whose rank only the device knows.
+enum { ONE = 0, MANY = 1, ON_DEVICE = 2 };
 enum { UNIT_GENERIC = 0, UNIT_S3S1P1 = 1, UNIT_S8S8S1P3P1D1 = 2 };
 
 constexpr int NPW = 12;                        // producer warps
-constexpr int FACT_THREADS = (8 + NPW) * 32;   // copy, MMA, 2 position warps; 4 epilogue warps; producers
+constexpr int FACT_THREADS = (8 + NPW) * 32;   // copy, 2 MMA warps, positions; 4 epilogue warps; producers
 constexpr int GROUP = 2;                       // units per ring slot: one wait and one commit for both
 constexpr int MIN_SLOTS = 4, MAX_SLOTS = 12;
 constexpr int MIN_UNITS = 2;                   // units of a tile (a smaller molecule gets an empty one)
@@ -73,7 +75,6 @@ struct FactParams {
   const FactMol* mols;     // device array of nmol molecules
   int nmol;
   int64_t ntiles;
-  int nsplit;
   uint32_t fmt;
   uint32_t nslots;         // ring slots
   uint32_t slot_magic;     // ceil(2^32 / nslots): group / nslots = umulhi(group, magic) below 2^28
@@ -81,9 +82,29 @@ struct FactParams {
   uint32_t resident;       // the whole factor behind the ring, loaded once (single molecule)
   int* err;
   uint64_t wait_ns;
-  const int* gate;
-  int gate_want;
+  const FactShape* shape;  // ON_DEVICE: the device's decision (the factor is streamed)
 };
+
+__host__ __device__ inline FactShape fact_shape(int rank, int nunits) {
+  FactShape f;
+  f.refused = rank <= 0;
+  f.r16 = rank > 16 ? (rank + 15) / 16 * 16 : 16;
+  f.sets = 2 * f.r16 <= 256 ? 2 : 1;
+  // The tensor core's additions truncate, so every K-step takes about 2^-24 of T away and the squares double that:
+  // a uniform loss, which only rescaling hides.  Units in turn on up to three accumulators divide it by as many where
+  // two buffers hold them (a third buffer's worth of TMEM is not given up for it).
+  int na = f.sets == 2 ? 256 / f.r16 - 1 : 1;
+  if (na > 3) na = 3;
+  if (na > nunits) na = nunits;
+  f.na = na < 1 ? 1 : na;
+  return f;
+}
+
+template <int WHO>
+__device__ __forceinline__ FactShape fact_shape_of(const FactParams& p, const FactMol& m) {
+  if (WHO == ON_DEVICE) return *p.shape;
+  return FactShape{0, m.r16, m.sets, m.na};
+}
 
 template <bool MULTI>
 __device__ __forceinline__ const FactMol& fact_mol(const FactParams& p, int64_t t) {
@@ -239,7 +260,7 @@ struct Disp {
 };
 
 // Displacement of the lane's two rows from an atom, correct to one FP32 rounding without FP64: the
-// positions come as hi + lo with hi a multiple of 2^-12 bohr (make_positions), the nuclear
+// positions come as hi + lo with hi a multiple of 2^-12 bohr (split_pos), the nuclear
 // coordinate is split the same way (adding and subtracting 3 * 2^10 rounds it to 2^-12), so the
 // difference of the hi parts is exact.
 __device__ __forceinline__ f2 disp1(const float4 p, float a) {
@@ -415,23 +436,26 @@ struct FactBars {
 // a warp of its own: a thread spends about 110 clocks on each MMA with new operands (waits, descriptors,
 // issue) whatever its N, more than the 58 to 128 the tensor core takes, and the two accumulator chains
 // never meet.
-template <int FMT, bool TWO, bool MULTI, bool MAIN>
+template <int FMT, bool TWO, int WHO, bool MAIN>
 __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint8_t* smem, uint8_t* res, uint32_t tmem) {
+  constexpr bool MULTI = WHO == MANY;
   uint32_t s = 0, ph = 0, tile_it = 0;   // slot and its phase
   int last_sets = 2;
   const bool leader = elect_one();
-  const bool streamed = MULTI || !p.resident;
+  const bool streamed = WHO != ONE || !p.resident;
   const uint32_t ring0 = smem_u32(smem);
   constexpr uint32_t UNIT_A = TWO ? 2 * PIECE : PIECE, ABYTES = GROUP * UNIT_A;
   bool ok = true, ready = false;
+  FactShape f = fact_shape_of<WHO>(p, p.one);
   if (!streamed) ok = mbar_wait_warp(&B.res_bar, 0u, &B.abort_flag, p.wait_ns);
   for (int64_t t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x, ++tile_it) {
     const FactMol& M = fact_mol<MULTI>(p, t);
     const int nunits = M.nunits;
-    const uint32_t r16 = (uint32_t)M.r16;
+    if (MULTI) f = fact_shape_of<WHO>(p, M);
+    const uint32_t r16 = (uint32_t)f.r16;
     // TMEM: a half per tile in turn, or (sets == 1) all of it; the tiles whose columns this one
     // overwrites must have been read
-    const int sets = M.sets;
+    const int sets = f.sets;
     const uint32_t set = tile_it & 1u, d0 = tmem + (sets == 2 ? set * 256u : 0u);
     if (tile_it >= 2) ok = mbar_wait_warp(&B.t_empty[set], ((tile_it - 2u) >> 1) & 1u, &B.abort_flag, p.wait_ns);
     if (ok && tile_it >= 1 && (sets == 1 || last_sets == 1))
@@ -439,7 +463,7 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
     if (!ok) break;
     last_sets = sets;
     tc_fence_after();
-    const uint32_t na = (uint32_t)M.na, S = d0 + na * r16;
+    const uint32_t na = (uint32_t)f.na, S = d0 + na * r16;
     const uint32_t idesc = make_idesc(p.fmt, 128, r16);
     const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * r16 * 32u, half = r16 * 32u;
     uint32_t acc = 0, ha = 0;   // accumulated before; H accumulator of the next unit (in turn)
@@ -499,10 +523,11 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
 }  // namespace
 
 // One persistent CTA per SM walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ...
-template <int FMT, bool TWO, bool MULTI>
+template <int FMT, bool TWO, int WHO>
 __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const __grid_constant__ FactParams p) {
+  constexpr bool MULTI = WHO == MANY;
   extern __shared__ uint8_t smem_dyn[];
-  if (p.gate && *p.gate != p.gate_want) return;   // the other launch of the pair does the work
+  if (WHO == ON_DEVICE && p.shape->refused) return;   // the unfactored launch of the pair does the work
   __shared__ FactBars B;
   __shared__ __align__(16) float4 pos_s[POS_DEPTH][3][64];   // {hi r, hi r + 64, lo r, lo r + 64}
   __shared__ double rho_s[128];
@@ -549,7 +574,7 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
   if (warp == 0) {
     // ---- the factor's K-step blocks ------------------------------------------------------------
     if (lane == 0) {
-      if (!MULTI && p.resident) {
+      if (WHO == ONE && p.resident) {
         const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * (uint32_t)p.one.r16 * 32u;
         mbar_expect_tx(&B.res_bar, blk * (uint32_t)p.one.nunits);
         for (int u = 0; u < p.one.nunits; ++u) bulk_load(res + (size_t)u * blk, p.one.B + (size_t)u * blk, blk, &B.res_bar);
@@ -557,10 +582,12 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
       } else {
         uint32_t s = 0, ph = 0, issued = 0, par = 0;
         bool ok = true;
+        FactShape f = fact_shape_of<WHO>(p, p.one);
         for (int64_t t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
           const FactMol& M = fact_mol<MULTI>(p, t);
           const int nunits = M.nunits;
-          const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * (uint32_t)M.r16 * 32u;
+          if (MULTI) f = fact_shape_of<WHO>(p, M);
+          const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * (uint32_t)f.r16 * 32u;
           const uint8_t* src = M.B;
           for (int u = 0; u < nunits; u += GROUP, src += GROUP * blk) {
             if (!mbar_wait(&B.empty[s], ph ^ 1u, &B.abort_flag, p.wait_ns)) {
@@ -584,9 +611,9 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
       }
     }
   } else if (warp == 1) {
-    issue_mma<FMT, TWO, MULTI, true>(p, B, smem, res, tmem);
+    issue_mma<FMT, TWO, WHO, true>(p, B, smem, res, tmem);
   } else if (warp == 2) {
-    if (TWO) issue_mma<FMT, TWO, MULTI, false>(p, B, smem, res, tmem);
+    if (TWO) issue_mma<FMT, TWO, WHO, false>(p, B, smem, res, tmem);
   } else if (warp == 3) {
     // ---- sample positions: a lane writes rows r and r + 64, r = lane and lane + 32 -------------------
     uint32_t tile_it = 0;
@@ -618,23 +645,25 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
     // ---- epilogue: rho = sum_k (2^-h_k T_k)^2, thread = row (TMEM lane) -----------------------------
     const int q = warp & 3, row = q * 32 + lane;
     uint32_t tile_it = 0;
+    FactShape f = fact_shape_of<WHO>(p, p.one);
     for (int64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x, ++tile_it) {
       const FactMol& M = fact_mol<MULTI>(p, t);
+      if (MULTI) f = fact_shape_of<WHO>(p, M);
       const uint32_t set = tile_it & 1u;
       // the four warps leave together: one of them giving up while the others go on would leave
       // those waiting at the next named barrier
       const bool got = mbar_wait(&B.t_full[set], (tile_it >> 1) & 1u, &B.abort_flag, p.wait_ns);
       if (barrier_any(1, 128, !got)) break;
       tc_fence_after();
-      const int r16 = M.r16;
-      const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + (M.sets == 2 ? set * 256u : 0u);
+      const int r16 = f.r16;
+      const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + (f.sets == 2 ? set * 256u : 0u);
       const float4* hs = reinterpret_cast<const float4*>(M.hscale);
       double acc = 0.0;
       // sixteen columns of H and S in flight while the sixteen before them are squared
       uint32_t ha[16], la[16], hb[16], lb[16];
       auto load = [&](int c, uint32_t(&h)[16], uint32_t(&l)[16]) {
         tmem_ld16_issue(base + (uint32_t)c, h);
-        if (TWO) tmem_ld16_issue(base + (uint32_t)(M.na * r16 + c), l);
+        if (TWO) tmem_ld16_issue(base + (uint32_t)(f.na * r16 + c), l);
       };
       auto square = [&](int c, uint32_t(&h)[16], uint32_t(&l)[16]) {
         f2 sq = 0ull;
@@ -657,18 +686,18 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
         tmem_ld16_wait(h);
         if (TWO) tmem_ld16_wait(l);
       };
-      if (M.na > 1) {
+      if (f.na > 1) {
         // several H accumulators: their sum takes the registers of the second block of columns
 #pragma unroll 1
         for (int c = 0; c < r16; c += 16) {
           load(c, ha, la);
           tmem_ld16_issue(base + (uint32_t)(r16 + c), hb);
-          if (M.na > 2) tmem_ld16_issue(base + (uint32_t)(2 * r16 + c), lb);
+          if (f.na > 2) tmem_ld16_issue(base + (uint32_t)(2 * r16 + c), lb);
           arrived(ha, la);
           tmem_ld16_wait(hb);
 #pragma unroll
           for (int j = 0; j < 16; ++j) ha[j] = __float_as_uint(__uint_as_float(ha[j]) + __uint_as_float(hb[j]));
-          if (M.na > 2) {
+          if (f.na > 2) {
             tmem_ld16_wait(lb);
 #pragma unroll
             for (int j = 0; j < 16; ++j) ha[j] = __float_as_uint(__uint_as_float(ha[j]) + __uint_as_float(lb[j]));
@@ -908,8 +937,8 @@ UnitTables build_units(const qmt_mol* m, const std::vector<float>& fs) {
 // column is a chain of latencies: the CTAs exchange their largest diagonals through distributed shared
 // memory (one cluster barrier; none with a single CTA), fetch the pivot's row of L from its owner while
 // P's row comes from L2, form their elements, eight lanes a row, and find their next largest diagonal.
-// info: [0] the rank, [1] set when it exceeds rmax or a remaining diagonal is negative beyond rounding
-// (the matrix is indefinite).
+// info: [0] the rank, 0 when it exceeds the limit or a remaining diagonal is negative beyond rounding (the matrix is
+// indefinite; [1] is set then).
 constexpr int PIV_THREADS = 512;
 constexpr int PIV_MAX_CTAS = 16;
 constexpr int PIV_PRE = 2;                    // rows per thread whose element of P is fetched early
@@ -917,6 +946,7 @@ struct PivotArgs {
   const double* P;
   int np, n, rmax, rows;      // rows per CTA
   int rows_in_smem, ld;       // row stride of L in shared memory
+  int limit;                  // of the rank (rmax: of the columns formed, at least 16)
   double tol;
   double* L;                  // n x rmax, FP64 (used when the rows do not fit in shared memory)
   float* L0;                  // n x ld0, FP32, zero beyond the rank up to a multiple of 16
@@ -1049,12 +1079,14 @@ __global__ void __launch_bounds__(PIV_THREADS, 1) fact_pivot_kernel(PivotArgs a)
   if (__syncthreads_or(bad) && t == 0) atomicExch(a.info + 1, 1);
   const int pad = max(16, (q + 15) / 16 * 16) - q;
   for (int i = t; i < nr * pad; i += PIV_THREADS) a.L0[(size_t)(r0 + i / pad) * a.ld0 + q + i % pad] = 0.f;
+  if (ncta > 1) cluster_barrier();   // no CTA leaves while another may still read its shared memory; every [1] is in
   if (c == 0 && t == 0) {
-    a.info[0] = q;
+    a.info[0] = __ldcg(a.info + 1) || q > a.limit ? 0 : q;
     *a.dmax = dmax;
   }
-  if (ncta > 1) cluster_barrier();   // no CTA leaves while another may still read its shared memory
 }
+
+__device__ __forceinline__ int ceil16(int r) { return r > 16 ? (r + 15) / 16 * 16 : 16; }
 
 // ---- refinement of the factor (FP64, device) ----------------------------------------------------
 // The float32 input matrix is L L^T only up to its rounding, and a pivoted Cholesky factor takes that
@@ -1062,10 +1094,16 @@ __global__ void __launch_bounds__(PIV_THREADS, 1) fact_pivot_kernel(PivotArgs a)
 // 1.25e-6 in all.  One power step spreads it over every column: with Y = P L0 and M = L0^T Y = C C^T,
 // L = Y C^-T is the Nystroem approximation of P on the range of Y (2e-7, as the truncated
 // eigendecomposition).  L0 only spans the space, so it comes as float32.
+//
+// The rank r is read from the device (info of fact_pivot_kernel), so that nothing here waits for the host: the grids are
+// sized for the largest one.
 __global__ void __launch_bounds__(256) fact_y_kernel(const double* __restrict__ P, int np, const float* __restrict__ L0,
-                                                     int ld0, int n, int r16, double* __restrict__ Y) {
+                                                     int ld0, int n, const int* __restrict__ rank,
+                                                     double* __restrict__ Y) {
   __shared__ double ps[32][33];
   __shared__ float ls[32][32];
+  const int r16 = ceil16(*rank);
+  if (*rank == 0 || (int)blockIdx.y * 32 >= r16) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = blockIdx.x * 32, q = blockIdx.y * 32 + tx;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int j0 = 0; j0 < n; j0 += 32) {
@@ -1091,11 +1129,12 @@ __global__ void __launch_bounds__(256) fact_y_kernel(const double* __restrict__ 
 
 // M = L0^T Y, r16 x r16; one block per 16 x 16 tile.
 __global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L0, int ld0, const double* __restrict__ Y,
-                                                     int n, int r16, double* __restrict__ M) {
+                                                     int n, const int* __restrict__ rank, double* __restrict__ M) {
   __shared__ float ls[32][17];
   __shared__ double ys[32][17];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, a = blockIdx.x * 16, b = blockIdx.y * 16;
-  if (b > a) return;   // the lower triangle is read
+  const int r16 = ceil16(*rank);
+  if (*rank == 0 || a >= r16 || b > a) return;   // the lower triangle is read
   double acc = 0.0;
   for (int i0 = 0; i0 < n; i0 += 32) {
     for (int r = ty; r < 32; r += 16) {
@@ -1117,12 +1156,15 @@ __global__ void __launch_bounds__(256) fact_m_kernel(const float* __restrict__ L
 // memory.  A column whose pivot is lost in rounding (1e-12 of its diagonal element: a pivot of L0 that was
 // the input's rounding) is left out, zero in CT; the residual check sees whether that mattered.
 constexpr int CHOL_NB = 16, CHOL_THREADS = 1024;
-__global__ void __launch_bounds__(CHOL_THREADS) fact_chol_kernel(double* __restrict__ M, int r, int r16, int in_smem,
-                                                                double* __restrict__ CT) {
+__global__ void __launch_bounds__(CHOL_THREADS) fact_chol_kernel(double* __restrict__ M, const int* __restrict__ rank,
+                                                                uint32_t smem, double* __restrict__ CT) {
   extern __shared__ double chol_s[];
   __shared__ double prow[2][CHOL_NB];
   __shared__ double pan[kFactorMaxR16][CHOL_NB + 1];   // the panel, scaled: C_ik
   const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+  const int r = *rank, r16 = ceil16(r);
+  if (r == 0) return;
+  const bool in_smem = (uint32_t)r * (uint32_t)(r16 + 1) * 8u <= smem;   // (beside the panel)
   double* a = in_smem ? chol_s : M;
   const int ld = in_smem ? r16 + 1 : r16;
   if (in_smem)
@@ -1187,10 +1229,13 @@ __global__ void __launch_bounds__(CHOL_THREADS) fact_chol_kernel(double* __restr
 // memory), in place, and the largest |L_iq| 2^-s_i of each column (as ordered bits of a non-negative double).
 constexpr int SOLVE_WARPS = 8;
 __global__ void __launch_bounds__(32 * SOLVE_WARPS) fact_solve_kernel(double* __restrict__ Y,
-                                                                      const double* __restrict__ CT, int n, int r,
-                                                                      int r16, const double* __restrict__ inv_s,
+                                                                      const double* __restrict__ CT, int n,
+                                                                      const int* __restrict__ rank,
+                                                                      const double* __restrict__ inv_s,
                                                                       unsigned long long* __restrict__ colmax) {
   extern __shared__ double ct_s[];   // 32 x r16
+  const int r = *rank, r16 = ceil16(r);
+  if (r == 0) return;
   const int row = blockIdx.x * SOLVE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const bool in = row < n;
   double y[kFactorMaxR16 / 32];
@@ -1226,10 +1271,10 @@ __global__ void __launch_bounds__(32 * SOLVE_WARPS) fact_solve_kernel(double* __
 
 // Column scales: 2^h_q brings the column's largest scaled element near 2^14 (h in [-100, 100]); then
 // 2^-h_q in FP32 for the squares (0 for the padding columns).
-__global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax, int r, int r16, double* __restrict__ two_h,
-                                  float* __restrict__ hscale) {
-  const int q = threadIdx.x;
-  if (q >= r16) return;
+__global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax, const int* __restrict__ rank,
+                                  double* __restrict__ two_h, float* __restrict__ hscale) {
+  const int q = threadIdx.x, r = *rank;
+  if (r == 0 || q >= ceil16(r)) return;
   const double mx = __longlong_as_double((long long)colmax[q]);
   int h = mx > 0 ? (int)floor(log2(16000.0 / mx)) : 0;
   h = max(-100, min(100, h));
@@ -1237,14 +1282,16 @@ __global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax,
   hscale[q] = q < r ? ldexpf(1.0f, -h) : 0.f;
 }
 
-// Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds rel * dmax; L row i at L[i * ld].  One block per
+// Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds rel * dmax; L row i at L[i * r16].  One block per
 // 32 x 32 tile on or below the diagonal.
 __global__ void __launch_bounds__(256) fact_residual_kernel(const double* __restrict__ P, int np,
-                                                            const double* __restrict__ L, int n, int ld, int r, double rel,
+                                                            const double* __restrict__ L, int n,
+                                                            const int* __restrict__ rank, double rel,
                                                             const double* __restrict__ dmax, int* bad) {
   __shared__ double li[32][33], lj[32][33];
+  const int r = *rank, ld = ceil16(r);
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  if (j0 > i0) return;
+  if (r == 0 || j0 > i0) return;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int q0 = 0; q0 < r; q0 += 32) {
 #pragma unroll
@@ -1275,9 +1322,19 @@ __global__ void __launch_bounds__(256) fact_residual_kernel(const double* __rest
 // q < r16, one row of 32 bytes per q and piece (hi rows then lo rows), the two 16-byte halves of a row
 // exchanged when bit 2 of q is set.
 // Element: W = L_jq 2^-s_j 2^h_q of the column's function j, split into hi + lo; zero for padding.
-__global__ void fact_split_kernel(const double* __restrict__ L, int ld, int r, const int* __restrict__ column, int nunits,
-                                  int r16, const double* __restrict__ inv_s, const double* __restrict__ two_h, int fmt,
-                                  int nsplit, uint8_t* __restrict__ out) {
+// The last kernel of a factorisation also says what it came to: the rank (0 where the check failed) in *usable for the
+// kernels and a host that waits, and with the factorisation's number in page-locked host memory for one that does not.
+__global__ void fact_split_kernel(const double* __restrict__ L, const int* __restrict__ rank, const int* __restrict__ column,
+                                  int nunits, const double* __restrict__ inv_s, const double* __restrict__ two_h, int fmt,
+                                  int nsplit, uint8_t* __restrict__ out, const int* __restrict__ bad, int* usable,
+                                  uint32_t number, volatile unsigned long long* mail) {
+  const int r = *rank, r16 = ceil16(r), ld = r16;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int u = *bad ? 0 : r;
+    *usable = u;
+    *mail = (unsigned long long)number << 32 | (unsigned)u;
+  }
+  if (r == 0) return;
   const int64_t tot = (int64_t)nunits * 16 * r16;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i / r16), q = (int)(i - (int64_t)c * r16), u = c >> 4;
@@ -1301,14 +1358,21 @@ __global__ void fact_split_kernel(const double* __restrict__ L, int ld, int r, c
   }
 }
 
+// The device's decision for a call that takes ranks up to `limit` (out[1].refused: the rank taken).
+__global__ void fact_decide_kernel(const int* __restrict__ usable, int limit, int nunits, FactShape* out) {
+  const int r = *usable <= limit ? *usable : 0;
+  out[0] = fact_shape(r, nunits);
+  out[1].refused = r;
+}
+
 constexpr int kBf16MaxRank = 128;
 constexpr double kFactorTol = 1e-7;
 constexpr double kFactorResid = 2e-7;
 
 }  // namespace
 
-static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double* L, float* L0, int ld0, int* info,
-                               double* dmax, cudaStream_t s) {
+static qmt_status launch_pivot(const double* P, int np, int n, int rmax, int limit, double* L, float* L0, int ld0,
+                               int* info, double* dmax, cudaStream_t s) {
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1321,6 +1385,7 @@ static qmt_status launch_pivot(const double* P, int np, int n, int rmax, double*
     a.rmax = rmax;
     a.rows = (n + ncta - 1) / ncta;
     a.ld = rmax + 8;   // (four rows of a warp on two sets of banks)
+    a.limit = limit;
     a.tol = kFactorTol;
     a.L = L;
     a.L0 = L0;
@@ -1369,11 +1434,16 @@ qmt_status ensure_unit_tables(qmt_mol* m, const std::vector<float>& fs, cudaStre
   return QMT_OK;
 }
 
-// Largest rank that is factored: half of n; with `any_rank` (fp16x3 and many sample points, see density_tc)
-// every rank of a matrix of up to 256 functions; bf16 as takes_factor says.
-static int factor_rmax(int n16, int fmt, bool any_rank) {
+static int rank_limit(int n16, int fmt, bool any_rank) {
   if (fmt != 0) return std::min(kBf16MaxRank, n16 / 2);
   return any_rank && n16 <= kFactorMaxR16 ? n16 : std::min(kFactorMaxR16, n16 / 2);
+}
+int factor_limit(const qmt_mol* m, int fmt, bool any_rank) {
+  const int lim = rank_limit((m->norbs + 15) / 16 * 16, fmt, any_rank);
+  // a density matrix of N_e electrons whose occupations are at most 2 has rank >= N_e / 2: with
+  // the nuclear charge for N_e (ions of up to 16 charges allowed for) a rank above the limit is known
+  // without factoring
+  return 0.5 * m->qtot > std::max(16, lim) + 8 ? 0 : lim;
 }
 
 // A density matrix of rank r (r = occupied orbitals for an SCF density, P = 2 C_occ C_occ^T) is
@@ -1382,30 +1452,35 @@ static int factor_rmax(int n16, int fmt, bool any_rank) {
 // used when the matrix it leaves out is at most kFactorResid of max |P| (float32 input rounding is
 // ~6e-8).  A matrix that is not positive semi-definite, or of high rank, takes the unfactored path.
 // The scaled factor W_jk = L_jk 2^(h_k - s_j) (so Phi' W = 2^h_k (Phi L)_k, each column scaled to a
-// maximum near 2^14) goes to the blocks of fact_split_kernel.  Sets fact_rank = 0 when the matrix is not
-// factored.  The host waits for the rank, once per matrix.
+// maximum near 2^14) goes to the blocks of fact_split_kernel.  Nothing waits: the rank and the check stay on the
+// device until factor_rank reads them.
 qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, cudaStream_t s) {
-  // built for this precision, or refused by at least this rank limit
-  if (m->fact_prec == prec && (m->fact_rank > 0 || m->fact_any_rank || !any_rank)) return QMT_OK;
   qmt_status st;
+  // built for this precision (rank -1: the device knows), or refused by at least this rank limit
+  int rank = 0;
+  if (m->fact_prec == prec && (st = factor_rank(m, false, &rank, s))) return st;
+  if (m->fact_prec == prec && (rank > 0 || m->fact_any_rank || !any_rank)) return QMT_OK;
   if ((st = ensure_basis_operands(m, kpad, s))) return st;
   const int n = m->norbs, np = m->npad, n16 = (n + 15) / 16 * 16;
-  m->fact_prec = prec;
-  m->fact_any_rank = any_rank;
-  m->fact_rank = 0;
-  const int rmax = std::max(16, factor_rmax(n16, fmt, any_rank));
-  // a density matrix of N_e electrons whose occupations are at most 2 has rank >= N_e / 2: with
-  // the nuclear charge for N_e (ions of up to 16 charges allowed for) a rank above rmax is known
-  // without factoring
-  if (0.5 * m->qtot > rmax + 8) return QMT_OK;
-  // device scratch for any rank: L (FP64), Y (then the refined L), M, C^T, column maxima, flag, info, L0.  The
-  // kernels work on whole blocks of 16 columns, so it is sized by the rank limit rounded up to them (n16 / 2 is an
-  // odd multiple of 8 for every second n16).
-  const int rbuf = (rmax + 15) / 16 * 16;
+  m->fact_prec = -1;   // (until all of it is enqueued)
+  // device scratch: L (FP64), Y (then the refined L), M, C^T, column maxima, info, L0.  The kernels work on whole
+  // blocks of 16 columns, so it is sized by the rank limit rounded up to them (n16 / 2 is an odd multiple of 8 for
+  // every second n16); for any rank where that may be asked for later, so that a call being captured in a graph
+  // allocates nothing.
+  const int rmax = std::max(16, rank_limit(n16, fmt, any_rank));
+  const int rbuf = (std::max(16, rank_limit(n16, fmt, true)) + 15) / 16 * 16;
   const size_t nr = (size_t)n * rbuf, rr = (size_t)rbuf * rbuf;
   if ((st = m->d_fact_L.reserve((2 * nr + 2 * rr + rbuf + 8) * sizeof(double) + nr * sizeof(float))) ||
-      (st = m->d_fact_scale.reserve(rbuf * (sizeof(double) + sizeof(float)))))
+      (st = m->d_fact_scale.reserve(kFactorMaxR16 * (sizeof(double) + sizeof(float)))) ||
+      (st = m->d_fact_B.reserve((size_t)m->fact_units * nsplit * rbuf * 32)))
     return st;
+  const int limit = factor_limit(m, fmt, any_rank);
+  if (limit == 0) {
+    m->fact_prec = prec;
+    m->fact_any_rank = any_rank;
+    m->fact_rank = 0;
+    return QMT_OK;
+  }
   double* Lp = m->d_fact_L.as<double>();
   double* Y = Lp + nr;
   double* M = Y + nr;
@@ -1413,75 +1488,85 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   unsigned long long* colmax = reinterpret_cast<unsigned long long*>(CT + rr);
   int* info = reinterpret_cast<int*>(colmax + rbuf);
   double* dmax = reinterpret_cast<double*>(colmax + rbuf + 1);
-  int* flag = reinterpret_cast<int*>(m->d_scalars.as<double>() + 9);   // beside the sum and the give-up flag
+  int* bad = reinterpret_cast<int*>(colmax + rbuf + 2);
   float* L0 = reinterpret_cast<float*>(colmax + rbuf + 8);
   double* two_h = m->d_fact_scale.as<double>();
   const double* P = m->d_P64.as<double>();
+  const int r16max = (rmax + 15) / 16 * 16;   // <= rbuf
   QMT_CUDA(cudaMemsetAsync(colmax, 0, (rbuf + 8) * sizeof(double), s));
-  QMT_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
-  if ((st = launch_pivot(P, np, n, rmax, Lp, L0, rbuf, info, dmax, s))) return st;
-  int got[2] = {0, 0};
-  QMT_CUDA(cudaMemcpyAsync(got, info, sizeof(got), cudaMemcpyDeviceToHost, s));
-  QMT_CUDA(cudaStreamSynchronize(s));
-  if (got[1] || got[0] <= 0 || got[0] > factor_rmax(n16, fmt, any_rank)) return QMT_OK;   // rank too high to pay, or indefinite
-  const int r = got[0], r16 = std::max(16, (r + 15) / 16 * 16);
-  if (r16 > rbuf) return fail(QMT_BAD_ARG, "factor rank beyond its workspace");
-  // refined on the device; what the factor then leaves out, max |P - L L^T|, is checked there too, into
-  // the gate flag and without a round trip: the factored launch runs when it is 0, the unfactored one
-  // when it is 1 (density_tc)
-  fact_y_kernel<<<dim3((n + 31) / 32, (r16 + 31) / 32), 256, 0, s>>>(P, np, L0, rbuf, n, r16, Y);
+  if ((st = launch_pivot(P, np, n, rmax, limit, Lp, L0, rbuf, info, dmax, s))) return st;
+  // refined, and what the factor then leaves out, max |P - L L^T|, checked
+  fact_y_kernel<<<dim3((n + 31) / 32, (r16max + 31) / 32), 256, 0, s>>>(P, np, L0, rbuf, n, info, Y);
   QMT_CHECK_LAUNCH("fact_y_kernel");
-  fact_m_kernel<<<dim3(r16 / 16, r16 / 16), 256, 0, s>>>(L0, rbuf, Y, n, r16, M);
+  fact_m_kernel<<<dim3(r16max / 16, r16max / 16), 256, 0, s>>>(L0, rbuf, Y, n, info, M);
   QMT_CHECK_LAUNCH("fact_m_kernel");
-  const size_t csm = (size_t)r * (r16 + 1) * sizeof(double);
-  const int in_smem = csm <= 180u * 1024u ? 1 : 0;   // (beside the panel)
-  if (in_smem)
-    QMT_CUDA(cudaFuncSetAttribute(fact_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024));
-  fact_chol_kernel<<<1, CHOL_THREADS, in_smem ? csm : 0, s>>>(M, r, r16, in_smem, CT);
+  const size_t csm = std::min<size_t>((size_t)rmax * (r16max + 1) * sizeof(double), 180u * 1024u);
+  QMT_CUDA(cudaFuncSetAttribute(fact_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024));
+  fact_chol_kernel<<<1, CHOL_THREADS, csm, s>>>(M, info, (uint32_t)csm, CT);
   QMT_CHECK_LAUNCH("fact_chol_kernel");
-  const size_t ssm = (size_t)32 * r16 * sizeof(double);
+  const size_t ssm = (size_t)32 * r16max * sizeof(double);
   QMT_CUDA(cudaFuncSetAttribute(fact_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 32 * kFactorMaxR16 * (int)sizeof(double)));
   fact_solve_kernel<<<(n + SOLVE_WARPS - 1) / SOLVE_WARPS, 32 * SOLVE_WARPS, ssm, s>>>(
-      Y, CT, n, r, r16, m->d_split_scale.as<double>(), colmax);
+      Y, CT, n, info, m->d_split_scale.as<double>(), colmax);
   QMT_CHECK_LAUNCH("fact_solve_kernel");
-  fact_scale_kernel<<<1, kFactorMaxR16, 0, s>>>(colmax, r, r16, two_h, reinterpret_cast<float*>(two_h + r16));
+  fact_scale_kernel<<<1, kFactorMaxR16, 0, s>>>(colmax, info, two_h, reinterpret_cast<float*>(two_h + kFactorMaxR16));
   QMT_CHECK_LAUNCH("fact_scale_kernel");
-  fact_residual_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), 256, 0, s>>>(P, np, Y, n, r16, r, kFactorResid, dmax, flag);
+  fact_residual_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), 256, 0, s>>>(P, np, Y, n, info, kFactorResid, dmax, bad);
   QMT_CHECK_LAUNCH("fact_residual_kernel");
-  m->fact_gate = flag;
-  m->fact_ok = -1;
-  const size_t total = (size_t)m->fact_units * nsplit * r16 * 32;   // bytes
-  if ((st = m->d_fact_B.reserve(total))) return st;
-  const int64_t tot = (int64_t)m->fact_units * 16 * r16;
+  const int64_t tot = (int64_t)m->fact_units * 16 * r16max;
   const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
+  if (++m->fact_number == 0) m->fact_number = 1;
   fact_split_kernel<<<std::max(blocks, 1), 256, 0, s>>>(
-      Y, r16, r, reinterpret_cast<const int*>(m->d_fact_tab.as<uint8_t>() + m->fact_col_off),
-      m->fact_units, r16, m->d_split_scale.as<double>(), two_h, fmt, nsplit,
-      m->d_fact_B.as<uint8_t>());
+      Y, info, reinterpret_cast<const int*>(m->d_fact_tab.as<uint8_t>() + m->fact_col_off), m->fact_units,
+      m->d_split_scale.as<double>(), two_h, fmt, nsplit, m->d_fact_B.as<uint8_t>(), bad, m->fact_usable(), m->fact_number,
+      m->fact_mail);
   QMT_CHECK_LAUNCH("fact_split_kernel");
-  m->fact_rank = r;
-  m->fact_r16 = r16;
+  m->fact_prec = prec;
+  m->fact_any_rank = any_rank;
+  m->fact_rank = -1;
   return QMT_OK;
 }
 
-void fact_mol_desc(const qmt_mol* m, const PointMap& pm, int64_t tile0, int64_t ntiles, float* qube, double outscale,
-                   FactMol& d) {
+qmt_status factor_rank(qmt_mol* m, bool wait, int* rank, cudaStream_t s) {
+  if (m->fact_rank < 0) {
+    const unsigned long long mail = *m->fact_mail;
+    if ((uint32_t)(mail >> 32) == m->fact_number) {
+      m->fact_rank = (int)(uint32_t)mail;
+    } else if (wait) {
+      int got = 0;
+      QMT_CUDA(cudaMemcpyAsync(&got, m->fact_usable(), sizeof(got), cudaMemcpyDeviceToHost, s));
+      QMT_CUDA(cudaStreamSynchronize(s));
+      m->fact_rank = got;
+    }
+  }
+  *rank = m->fact_rank;
+  return QMT_OK;
+}
+
+qmt_status decide_on_device(qmt_mol* m, int limit, const FactShape** shape, cudaStream_t s) {
+  FactShape* out = reinterpret_cast<FactShape*>(m->fact_decision());
+  fact_decide_kernel<<<1, 1, 0, s>>>(m->fact_usable(), limit, m->fact_units, out);
+  QMT_CHECK_LAUNCH("fact_decide_kernel");
+  *shape = out;
+  return QMT_OK;
+}
+
+void fact_mol_desc(const qmt_mol* m, int rank, const PointMap& pm, int64_t tile0, int64_t ntiles, float* qube,
+                   double outscale, FactMol& d) {
   d = FactMol{};
   d.pm = pm;
   d.tile0 = tile0;
   d.ntiles = ntiles;
   d.nunits = m->fact_units;
-  d.r16 = m->fact_r16;
-  d.sets = 2 * d.r16 <= 256 ? 2 : 1;
-  // The tensor core's additions truncate, so every K-step takes about 2^-24 of T away and the squares double that:
-  // a uniform loss, which only rescaling hides.  Units in turn on up to three accumulators divide it by as many where
-  // two buffers hold them (a third buffer's worth of TMEM is not given up for it).
-  d.na = d.sets == 2 ? std::clamp(256 / d.r16 - 1, 1, std::min(3, d.nunits)) : 1;
+  const FactShape f = fact_shape(rank, d.nunits);
+  d.r16 = f.r16;
+  d.sets = f.sets;
+  d.na = f.na;
   d.B = m->d_fact_B.as<uint8_t>();
   d.units = m->d_fact_tab.as<int4>();
   d.coords = m->d_coords.as<float>();
-  d.hscale = reinterpret_cast<const float*>(m->d_fact_scale.as<double>() + d.r16);
+  d.hscale = reinterpret_cast<const float*>(m->d_fact_scale.as<double>() + kFactorMaxR16);
   d.qube = qube;
   d.partials = m->d_partials.as<double>();
   d.outscale = outscale;
@@ -1489,9 +1574,9 @@ void fact_mol_desc(const qmt_mol* m, const PointMap& pm, int64_t tile0, int64_t 
 
 namespace {
 
-template <int FMT, bool TWO, bool MULTI>
+template <int FMT, bool TWO, int WHO>
 qmt_status launch_as(FactParams& p, int blk_max, int nunits, cudaStream_t s) {
-  auto kern = density_factored_kernel<FMT, TWO, MULTI>;
+  auto kern = density_factored_kernel<FMT, TWO, WHO>;
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1502,7 +1587,7 @@ qmt_status launch_as(FactParams& p, int blk_max, int nunits, cudaStream_t s) {
   // the factor stays in shared memory when at least MIN_SLOTS slots fit beside it; else its blocks
   // stream through the slots
   const int64_t whole = (int64_t)blk_max * nunits;
-  p.resident = !MULTI && whole + MIN_SLOTS * abytes <= avail ? 1 : 0;
+  p.resident = WHO == ONE && whole + MIN_SLOTS * abytes <= avail ? 1 : 0;
   p.slot_bytes = (uint32_t)(abytes + (p.resident ? 0 : GROUP * blk_max));
   const int64_t room = avail - (p.resident ? whole : 0);
   p.nslots = (uint32_t)std::min<int64_t>(MAX_SLOTS, room / p.slot_bytes);
@@ -1517,10 +1602,17 @@ qmt_status launch_as(FactParams& p, int blk_max, int nunits, cudaStream_t s) {
   return QMT_OK;
 }
 
+template <int FMT, bool TWO>
+qmt_status launch_whose(FactParams& p, int blk_max, cudaStream_t s) {
+  if (p.nmol > 1) return launch_as<FMT, TWO, MANY>(p, blk_max, 0, s);
+  if (p.shape) return launch_as<FMT, TWO, ON_DEVICE>(p, blk_max, p.one.nunits, s);
+  return launch_as<FMT, TWO, ONE>(p, blk_max, p.one.nunits, s);
+}
+
 }  // namespace
 
 qmt_status launch_factored(const FactMol* host, const FactMol* dev, int nmol, int64_t ntiles, int fmt, int nsplit,
-                           int* err, const int* gate, int gate_want, cudaStream_t s) {
+                           int* err, const FactShape* shape, cudaStream_t s) {
   FactParams p{};
   int r16 = 0;
   for (int i = 0; i < nmol; ++i) r16 = std::max(r16, host[i].r16);
@@ -1528,18 +1620,13 @@ qmt_status launch_factored(const FactMol* host, const FactMol* dev, int nmol, in
   p.mols = dev;
   p.nmol = nmol;
   p.ntiles = ntiles;
-  p.nsplit = nsplit;
   p.fmt = (uint32_t)fmt;
   p.err = err;
   p.wait_ns = wait_limit_ns();
-  p.gate = gate;
-  p.gate_want = gate_want;
+  p.shape = shape;
   const int blk = nsplit * r16 * 32;
-  const bool multi = nmol > 1;
-  if (fmt == 0) return multi ? launch_as<0, true, true>(p, blk, 0, s) : launch_as<0, true, false>(p, blk, p.one.nunits, s);
-  if (nsplit == 2)
-    return multi ? launch_as<1, true, true>(p, blk, 0, s) : launch_as<1, true, false>(p, blk, p.one.nunits, s);
-  return multi ? launch_as<1, false, true>(p, blk, 0, s) : launch_as<1, false, false>(p, blk, p.one.nunits, s);
+  if (fmt == 0) return launch_whose<0, true>(p, blk, s);
+  return nsplit == 2 ? launch_whose<1, true>(p, blk, s) : launch_whose<1, false>(p, blk, s);
 }
 
 }  // namespace qmt

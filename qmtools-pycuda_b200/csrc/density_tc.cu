@@ -1897,13 +1897,10 @@ constexpr int kBf16FusedMaxR16 = 64;
 // that equal calls give equal results.
 constexpr int64_t kAnyRankTiles = 8192;
 static bool any_rank_pays(const TcShape& sh, int64_t ntiles) { return sh.fmt == FMT_F16 && ntiles >= kAnyRankTiles; }
-static bool takes_factor(const qmt_mol* m, const TcShape& sh, bool fused, int64_t ntiles) {
-  if (m->fact_rank <= 0) return false;
-  if (sh.fmt != FMT_F16) return !fused || m->fact_r16 <= kBf16FusedMaxR16;
-  // (a call on a small grid does not factor a molecule whose charge rules out a rank of half of N, and so leaves alone
-  // what a call on a large one has factored)
-  const int half = (m->norbs + 15) / 16 * 8;
-  return any_rank_pays(sh, ntiles) || (m->fact_rank <= half && 0.5 * m->qtot <= std::max(16, half) + 8);
+// The largest rank that a call takes (0: the charge rules its factor out), whatever rank an earlier call has factored.
+static int call_limit(const qmt_mol* m, const TcShape& sh, bool fused, bool any_rank) {
+  const int lim = factor_limit(m, sh.fmt, any_rank);
+  return sh.fmt != FMT_F16 && fused ? std::min(lim, kBf16FusedMaxR16) : lim;
 }
 
 // The fused path takes fp16/bf16 contractions of up to 320 functions whose tile, stages and tables
@@ -1929,29 +1926,34 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   const bool fused = g_density_path == 1 ? false : fusable;
   if (g_density_path == 2 && !fusable)
     return fail(QMT_BAD_ARG, "fused density path needs fp16/bf16, N <= 320 and molecule tables that fit in shared memory");
-  // the factored matrix when there is one (automatic, or asked for)
+  // The factored matrix when there is one (automatic, or asked for).  Whether there is one the device knows first.
+  // A call that returns a sum, and so waits anyway, reads it; an asynchronous one takes it where the host has seen it,
+  // and else launches both kernels, one of which the device's decision sends home.
   bool fact = false;
+  int rank = 0;
+  const FactShape* shape = nullptr;
   if (sh.fmt != FMT_TF32 && g_density_path != 1 && g_density_path != 2) {
-    const bool any = g_density_path == 0 && any_rank_pays(sh, ntiles);
-    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, s))) return st;
-    fact = takes_factor(mol, sh, fused, ntiles);
-    if (g_density_path == 3 && (!fact || mol->fact_rank > std::min(kFactorAskedRank, fused_n16(mol) / 2)))
-      return fail(QMT_BAD_ARG, "factored density path needs a positive semi-definite density matrix of low rank");
-  }
-  // The device checks what a factor leaves out.  Once the host has read the check it decides; a call that
-  // returns a sum reads it afterwards and comes back for the unfactored kernel should it have failed; an
-  // asynchronous call before that launches both, and the check picks one on the device.
-  if (fact && mol->fact_ok == 0) fact = false;
-  const bool known = fact && mol->fact_ok == 1, pair = fact && !known && !sum_out;
-  const int* gate = fact && !known ? mol->fact_gate : nullptr;
-  if (fact) {
-    FactMol d;
-    fact_mol_desc(mol, pm, 0, ntiles, qube, outscale, d);
-    if ((st = launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit,
-                              reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), gate, 0, s)))
+    const bool asked = g_density_path == 3;
+    bool any = !asked && any_rank_pays(sh, ntiles);
+    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, s)) ||
+        (st = factor_rank(mol, asked || sum_out, &rank, s)))
       return st;
+    int limit = call_limit(mol, sh, fused, any);
+    if (asked) limit = std::min(limit, std::min(kFactorAskedRank, fused_n16(mol) / 2));
+    fact = limit > 0 && (rank < 0 || (rank > 0 && rank <= limit));
+    if (asked && !fact)
+      return fail(QMT_BAD_ARG, "factored density path needs a positive semi-definite density matrix of low rank");
+    if (fact) {
+      if (rank < 0 && (st = decide_on_device(mol, limit, &shape, s))) return st;
+      FactMol d;
+      fact_mol_desc(mol, rank < 0 ? limit : rank, pm, 0, ntiles, qube, outscale, d);
+      if ((st = launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit,
+                                reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), shape, s)))
+        return st;
+    }
   }
-  if (fact && !pair) {
+  const int* gate = shape ? &shape->refused : nullptr;
+  if (fact && !shape) {
   } else if (fused) {
     if ((st = ensure_fused_operands(mol, precision, sh, s))) return st;
     if (sh.fmt == FMT_F16) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
@@ -1970,7 +1972,7 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   // synchronises anyway) reads it beside the sum and clears it; fully asynchronous calls leave it for
   // the next synchronous call on this molecule.
   if (sum_out) {
-    double h[10];   // [0] sum, [8] give-up flag, [9] the factor's check
+    double h[9];   // [0] sum, [8] give-up flag
     QMT_CUDA(cudaMemcpyAsync(h, mol->d_scalars.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     QMT_CUDA(cudaStreamSynchronize(s));
     *sum_out = h[0];
@@ -1979,13 +1981,6 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
     if (err) {
       QMT_CUDA(cudaMemsetAsync(mol->d_scalars.as<double>() + 8, 0, sizeof(int), s));
       return fail(QMT_CUDA_ERR, "tensor-core density kernel gave up waiting on a barrier");
-    }
-    if (fact && !known) {
-      int refused = 0;
-      std::memcpy(&refused, h + 9, sizeof(refused));
-      mol->fact_ok = refused ? 0 : 1;
-      if (refused)
-        return density_tc(mol, nx, ny, nz, step, ox, oy, oz, subgrid, precision, rescale, qube, sum_out, s);
     }
     if (!std::isfinite(h[0])) return fail(QMT_NAN, "non-finite density sum");
   }
@@ -2006,6 +2001,7 @@ struct BatchItem {
   double outscale;
   bool fused;  // N <= 320: the fused kernel takes it
   bool fact;   // on the factored launch
+  int rank;    // its factor's
 };
 
 }  // namespace qmt
@@ -2099,7 +2095,7 @@ static qmt_status batch_run(qmt_batch* b, int rescale, bool refresh, cudaStream_
     constexpr int F = FMT == FMT_TF32 ? FMT_F16 : FMT;
     if (!b->fact.empty() &&
         (st = launch_factored(b->fact.data(), b->d_fact.as<FactMol>(), (int)b->fact.size(), b->fact_tiles, F, b->nsplit,
-                              b->d_err.as<int>(), nullptr, 0, s)))
+                              b->d_err.as<int>(), nullptr, s)))
       return st;
     if ((st = batch_launch<F>(b, b->fused, s))) return st;
   }
@@ -2158,18 +2154,11 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
     it.fused = path == 2 || ((path == 0 || path == 3) && fits);
     it.fact = false;
     if (path == 3 && it.sh.fmt != FMT_TF32) {   // factored when the matrix has a factor that passes the check
-      int gate = 1;
-      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, any_rank_pays(it.sh, it.ntiles), s))) break;
-      if (m->fact_rank > 0) {
-        const cudaError_t e1 = cudaMemcpyAsync(&gate, m->fact_gate, sizeof(int), cudaMemcpyDeviceToHost, s);
-        const cudaError_t e2 = cudaStreamSynchronize(s);
-        if (e1 != cudaSuccess || e2 != cudaSuccess) {
-          st = cuda_fail(e1 != cudaSuccess ? e1 : e2, "factor check");
-          break;
-        }
-      }
-      m->fact_ok = m->fact_rank > 0 ? gate == 0 : -1;
-      it.fact = gate == 0 && takes_factor(m, it.sh, it.fused, it.ntiles);
+      const bool any = any_rank_pays(it.sh, it.ntiles);
+      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, any, s)) ||
+          (st = factor_rank(m, true, &it.rank, s)))
+        break;
+      it.fact = it.rank > 0 && it.rank <= call_limit(m, it.sh, it.fused, any);
     }
     if ((st = m->d_partials.reserve(it.ntiles * sizeof(double))) || (st = m->d_scalars.reserve(64 * sizeof(double))))
       break;
@@ -2190,7 +2179,7 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
   for (const BatchItem& it : b->items) {
     if (!it.fact) continue;
     FactMol d;
-    fact_mol_desc(it.mol, it.pm, b->fact_tiles, it.ntiles, it.qube, it.outscale, d);
+    fact_mol_desc(it.mol, it.rank, it.pm, b->fact_tiles, it.ntiles, it.qube, it.outscale, d);
     b->fact_tiles += it.ntiles;
     b->fact.push_back(d);
   }
@@ -2283,13 +2272,9 @@ qmt_status qmt_batch_destroy(qmt_batch* b) {
 extern "C" qmt_status qmt_density_factor_rank(qmt_mol* mol, int* rank_out, void* stream) {
   if (!mol || !rank_out) return qmt::fail(QMT_BAD_ARG, "null argument");
   *rank_out = 0;
-  if (mol->fact_prec < 0 || mol->fact_rank <= 0 || !mol->fact_gate) return QMT_OK;
-  int gate = 1;
-  cudaStream_t s = qmt::as_stream(stream);
-  QMT_CUDA(cudaMemcpyAsync(&gate, mol->fact_gate, sizeof(int), cudaMemcpyDeviceToHost, s));
-  QMT_CUDA(cudaStreamSynchronize(s));
-  if (gate == 0) *rank_out = mol->fact_rank;
-  return QMT_OK;
+  if (mol->fact_prec < 0) return QMT_OK;
+  qmt_status st = qmt::factor_rank(mol, true, rank_out, qmt::as_stream(stream));
+  return st;
 }
 
 extern "C" qmt_status qmt_set_density_path(int mode) {

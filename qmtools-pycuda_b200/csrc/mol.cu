@@ -91,6 +91,7 @@ qmt_mol::~qmt_mol() {
                     &d_fused_tab, &d_split_scale,
                     &d_dm_raw, &d_gscale, &d_pairs32, &d_gto_part})
     b->release();
+  if (fact_mail) cudaFreeHost(const_cast<unsigned long long*>(fact_mail));
 }
 
 namespace qmt {
@@ -268,6 +269,12 @@ static qmt_status mol_init(qmt_mol* m, int natoms, const int32_t* types, const f
     return st;
   }
   QMT_CUDA(cudaMemsetAsync(m->d_scalars.ptr, 0, 64 * sizeof(double), s));
+  if (!m->fact_mail) {   // here, where the call waits anyway: page-locking may
+    void* p = nullptr;
+    QMT_CUDA(cudaHostAlloc(&p, sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped));
+    m->fact_mail = static_cast<volatile unsigned long long*>(p);
+    *m->fact_mail = 0;
+  }
   QMT_CUDA(cudaStreamSynchronize(s));
   return QMT_OK;
 }

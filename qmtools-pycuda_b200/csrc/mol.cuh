@@ -47,16 +47,20 @@ struct qmt_mol {
   qmt::DevBuf d_split_scale;    // 2^-s_j per function for the device split of the density matrix
   int fact_prec = -1;           // precision of the factored-path operands below (-1: not built)
   bool fact_any_rank = false;   // the rank limit they were built (or refused) with
-  int fact_rank = 0;            // rank of the density-matrix factor P = L L^T (0: not factored)
-  int fact_r16 = 0;             // the rank rounded up to 16 (the MMA N)
-  qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of fact_r16 rows a piece
+  int fact_rank = 0;            // rank of the density-matrix factor P = L L^T (0: none, or it failed its check;
+                                // -1: known on the device only)
+  uint32_t fact_number = 0;     // number of the last factorisation, and the page-locked word in which the device
+  volatile unsigned long long* fact_mail = nullptr;   // leaves (number << 32 | rank) once it is done
+  qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of the rank rounded up to 16 rows a piece
   qmt::DevBuf d_fact_tab;       // unit and class tables, then the function of each column
   int fact_units = 0;           // units of 16 columns
   size_t fact_col_off = 0;      // byte offset of the column table
   qmt::DevBuf d_fact_L;         // factorisation scratch: the factor (FP64), its refinement, the flag of the residual check
-  const int* fact_gate = nullptr; // device flag: 0 when the factor reproduces P, 1 when it does not
-  int fact_ok = -1;             // the same as last read by the host (1: it does, 0: it does not, -1: not read)
-  qmt::DevBuf d_fact_scale;     // per factor column k: 2^h_k (FP64), then 2^-h_k (FP32)
+  qmt::DevBuf d_fact_scale;     // per factor column k: 2^h_k (FP64), then from the 256th double on 2^-h_k (FP32)
+  // words of d_scalars ([0] the sum, [8] the give-up flag): the factor's rank as the device has it, and its decision
+  // for the last call that left it to the device
+  int* fact_usable() const { return reinterpret_cast<int*>(d_scalars.as<double>() + 9); }
+  int* fact_decision() const { return reinterpret_cast<int*>(d_scalars.as<double>() + 10); }
   qmt::DevBuf d_fused_tab;      // fused path: packed shell records, then (alpha, scaled coefficient) pairs
   qmt::DevBuf d_coords, d_types, d_shells, d_alpha, d_coeff, d_alpha64, d_coeff64;
   qmt::DevBuf d_P32, d_P64;
