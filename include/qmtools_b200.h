@@ -126,8 +126,9 @@ qmt_status qmt_density(qmt_mol* mol, int nx, int ny, int nz, float step,
  * both kernels, of which the device's decision runs one. */
 qmt_status qmt_set_density_path(int mode);
 
-/* Rank of the factor the last density call on `mol` contracted with (new): 0 when it ran the
- * unfactored kernel.  Synchronises `stream` (the device-side check decides). */
+/* Rank of the factor the last density call on `mol` contracted with (new): 0 when it ran an
+ * unfactored kernel, or when there was none since the last qmt_mol_set_dm.  Synchronises `stream`
+ * where that call left the decision to the device. */
 qmt_status qmt_density_factor_rank(qmt_mol* mol, int* rank_out, void* stream);
 
 /* ---- batches of molecules (new; no reference counterpart) ---------------------------- */

@@ -346,6 +346,7 @@ extern "C" qmt_status qmt_density(qmt_mol* mol, int nx, int ny, int nz, float st
     if ((st = mol->d_partials.reserve(ntiles * sizeof(double)))) return st;
     const double outscale = 2.0 * (double)step * step * step / s3;
     double* part = mol->d_partials.as<double>();
+    mol->last_rank = 0;
     if (!fp64) {
       if (rows == 64) st = launch_simt<float, 64>(mol, pm, ntiles, qube_dev, part, outscale, s);
       else if (rows == 32) st = launch_simt<float, 32>(mol, pm, ntiles, qube_dev, part, outscale, s);

@@ -1952,6 +1952,7 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
         return st;
     }
   }
+  mol->last_rank = fact ? rank : 0;
   const int* gate = shape ? &shape->refused : nullptr;
   if (fact && !shape) {
   } else if (fused) {
@@ -2103,8 +2104,10 @@ static qmt_status batch_run(qmt_batch* b, int rescale, bool refresh, cudaStream_
     if (!it.fused && !it.fact && (st = run_tc<FMT>(it.mol, it.sh, it.pm, it.ntiles, b->precision, it.qube, it.outscale, s,
                                        &b->phi_hi, &b->phi_lo, BATCH_STAGE_BYTES)))
       return st;
-  for (const BatchItem& it : b->items)
+  for (const BatchItem& it : b->items) {
     if ((st = finish_density(it.mol, it.pm.nvox, it.ntiles, rescale, it.qube, nullptr, s))) return st;
+    it.mol->last_rank = it.fact ? it.rank : 0;
+  }
   return QMT_OK;
 }
 
@@ -2271,10 +2274,14 @@ qmt_status qmt_batch_destroy(qmt_batch* b) {
 
 extern "C" qmt_status qmt_density_factor_rank(qmt_mol* mol, int* rank_out, void* stream) {
   if (!mol || !rank_out) return qmt::fail(QMT_BAD_ARG, "null argument");
-  *rank_out = 0;
-  if (mol->fact_prec < 0) return QMT_OK;
-  qmt_status st = qmt::factor_rank(mol, true, rank_out, qmt::as_stream(stream));
-  return st;
+  *rank_out = mol->last_rank;
+  if (mol->last_rank >= 0) return QMT_OK;
+  cudaStream_t s = qmt::as_stream(stream);
+  qmt::FactShape decision[2];
+  QMT_CUDA(cudaMemcpyAsync(decision, mol->fact_decision(), sizeof(decision), cudaMemcpyDeviceToHost, s));
+  QMT_CUDA(cudaStreamSynchronize(s));
+  *rank_out = decision[1].refused;   // the rank taken (fact_decide_kernel)
+  return QMT_OK;
 }
 
 extern "C" qmt_status qmt_set_density_path(int mode) {

@@ -165,6 +165,7 @@ qmt_status qmt_mol::upload_dm(const float* dm, cudaStream_t s) {
   tc_prec = -1;
   fused_prec = -1;
   fact_prec = -1;
+  last_rank = 0;
   gto_ready = false;
   return QMT_OK;
 }

@@ -49,6 +49,7 @@ struct qmt_mol {
   bool fact_any_rank = false;   // the rank limit they were built (or refused) with
   int fact_rank = 0;            // rank of the density-matrix factor P = L L^T (0: none, or it failed its check;
                                 // -1: known on the device only)
+  int last_rank = 0;            // rank of the factor that the last density call took (0: none; -1: see fact_decision)
   uint32_t fact_number = 0;     // number of the last factorisation, and the page-locked word in which the device
   volatile unsigned long long* fact_mail = nullptr;   // leaves (number << 32 | rank) once it is done
   qmt::DevBuf d_fact_B;         // scaled factor pieces, K-step blocks of the rank rounded up to 16 rows a piece

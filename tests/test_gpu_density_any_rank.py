@@ -30,7 +30,7 @@ def _low_rank(rank):
     return m
 
 
-def _density(mol, shape, prec, subgrid=1):
+def _density(mol, shape, prec, subgrid=1, wait=True):
     import torch
     span = float(np.ptp(np.asarray(mol.coords), axis=0).max()) + 6.0
     h = span / max(shape)
@@ -38,8 +38,8 @@ def _density(mol, shape, prec, subgrid=1):
     q = torch.empty(int(np.prod(shape)), device="cuda")
     s = C.c_double()
     N.ensure_device()
-    N.call("qmt_density", mol.handle, *shape, h, *org, subgrid, N.PREC[prec], 0, C.c_void_p(q.data_ptr()), C.byref(s),
-           N.stream_handle())
+    N.call("qmt_density", mol.handle, *shape, h, *org, subgrid, N.PREC[prec], 0, C.c_void_p(q.data_ptr()),
+           C.byref(s) if wait else None, N.stream_handle())
     return q
 
 
@@ -51,4 +51,42 @@ def test_equal_calls_give_equal_results(basis):
     before = _density(mol, SMALL, "fp16x3")
     _density(mol, LARGE, "fp16x3")
     assert torch.equal(_density(mol, SMALL, "fp16x3"), before)
+    mol.release()
+
+
+def _full_rank(n, rng):
+    q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    return (q * np.where(np.arange(n) < n // 3, 0.98, 0.02)) @ q.T
+
+
+def _rank(mol):
+    r = C.c_int()
+    N.call("qmt_density_factor_rank", mol.handle, C.byref(r), N.stream_handle())
+    return r.value
+
+
+def test_rank_of_the_last_call(basis):
+    """The rank that is asked for is that of the last call's contraction, whatever has been factored."""
+    mol = _molecule(basis, [6] * 6 + [1] * 4, _full_rank)
+    n = int(mol.norbs)
+    for shape, prec, path, rank in ((LARGE, "fp16x3", 0, n), (SMALL, "fp16x3", 0, 0), (LARGE, "fp16x3", 0, n),
+                                    (LARGE, "fp16x3", 2, 0), (LARGE, "fp16x3", 0, n), (SMALL, "fp64", 0, 0)):
+        N.call("qmt_set_density_path", path)
+        try:
+            _density(mol, shape, prec)
+        finally:
+            N.call("qmt_set_density_path", 0)
+        assert _rank(mol) == rank, (shape, prec, path)
+    mol.release()
+
+
+@pytest.mark.parametrize("rank", [20, 60, 104])
+def test_rank_of_an_asynchronous_call(basis, rank):
+    """The same where the call left the decision to the device: 104 functions, whose half is 52, rounded up to 56."""
+    mol = _molecule(basis, [6] * 6 + [1] * 4, _full_rank)
+    for shape, most in ((SMALL, 56), (LARGE, 104)):
+        mol.set_dm(_low_rank(rank)(int(mol.norbs), np.random.default_rng(7)))
+        _density(mol, shape, "fp16x3", wait=False)
+        # (an exact projector has eigenvalues 0, which the float32 matrix has to rounding: a few more pivots at most)
+        assert rank <= _rank(mol) <= most if rank <= most else _rank(mol) == 0
     mol.release()
