@@ -1897,6 +1897,15 @@ constexpr int kBf16FusedMaxR16 = 64;
 // that equal calls give equal results.
 constexpr int64_t kAnyRankTiles = 8192;
 static bool any_rank_pays(const TcShape& sh, int64_t ntiles) { return sh.fmt == FMT_F16 && ntiles >= kAnyRankTiles; }
+static bool factored_at_any_rank(const qmt_mol* m, int prec) { return m->fact_prec == prec && m->fact_any_rank; }
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {   // the default stream while another one is being captured
+    cudaGetLastError();
+    return false;
+  }
+  return c != cudaStreamCaptureStatusNone;
+}
 // The largest rank that a call takes (0: the charge rules its factor out), whatever rank an earlier call has factored.
 static int call_limit(const qmt_mol* m, const TcShape& sh, bool fused, bool any_rank) {
   const int lim = factor_limit(m, sh.fmt, any_rank);
@@ -1929,16 +1938,18 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   // The factored matrix when there is one (automatic, or asked for).  Whether there is one the device knows first.
   // A call that returns a sum, and so waits anyway, reads it; an asynchronous one takes it where the host has seen it,
   // and else launches both kernels, one of which the device's decision sends home.
-  bool fact = false;
+  bool fact = false, both = false;
   int rank = 0;
   const FactShape* shape = nullptr;
   if (sh.fmt != FMT_TF32 && g_density_path != 1 && g_density_path != 2) {
     const bool asked = g_density_path == 3;
-    bool any = !asked && any_rank_pays(sh, ntiles);
+    // (a call that is captured in a graph takes the operands that are there)
+    const bool any = !asked && any_rank_pays(sh, ntiles) && (factored_at_any_rank(mol, precision) || !capturing(s));
     if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, s)) ||
         (st = factor_rank(mol, asked || sum_out, &rank, s)))
       return st;
-    int limit = call_limit(mol, sh, fused, any);
+    const int every = call_limit(mol, sh, fused, false);   // of a call on any grid
+    int limit = any ? call_limit(mol, sh, fused, true) : every;
     if (asked) limit = std::min(limit, std::min(kFactorAskedRank, fused_n16(mol) / 2));
     fact = limit > 0 && (rank < 0 || (rank > 0 && rank <= limit));
     if (asked && !fact)
@@ -1950,10 +1961,14 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
       if ((st = launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit,
                                 reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), shape, s)))
         return st;
+      // a smaller grid's call would not take this factor, and may be captured: its operands too
+      both = !shape && rank > every && !capturing(s);
     }
   }
   mol->last_rank = fact ? rank : 0;
   const int* gate = shape ? &shape->refused : nullptr;
+  if (both && (st = fused ? ensure_fused_operands(mol, precision, sh, s) : ensure_tc_operands(mol, precision, sh, s)))
+    return st;
   if (fact && !shape) {
   } else if (fused) {
     if ((st = ensure_fused_operands(mol, precision, sh, s))) return st;

@@ -90,3 +90,41 @@ def test_rank_of_an_asynchronous_call(basis, rank):
         # (an exact projector has eigenvalues 0, which the float32 matrix has to rounding: a few more pivots at most)
         assert rank <= _rank(mol) <= most if rank <= most else _rank(mol) == 0
     mol.release()
+
+
+def _captured(mol, shape, prec):
+    """The density of an asynchronous call captured in a graph and replayed."""
+    import torch
+    span = float(np.ptp(np.asarray(mol.coords), axis=0).max()) + 6.0
+    h = span / max(shape)
+    org = [float(o) for o in np.asarray(mol.coords).mean(axis=0) - np.array(shape) * h / 2]
+    q = torch.zeros(int(np.prod(shape)), device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        N.call("qmt_density", mol.handle, *shape, h, *org, 1, N.PREC[prec], 0, C.c_void_p(q.data_ptr()), None,
+               N.stream_handle())
+    g.replay()
+    torch.cuda.synchronize()
+    return q
+
+
+def test_a_small_grid_is_captured_after_a_large_one(basis):
+    """The operands of every grid exist after the first call."""
+    import torch
+    mol = _molecule(basis, [6] * 6 + [1] * 4, _full_rank)
+    _density(mol, LARGE, "fp16x3")
+    q = _captured(mol, SMALL, "fp16x3")
+    assert torch.equal(q, _density(mol, SMALL, "fp16x3"))
+    mol.release()
+
+
+def test_a_large_grid_is_captured_after_a_small_one(basis):
+    import torch
+    mol = _molecule(basis, [6] * 6 + [1] * 4, _full_rank)
+    ref = _density(mol, LARGE, "fp64")          # (this also makes the buffers that the large grid needs)
+    _density(mol, SMALL, "fp16x3")
+    q = _captured(mol, LARGE, "fp16x3")
+    # an FP32 addition per K-step, doubled by the square, and two operands of 2^-21
+    tol = 2 * (int(mol.norbs) / 16 + 2) * 2.0 ** -23 + 4 * 2.0 ** -21
+    assert ((q.double() - ref.double()).norm() / ref.double().norm()).item() <= tol
+    mol.release()
