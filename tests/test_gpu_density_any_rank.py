@@ -128,3 +128,66 @@ def test_a_large_grid_is_captured_after_a_small_one(basis):
     tol = 2 * (int(mol.norbs) / 16 + 2) * 2.0 ** -23 + 4 * 2.0 ** -21
     assert ((q.double() - ref.double()).norm() / ref.double().norm()).item() <= tol
     mol.release()
+
+
+def _indefinite(n, rng):
+    q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    return (q * np.where(np.arange(n) < n // 3, 0.98, np.where(np.arange(n) < n - 3, 0.02, -0.05))) @ q.T
+
+
+# 15, 42, 104, 148 and 256 functions, and 270, above the limit
+FULL = [[1] * 3, [6] * 3, [6] * 6 + [1] * 4, [35, 17, 17] + [6] * 5 + [1] * 3, [6] * 17 + [17] * 1, [6] * 18 + [17]]
+
+
+@pytest.mark.parametrize("zs", FULL, ids=[str(len(z)) for z in FULL])
+@pytest.mark.parametrize("matrix", [_full_rank, _indefinite], ids=["definite", "indefinite"])
+def test_full_rank_matrices_on_large_grids(basis, zs, matrix):
+    """Against the FP64 path, on a 2^3 subgrid as training takes it and on single points, with the same molecule on a
+    small grid before and after."""
+    import torch
+    mol = _molecule(basis, zs, matrix)
+    n = int(mol.norbs)
+    # an FP32 addition per K-step, doubled by the square of the factored contraction, or the row products' partial sums;
+    # operands of 2^-21 each.  An indefinite matrix's terms cancel: as much again.
+    tol = (2 * (n / 16 + 2) * 2.0 ** -23 + 4 * 2.0 ** -21) * (2 if matrix is _indefinite else 1)
+
+    def off(a, b):
+        return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+    small = _density(mol, SMALL, "fp16x3")
+    assert _rank(mol) == 0
+    assert off(small, _density(mol, SMALL, "fp64")) <= tol
+    for shape, sub in ((LARGE, 1), ((56, 48, 56), 2)):
+        ref = _density(mol, shape, "fp64", sub)
+        got = _density(mol, shape, "fp16x3", sub)
+        assert _rank(mol) == (n if n <= 256 and matrix is _full_rank else 0)
+        assert off(got, ref) <= tol
+    assert torch.equal(_density(mol, SMALL, "fp16x3"), small)
+    mol.release()
+
+
+def test_full_rank_matrix_in_a_batch(basis, tmp_path):
+    """One factored launch of a full-rank and a low-rank molecule, the full-rank one on a grid where it pays."""
+    from qmtools.autotune import Tuner
+    from qmtools.batch import BatchEvaluator
+    mols = [_molecule(basis, [6] * 6 + [1] * 4, _full_rank), _molecule(basis, [6] * 6, _low_rank(17)),
+            _molecule(basis, [6] * 6 + [1] * 4, _full_rank, 1)]
+    shapes = [LARGE, (24, 32, 16), SMALL]
+    grids = []
+    for m, shape in zip(mols, shapes):
+        c = np.asarray(m.coords)
+        h = (float(np.ptp(c, axis=0).max()) + 6.0) / max(shape)
+        grids.append(qmtools.Grid((1,) + shape, h / qmtools.ANG2BOR, list(c.mean(axis=0) - np.array(shape) * h / 2)))
+    ev = BatchEvaluator(mols, grids, tuner=Tuner(path=tmp_path / "t.json", measure=False), hartree=False)
+    try:
+        assert ev.factored_count == 2
+        ev.run()
+        ev.synchronize()
+        for k, (m, g) in enumerate(zip(mols, grids)):
+            ref = qmtools.QMTools.Compute_density(g, m, precision="fp64").qube.ravel()
+            tol = 2 * (int(m.norbs) / 16 + 2) * 2.0 ** -23 + 4 * 2.0 ** -21
+            assert np.linalg.norm(ev.density(k).ravel() - ref) <= tol * np.linalg.norm(ref)
+    finally:
+        ev.close()
+        for m in mols:
+            m.release()
