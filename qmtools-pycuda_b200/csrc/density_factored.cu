@@ -76,13 +76,10 @@ struct FactParams {
   int nmol;
   int64_t ntiles;
   uint32_t fmt;
-  uint32_t nslots;         // ring slots
-  uint32_t slot_magic;     // ceil(2^32 / nslots): group / nslots = umulhi(group, magic) below 2^28
-  uint32_t slot_bytes;     // A pieces, then (streamed factor) the factor's K-step block
-  uint32_t resident;       // the whole factor behind the ring, loaded once (single molecule)
+  FactPlan plan;
   int* err;
   uint64_t wait_ns;
-  const FactShape* shape;  // ON_DEVICE: the device's decision (the factor is streamed)
+  const FactDecision* decision;   // ON_DEVICE: the device's, in place of the host's shape and plan
 };
 
 __host__ __device__ inline FactShape fact_shape(int rank, int nunits) {
@@ -102,8 +99,25 @@ __host__ __device__ inline FactShape fact_shape(int rank, int nunits) {
 
 template <int WHO>
 __device__ __forceinline__ FactShape fact_shape_of(const FactParams& p, const FactMol& m) {
-  if (WHO == ON_DEVICE) return *p.shape;
+  if (WHO == ON_DEVICE) return p.decision->shape;
   return FactShape{0, m.r16, m.sets, m.na};
+}
+
+// The factor stays in shared memory when at least MIN_SLOTS slots fit beside it; else its blocks (blk bytes each) stream
+// through the slots.
+__host__ __device__ inline FactPlan fact_plan(int64_t avail, int abytes, int blk, int nunits, bool one) {
+  const int64_t whole = (int64_t)blk * nunits;
+  FactPlan f;
+  f.resident = one && whole + MIN_SLOTS * abytes <= avail ? 1 : 0;
+  f.slot_bytes = (uint32_t)(abytes + (f.resident ? 0 : GROUP * blk));
+  const int64_t fit = (avail - (f.resident ? whole : 0)) / f.slot_bytes;
+  f.nslots = fit < MAX_SLOTS ? (uint32_t)fit : (uint32_t)MAX_SLOTS;
+  f.slot_magic = f.nslots ? (uint32_t)(((1ull << 32) + f.nslots - 1) / f.nslots) : 0u;
+  return f;
+}
+template <int WHO>
+__device__ __forceinline__ FactPlan fact_plan_of(const FactParams& p) {
+  return WHO == ON_DEVICE ? p.decision->plan : p.plan;
 }
 
 template <bool MULTI>
@@ -442,7 +456,8 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
   uint32_t s = 0, ph = 0, tile_it = 0;   // slot and its phase
   int last_sets = 2;
   const bool leader = elect_one();
-  const bool streamed = WHO != ONE || !p.resident;
+  const FactPlan plan = fact_plan_of<WHO>(p);
+  const bool streamed = MULTI || !plan.resident;
   const uint32_t ring0 = smem_u32(smem);
   constexpr uint32_t UNIT_A = TWO ? 2 * PIECE : PIECE, ABYTES = GROUP * UNIT_A;
   bool ok = true, ready = false;
@@ -474,9 +489,9 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
       if (!ok) break;
       tc_fence_after();
       // the next group's state, read while this one's MMAs are issued
-      const uint32_t sn = s + 1 == p.nslots ? 0 : s + 1, phn = s + 1 == p.nslots ? ph ^ 1u : ph;
+      const uint32_t sn = s + 1 == plan.nslots ? 0 : s + 1, phn = s + 1 == plan.nslots ? ph ^ 1u : ph;
       const bool peek = mbar_test_wait(&B.a_full[sn], phn);
-      const uint32_t slot = ring0 + s * p.slot_bytes;
+      const uint32_t slot = ring0 + s * plan.slot_bytes;
       uint32_t a = slot, b = streamed ? slot + ABYTES : bres;
 #pragma unroll
       for (int k = 0; k < GROUP; ++k) {
@@ -527,7 +542,7 @@ template <int FMT, bool TWO, int WHO>
 __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const __grid_constant__ FactParams p) {
   constexpr bool MULTI = WHO == MANY;
   extern __shared__ uint8_t smem_dyn[];
-  if (WHO == ON_DEVICE && p.shape->refused) return;   // the unfactored launch of the pair does the work
+  if (WHO == ON_DEVICE && p.decision->shape.refused) return;   // the unfactored launch of the pair does the work
   __shared__ FactBars B;
   __shared__ __align__(16) float4 pos_s[POS_DEPTH][3][64];   // {hi r, hi r + 64, lo r, lo r + 64}
   __shared__ double rho_s[128];
@@ -537,10 +552,11 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const uint32_t nslots = p.nslots;
+  const FactPlan plan = fact_plan_of<WHO>(p);
+  const uint32_t nslots = plan.nslots;
   constexpr uint32_t UNIT_A = TWO ? 2 * PIECE : PIECE, ABYTES = GROUP * UNIT_A;
   constexpr uint32_t NISSUE = TWO ? 2 : 1;   // MMA-issuing warps
-  uint8_t* res = smem + (size_t)nslots * p.slot_bytes;   // the resident factor
+  uint8_t* res = smem + (size_t)nslots * plan.slot_bytes;   // the resident factor
 
   if (threadIdx.x == 0) {
     B.abort_flag = 0;
@@ -574,8 +590,8 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
   if (warp == 0) {
     // ---- the factor's K-step blocks ------------------------------------------------------------
     if (lane == 0) {
-      if (WHO == ONE && p.resident) {
-        const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * (uint32_t)p.one.r16 * 32u;
+      if (!MULTI && plan.resident) {
+        const uint32_t blk = (uint32_t)(TWO ? 2 : 1) * (uint32_t)fact_shape_of<WHO>(p, p.one).r16 * 32u;
         mbar_expect_tx(&B.res_bar, blk * (uint32_t)p.one.nunits);
         for (int u = 0; u < p.one.nunits; ++u) bulk_load(res + (size_t)u * blk, p.one.B + (size_t)u * blk, blk, &B.res_bar);
         mbar_wait_drain(&B.res_bar, 0u, p.wait_ns < 100000000ull ? 100000000ull : p.wait_ns);
@@ -596,7 +612,7 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
             }
             const uint32_t bytes = blk * (uint32_t)min(GROUP, nunits - u);
             mbar_expect_tx(&B.b_full[s], bytes);
-            bulk_load(smem + (size_t)s * p.slot_bytes + ABYTES, src, bytes, &B.b_full[s]);
+            bulk_load(smem + (size_t)s * plan.slot_bytes + ABYTES, src, bytes, &B.b_full[s]);
             issued |= 1u << s;
             par = (par & ~(1u << s)) | (ph << s);
             if (++s == nslots) {
@@ -768,7 +784,7 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
       }
       if (t >= p.ntiles) break;
       const int u = (itm - base) >> 1, r0 = ((itm - base) & 1) * 32 + lane;
-      const uint32_t kg = kg0 + (uint32_t)(u / GROUP), round = __umulhi(kg, p.slot_magic), s = kg - round * nslots;
+      const uint32_t kg = kg0 + (uint32_t)(u / GROUP), round = __umulhi(kg, plan.slot_magic), s = kg - round * nslots;
       const uint32_t ph = round & 1u, b = tile_it % POS_DEPTH;
       const int4 u0 = __ldg(units + 2 * u), u1 = __ldg(units + 2 * u + 1);
       if ((seen != tile_it && !mbar_wait_warp(&B.pos_full[b], (tile_it / POS_DEPTH) & 1u, &B.abort_flag, p.wait_ns)) ||
@@ -777,7 +793,7 @@ __global__ void __launch_bounds__(FACT_THREADS, 1) density_factored_kernel(const
       seen = tile_it;
       // (the next item is taken only now: a warp holds at most one item that has not passed its waits)
       if (lane == 0) nxt = atomicAdd(&item_ctr, 1);
-      uint8_t* slot = smem + (size_t)s * p.slot_bytes + (u % GROUP) * UNIT_A;
+      uint8_t* slot = smem + (size_t)s * plan.slot_bytes + (u % GROUP) * UNIT_A;
       const float4* tab = reinterpret_cast<const float4*>(units);
       const int kind = u0.x & 0xff;
       if (kind == UNIT_S8S8S1P3P1D1)
@@ -953,7 +969,11 @@ struct PivotArgs {
   int ld0;                    // (at least rmax rounded up to 16)
   int* info;
   double* dmax;               // the first pivot
+  int* usable;                // as fact_split_kernel leaves them, here where there is no factor; else the word's
+  uint32_t number;            // kMailPending
+  volatile unsigned long long* mail;
 };
+constexpr unsigned kMailPending = 1u << 30;   // there is a rank, the check is to come
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
   uint32_t r;
@@ -1081,8 +1101,11 @@ __global__ void __launch_bounds__(PIV_THREADS, 1) fact_pivot_kernel(PivotArgs a)
   for (int i = t; i < nr * pad; i += PIV_THREADS) a.L0[(size_t)(r0 + i / pad) * a.ld0 + q + i % pad] = 0.f;
   if (ncta > 1) cluster_barrier();   // no CTA leaves while another may still read its shared memory; every [1] is in
   if (c == 0 && t == 0) {
-    a.info[0] = __ldcg(a.info + 1) || q > a.limit ? 0 : q;
+    const int r = __ldcg(a.info + 1) || q > a.limit ? 0 : q;
+    a.info[0] = r;
     *a.dmax = dmax;
+    if (r == 0) *a.usable = 0;
+    *a.mail = (unsigned long long)a.number << 32 | (r ? kMailPending | (unsigned)r : 0u);
   }
 }
 
@@ -1358,11 +1381,14 @@ __global__ void fact_split_kernel(const double* __restrict__ L, const int* __res
   }
 }
 
-// The device's decision for a call that takes ranks up to `limit` (out[1].refused: the rank taken).
-__global__ void fact_decide_kernel(const int* __restrict__ usable, int limit, int nunits, FactShape* out) {
+// The device's decision for a call that takes ranks up to `limit`.
+__global__ void fact_decide_kernel(const int* __restrict__ usable, int limit, int nunits, int64_t avail, int abytes,
+                                   int nsplit, FactDecision* out) {
   const int r = *usable <= limit ? *usable : 0;
-  out[0] = fact_shape(r, nunits);
-  out[1].refused = r;
+  const FactShape f = fact_shape(r, nunits);
+  out->shape = f;
+  out->plan = fact_plan(avail, abytes, nsplit * f.r16 * 32, nunits, true);
+  out->rank = r;
 }
 
 constexpr int kBf16MaxRank = 128;
@@ -1371,16 +1397,17 @@ constexpr double kFactorResid = 2e-7;
 
 }  // namespace
 
-static qmt_status launch_pivot(const double* P, int np, int n, int rmax, int limit, double* L, float* L0, int ld0,
-                               int* info, double* dmax, cudaStream_t s) {
+static qmt_status launch_pivot(qmt_mol* m, int rmax, int limit, double* L, float* L0, int ld0, int* info, double* dmax,
+                               cudaStream_t s) {
+  const int n = m->norbs;
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   QMT_CUDA(cudaFuncSetAttribute(fact_pivot_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   for (int ncta = n > 320 ? PIV_MAX_CTAS : (n > 128 ? 8 : 1); ncta >= 1; ncta /= 2) {
     PivotArgs a{};
-    a.P = P;
-    a.np = np;
+    a.P = m->d_P64.as<double>();
+    a.np = m->npad;
     a.n = n;
     a.rmax = rmax;
     a.rows = (n + ncta - 1) / ncta;
@@ -1392,6 +1419,9 @@ static qmt_status launch_pivot(const double* P, int np, int n, int rmax, int lim
     a.ld0 = ld0;
     a.info = info;
     a.dmax = dmax;
+    a.usable = m->fact_usable();
+    a.number = m->fact_number;
+    a.mail = m->fact_mail;
     const size_t base = (size_t)(a.rows + rmax) * sizeof(double), rows = (size_t)a.rows * a.ld * sizeof(double);
     if (base > (size_t)maxsm - 2048) continue;
     a.rows_in_smem = base + rows <= (size_t)maxsm - 2048 ? 1 : 0;
@@ -1446,15 +1476,40 @@ int factor_limit(const qmt_mol* m, int fmt, bool any_rank) {
   return 0.5 * m->qtot > std::max(16, lim) + 8 ? 0 : lim;
 }
 
+// What the device has left of the molecule's last factorisation in the page-locked word; with `pending` also a rank that
+// is still to be checked.
+static bool mail_arrived(const qmt_mol* m, unsigned pending, unsigned* word) {
+  const unsigned long long mail = *m->fact_mail;
+  *word = (unsigned)mail;
+  return (uint32_t)(mail >> 32) == m->fact_number && !(*word & kMailPending & ~pending);
+}
+// Polled for as long as the stream works: the word is there before a copy of the rank and a synchronisation would have
+// been (a first call with a sum, 16^3 points: 218 -> 208 us).
+static qmt_status read_mail(qmt_mol* m, unsigned pending, unsigned* word, cudaStream_t s) {
+  for (;;) {
+    const cudaError_t e = cudaStreamQuery(s);   // (before the look: what the stream has done is then there)
+    if (mail_arrived(m, pending, word)) {
+      if (e == cudaErrorNotReady) cudaGetLastError();   // (the query leaves its answer there)
+      return QMT_OK;
+    }
+    if (e != cudaErrorNotReady) {
+      QMT_CUDA(e);
+      return fail(QMT_CUDA_ERR, "the factorisation left no rank");
+    }
+    cudaGetLastError();
+  }
+}
+
 // A density matrix of rank r (r = occupied orbitals for an SCF density, P = 2 C_occ C_occ^T) is
 // P = L L^T with L n x r.  L comes from a pivoted Cholesky factorisation (fact_pivot_kernel), stopped
 // once every remaining diagonal element is at most kFactorTol of the largest one, and is refined; it is
 // used when the matrix it leaves out is at most kFactorResid of max |P| (float32 input rounding is
 // ~6e-8).  A matrix that is not positive semi-definite, or of high rank, takes the unfactored path.
 // The scaled factor W_jk = L_jk 2^(h_k - s_j) (so Phi' W = 2^h_k (Phi L)_k, each column scaled to a
-// maximum near 2^14) goes to the blocks of fact_split_kernel.  Nothing waits: the rank and the check stay on the
-// device until factor_rank reads them.
-qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, cudaStream_t s) {
+// maximum near 2^14) goes to the blocks of fact_split_kernel.  Unless the call may wait, nothing does: the rank and the
+// check stay on the device until factor_rank reads them.
+qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, bool wait,
+                         cudaStream_t s) {
   qmt_status st;
   // built for this precision (rank -1: the device knows), or refused by at least this rank limit
   int rank = 0;
@@ -1494,7 +1549,18 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   const double* P = m->d_P64.as<double>();
   const int r16max = (rmax + 15) / 16 * 16;   // <= rbuf
   QMT_CUDA(cudaMemsetAsync(colmax, 0, (rbuf + 8) * sizeof(double), s));
-  if ((st = launch_pivot(P, np, n, rmax, limit, Lp, L0, rbuf, info, dmax, s))) return st;
+  if (++m->fact_number == 0) m->fact_number = 1;
+  if ((st = launch_pivot(m, rmax, limit, Lp, L0, rbuf, info, dmax, s))) return st;
+  if (wait) {   // the pivots alone may refuse the matrix, and the rest need not run
+    unsigned word = 0;
+    if ((st = read_mail(m, kMailPending, &word, s))) return st;
+    if (word == 0) {
+      m->fact_prec = prec;
+      m->fact_any_rank = any_rank;
+      m->fact_rank = 0;
+      return QMT_OK;
+    }
+  }
   // refined, and what the factor then leaves out, max |P - L L^T|, checked
   fact_y_kernel<<<dim3((n + 31) / 32, (r16max + 31) / 32), 256, 0, s>>>(P, np, L0, rbuf, n, info, Y);
   QMT_CHECK_LAUNCH("fact_y_kernel");
@@ -1516,7 +1582,6 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   QMT_CHECK_LAUNCH("fact_residual_kernel");
   const int64_t tot = (int64_t)m->fact_units * 16 * r16max;
   const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
-  if (++m->fact_number == 0) m->fact_number = 1;
   fact_split_kernel<<<std::max(blocks, 1), 256, 0, s>>>(
       Y, info, reinterpret_cast<const int*>(m->d_fact_tab.as<uint8_t>() + m->fact_col_off), m->fact_units,
       m->d_split_scale.as<double>(), two_h, fmt, nsplit, m->d_fact_B.as<uint8_t>(), bad, m->fact_usable(), m->fact_number,
@@ -1529,26 +1594,17 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
 }
 
 qmt_status factor_rank(qmt_mol* m, bool wait, int* rank, cudaStream_t s) {
+  unsigned word = 0;
   if (m->fact_rank < 0) {
-    const unsigned long long mail = *m->fact_mail;
-    if ((uint32_t)(mail >> 32) == m->fact_number) {
-      m->fact_rank = (int)(uint32_t)mail;
+    if (mail_arrived(m, 0, &word)) {
+      m->fact_rank = (int)word;
     } else if (wait) {
-      int got = 0;
-      QMT_CUDA(cudaMemcpyAsync(&got, m->fact_usable(), sizeof(got), cudaMemcpyDeviceToHost, s));
-      QMT_CUDA(cudaStreamSynchronize(s));
-      m->fact_rank = got;
+      qmt_status st = read_mail(m, 0, &word, s);
+      if (st) return st;
+      m->fact_rank = (int)word;
     }
   }
   *rank = m->fact_rank;
-  return QMT_OK;
-}
-
-qmt_status decide_on_device(qmt_mol* m, int limit, const FactShape** shape, cudaStream_t s) {
-  FactShape* out = reinterpret_cast<FactShape*>(m->fact_decision());
-  fact_decide_kernel<<<1, 1, 0, s>>>(m->fact_usable(), limit, m->fact_units, out);
-  QMT_CHECK_LAUNCH("fact_decide_kernel");
-  *shape = out;
   return QMT_OK;
 }
 
@@ -1574,8 +1630,9 @@ void fact_mol_desc(const qmt_mol* m, int rank, const PointMap& pm, int64_t tile0
 
 namespace {
 
+// `blk`: bytes of the largest K-step block of the launch.  ON_DEVICE asks the device to decide for ranks up to `limit`.
 template <int FMT, bool TWO, int WHO>
-qmt_status launch_as(FactParams& p, int blk_max, int nunits, cudaStream_t s) {
+qmt_status launch_as(FactParams& p, int blk, const int* usable, int limit, cudaStream_t s) {
   auto kern = density_factored_kernel<FMT, TWO, WHO>;
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
@@ -1584,35 +1641,46 @@ qmt_status launch_as(FactParams& p, int blk_max, int nunits, cudaStream_t s) {
   QMT_CUDA(cudaFuncGetAttributes(&fa, kern));
   const int64_t avail = (int64_t)maxsm - (int64_t)fa.sharedSizeBytes - 1024;
   const int abytes = GROUP * (TWO ? 2 * (int)PIECE : (int)PIECE);
-  // the factor stays in shared memory when at least MIN_SLOTS slots fit beside it; else its blocks
-  // stream through the slots
-  const int64_t whole = (int64_t)blk_max * nunits;
-  p.resident = WHO == ONE && whole + MIN_SLOTS * abytes <= avail ? 1 : 0;
-  p.slot_bytes = (uint32_t)(abytes + (p.resident ? 0 : GROUP * blk_max));
-  const int64_t room = avail - (p.resident ? whole : 0);
-  p.nslots = (uint32_t)std::min<int64_t>(MAX_SLOTS, room / p.slot_bytes);
-  if (p.nslots < (uint32_t)MIN_SLOTS) return fail(QMT_BAD_ARG, "factored density slots do not fit in shared memory");
-  p.slot_magic = (uint32_t)(((1ull << 32) + p.nslots - 1) / p.nslots);
-  const size_t dyn = (size_t)p.slot_bytes * p.nslots + (p.resident ? whole : 0) + 1024;
-  QMT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  // (streamed, the largest rank has the fewest slots)
+  if (fact_plan(avail, abytes, blk, p.one.nunits, false).nslots < (uint32_t)MIN_SLOTS)
+    return fail(QMT_BAD_ARG, "factored density slots do not fit in shared memory");
+  p.plan = fact_plan(avail, abytes, blk, p.one.nunits, WHO == ONE);
+  size_t dyn = (size_t)p.plan.slot_bytes * p.plan.nslots + (p.plan.resident ? (size_t)blk * p.one.nunits : 0) + 1024;
   const int grid = (int)std::min<int64_t>(p.ntiles, sm_count());
   if (grid <= 0) return QMT_OK;
+  if (WHO == ON_DEVICE) {
+    dyn = (size_t)avail + 1024;
+    fact_decide_kernel<<<1, 1, 0, s>>>(usable, limit, p.one.nunits, avail, abytes, TWO ? 2 : 1,
+                                       const_cast<FactDecision*>(p.decision));
+    QMT_CHECK_LAUNCH("fact_decide_kernel");
+  }
+  QMT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   kern<<<grid, FACT_THREADS, dyn, s>>>(p);
   QMT_CHECK_LAUNCH("density_factored_kernel");
   return QMT_OK;
 }
 
 template <int FMT, bool TWO>
-qmt_status launch_whose(FactParams& p, int blk_max, cudaStream_t s) {
-  if (p.nmol > 1) return launch_as<FMT, TWO, MANY>(p, blk_max, 0, s);
-  if (p.shape) return launch_as<FMT, TWO, ON_DEVICE>(p, blk_max, p.one.nunits, s);
-  return launch_as<FMT, TWO, ONE>(p, blk_max, p.one.nunits, s);
+qmt_status launch_whose(FactParams& p, int blk, const int* usable, int limit, cudaStream_t s) {
+  if (p.nmol > 1) return launch_as<FMT, TWO, MANY>(p, blk, usable, limit, s);
+  if (p.decision) return launch_as<FMT, TWO, ON_DEVICE>(p, blk, usable, limit, s);
+  return launch_as<FMT, TWO, ONE>(p, blk, usable, limit, s);
+}
+
+qmt_status launch_params(FactParams& p, int r16, int fmt, int nsplit, const int* usable, int limit, int* err,
+                         cudaStream_t s) {
+  p.fmt = (uint32_t)fmt;
+  p.err = err;
+  p.wait_ns = wait_limit_ns();
+  const int blk = nsplit * r16 * 32;
+  if (fmt == 0) return launch_whose<0, true>(p, blk, usable, limit, s);
+  return nsplit == 2 ? launch_whose<1, true>(p, blk, usable, limit, s) : launch_whose<1, false>(p, blk, usable, limit, s);
 }
 
 }  // namespace
 
 qmt_status launch_factored(const FactMol* host, const FactMol* dev, int nmol, int64_t ntiles, int fmt, int nsplit,
-                           int* err, const FactShape* shape, cudaStream_t s) {
+                           int* err, cudaStream_t s) {
   FactParams p{};
   int r16 = 0;
   for (int i = 0; i < nmol; ++i) r16 = std::max(r16, host[i].r16);
@@ -1620,13 +1688,17 @@ qmt_status launch_factored(const FactMol* host, const FactMol* dev, int nmol, in
   p.mols = dev;
   p.nmol = nmol;
   p.ntiles = ntiles;
-  p.fmt = (uint32_t)fmt;
-  p.err = err;
-  p.wait_ns = wait_limit_ns();
-  p.shape = shape;
-  const int blk = nsplit * r16 * 32;
-  if (fmt == 0) return launch_whose<0, true>(p, blk, s);
-  return nsplit == 2 ? launch_whose<1, true>(p, blk, s) : launch_whose<1, false>(p, blk, s);
+  return launch_params(p, r16, fmt, nsplit, nullptr, 0, err, s);
+}
+
+qmt_status launch_factored_on_device(qmt_mol* m, const FactMol& d, int limit, int fmt, int nsplit, int* err,
+                                     const FactDecision** decision, cudaStream_t s) {
+  FactParams p{};
+  p.one = d;
+  p.nmol = 1;
+  p.ntiles = d.ntiles;
+  *decision = p.decision = reinterpret_cast<const FactDecision*>(m->fact_decision());
+  return launch_params(p, d.r16, fmt, nsplit, m->fact_usable(), limit, err, s);
 }
 
 }  // namespace qmt

@@ -16,6 +16,21 @@ struct FactShape {
   int na;                  // H accumulators: up to three where two buffers hold them, else one
 };
 
+// Shared memory of a launch: the ring, then the factor where it stays.
+struct FactPlan {
+  uint32_t nslots;         // ring slots
+  uint32_t slot_magic;     // ceil(2^32 / nslots): group / nslots = umulhi(group, magic) below 2^28
+  uint32_t slot_bytes;     // A pieces, then (streamed factor) the factor's K-step block
+  uint32_t resident;       // the whole factor behind the ring, loaded once (single molecule)
+};
+
+// What the device leaves for a launch whose rank the host does not know.
+struct FactDecision {
+  FactShape shape;
+  FactPlan plan;
+  int rank;                // 0: refused
+};
+
 // One molecule of a factored launch.  A launch covers the tiles of one or more molecules; global
 // tile t belongs to the molecule with tile0 <= t < tile0 + ntiles.
 struct FactMol {
@@ -39,20 +54,22 @@ qmt_status ensure_unit_tables(qmt_mol* m, const std::vector<float>& fs, cudaStre
 // Largest rank that a call may take: half of N; with `any_rank` (fp16x3 and many sample points) any rank of up to
 // 256 functions.  0 when the nuclear charge already bounds the rank above it.
 int factor_limit(const qmt_mol* m, int fmt, bool any_rank);
-// Enqueues P = L L^T and the split factor, where they are not there yet, without waiting.
-qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, cudaStream_t s);
+// Enqueues P = L L^T and the split factor, where they are not there yet, without waiting unless it may.
+qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bool any_rank, bool wait,
+                         cudaStream_t s);
 // The factor's rank, 0 when there is none that passed its check; -1 while only the device knows (wait: never).
 qmt_status factor_rank(qmt_mol* m, bool wait, int* rank, cudaStream_t s);
-// Enqueues the device's own decision for a call that takes ranks up to `limit`; the shape it leaves on the device.
-qmt_status decide_on_device(qmt_mol* m, int limit, const FactShape** shape, cudaStream_t s);
 // Descriptor of the molecule in a launch, its tiles starting at global tile `tile0`, for a factor of rank `rank`.
 void fact_mol_desc(const qmt_mol* m, int rank, const PointMap& pm, int64_t tile0, int64_t ntiles, float* qube,
                    double outscale, FactMol& d);
 // One persistent launch over the tiles of one molecule (host descriptor), or of nmol > 1 (device
-// array `dev`, host copies for the shared-memory plan).  With `shape` (one molecule) the device has the rank, and the
-// host's descriptor the largest one that it may be.
+// array `dev`, host copies for the shared-memory plan).
 qmt_status launch_factored(const FactMol* host, const FactMol* dev, int nmol, int64_t ntiles, int fmt, int nsplit,
-                           int* err, const FactShape* shape, cudaStream_t s);
+                           int* err, cudaStream_t s);
+// The launch of a molecule whose rank only the device knows, `d` described for the largest rank that the call takes:
+// the device decides first, and what it decided is left in *decision.
+qmt_status launch_factored_on_device(qmt_mol* m, const FactMol& d, int limit, int fmt, int nsplit, int* err,
+                                     const FactDecision** decision, cudaStream_t s);
 
 // Column scales and producer tables, once per molecule (density_tc.cu).
 qmt_status ensure_basis_operands(qmt_mol* m, int K, cudaStream_t s);

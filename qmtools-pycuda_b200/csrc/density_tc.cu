@@ -1940,13 +1940,14 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
   // and else launches both kernels, one of which the device's decision sends home.
   bool fact = false, both = false;
   int rank = 0;
-  const FactShape* shape = nullptr;
+  const FactDecision* decision = nullptr;
   if (sh.fmt != FMT_TF32 && g_density_path != 1 && g_density_path != 2) {
     const bool asked = g_density_path == 3;
     // (a call that is captured in a graph takes the operands that are there)
     const bool any = !asked && any_rank_pays(sh, ntiles) && (factored_at_any_rank(mol, precision) || !capturing(s));
-    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, s)) ||
-        (st = factor_rank(mol, asked || sum_out, &rank, s)))
+    const bool wait = asked || sum_out;
+    if ((st = ensure_factor(mol, precision, sh.fmt, sh.nsplit, sh.kpad, any, wait, s)) ||
+        (st = factor_rank(mol, wait, &rank, s)))
       return st;
     const int every = call_limit(mol, sh, fused, false);   // of a call on any grid
     int limit = any ? call_limit(mol, sh, fused, true) : every;
@@ -1955,21 +1956,21 @@ qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox
     if (asked && !fact)
       return fail(QMT_BAD_ARG, "factored density path needs a positive semi-definite density matrix of low rank");
     if (fact) {
-      if (rank < 0 && (st = decide_on_device(mol, limit, &shape, s))) return st;
       FactMol d;
+      int* err = reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8);
       fact_mol_desc(mol, rank < 0 ? limit : rank, pm, 0, ntiles, qube, outscale, d);
-      if ((st = launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit,
-                                reinterpret_cast<int*>(mol->d_scalars.as<double>() + 8), shape, s)))
-        return st;
+      st = rank < 0 ? launch_factored_on_device(mol, d, limit, sh.fmt, sh.nsplit, err, &decision, s)
+                    : launch_factored(&d, nullptr, 1, ntiles, sh.fmt, sh.nsplit, err, s);
+      if (st) return st;
       // a smaller grid's call would not take this factor, and may be captured: its operands too
-      both = !shape && rank > every && !capturing(s);
+      both = !decision && rank > every && !capturing(s);
     }
   }
   mol->last_rank = fact ? rank : 0;
-  const int* gate = shape ? &shape->refused : nullptr;
+  const int* gate = decision ? &decision->shape.refused : nullptr;
   if (both && (st = fused ? ensure_fused_operands(mol, precision, sh, s) : ensure_tc_operands(mol, precision, sh, s)))
     return st;
-  if (fact && !shape) {
+  if (fact && !decision) {
   } else if (fused) {
     if ((st = ensure_fused_operands(mol, precision, sh, s))) return st;
     if (sh.fmt == FMT_F16) st = run_fused<FMT_F16>(mol, sh, pm, ntiles, qube, outscale, s, gate, 1);
@@ -2111,7 +2112,7 @@ static qmt_status batch_run(qmt_batch* b, int rescale, bool refresh, cudaStream_
     constexpr int F = FMT == FMT_TF32 ? FMT_F16 : FMT;
     if (!b->fact.empty() &&
         (st = launch_factored(b->fact.data(), b->d_fact.as<FactMol>(), (int)b->fact.size(), b->fact_tiles, F, b->nsplit,
-                              b->d_err.as<int>(), nullptr, s)))
+                              b->d_err.as<int>(), s)))
       return st;
     if ((st = batch_launch<F>(b, b->fused, s))) return st;
   }
@@ -2173,7 +2174,7 @@ qmt_status qmt_batch_create(int nmol, qmt_mol* const* mols, const int32_t* shape
     it.fact = false;
     if (path == 3 && it.sh.fmt != FMT_TF32) {   // factored when the matrix has a factor that passes the check
       const bool any = any_rank_pays(it.sh, it.ntiles);
-      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, any, s)) ||
+      if ((st = ensure_factor(m, precision, it.sh.fmt, it.sh.nsplit, it.sh.kpad, any, true, s)) ||
           (st = factor_rank(m, true, &it.rank, s)))
         break;
       it.fact = it.rank > 0 && it.rank <= call_limit(m, it.sh, it.fused, any);
@@ -2292,10 +2293,10 @@ extern "C" qmt_status qmt_density_factor_rank(qmt_mol* mol, int* rank_out, void*
   *rank_out = mol->last_rank;
   if (mol->last_rank >= 0) return QMT_OK;
   cudaStream_t s = qmt::as_stream(stream);
-  qmt::FactShape decision[2];
-  QMT_CUDA(cudaMemcpyAsync(decision, mol->fact_decision(), sizeof(decision), cudaMemcpyDeviceToHost, s));
+  qmt::FactDecision d;
+  QMT_CUDA(cudaMemcpyAsync(&d, mol->fact_decision(), sizeof(d), cudaMemcpyDeviceToHost, s));
   QMT_CUDA(cudaStreamSynchronize(s));
-  *rank_out = decision[1].refused;   // the rank taken (fact_decide_kernel)
+  *rank_out = d.rank;
   return QMT_OK;
 }
 
