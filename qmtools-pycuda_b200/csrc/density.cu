@@ -207,12 +207,9 @@ template <typename T, int TP>
 static size_t simt_smem(int npad, bool resident) {
   return sizeof(T) * ((size_t)(resident ? npad : 32) * 16 * simt_cpt(npad) + (size_t)TP * (npad + 16 / (TP / 16)));
 }
-// P stays in shared memory while three CTAs of 64 rows fit beside each other (up to 64 functions in FP64, 96 in
-// FP32); larger ones read it chunk by chunk.
-template <typename T>
-static bool simt_resident(int npad) {
-  return simt_cpt(npad) <= 8 && npad <= 128 && simt_smem<T, 64>(npad, true) <= 72u * 1024u;
-}
+// P stays in shared memory for the narrowest panel, up to 64 functions (three CTAs of 64 rows and 66 KB fit beside
+// each other in FP64); larger ones read it chunk by chunk.
+static bool simt_resident(int npad) { return simt_cpt(npad) == 4; }
 
 template <typename T, int TP, int CPT, bool RES>
 static qmt_status launch_simt_as(qmt_mol* mol, const PointMap& pm, int64_t ntiles, float* qube, double* partials,
@@ -233,14 +230,9 @@ static qmt_status launch_simt_as(qmt_mol* mol, const PointMap& pm, int64_t ntile
 template <typename T, int TP>
 static qmt_status launch_simt(qmt_mol* mol, const PointMap& pm, int64_t ntiles, float* qube,
                               double* partials, double outscale, cudaStream_t s) {
-  const bool res = simt_resident<T>(mol->npad);
   switch (simt_cpt(mol->npad)) {
-    case 4:
-      return res ? launch_simt_as<T, TP, 4, true>(mol, pm, ntiles, qube, partials, outscale, s)
-                 : launch_simt_as<T, TP, 4, false>(mol, pm, ntiles, qube, partials, outscale, s);
-    case 8:
-      return res ? launch_simt_as<T, TP, 8, true>(mol, pm, ntiles, qube, partials, outscale, s)
-                 : launch_simt_as<T, TP, 8, false>(mol, pm, ntiles, qube, partials, outscale, s);
+    case 4: return launch_simt_as<T, TP, 4, true>(mol, pm, ntiles, qube, partials, outscale, s);
+    case 8: return launch_simt_as<T, TP, 8, false>(mol, pm, ntiles, qube, partials, outscale, s);
     case 10: return launch_simt_as<T, TP, 10, false>(mol, pm, ntiles, qube, partials, outscale, s);
     case 12: return launch_simt_as<T, TP, 12, false>(mol, pm, ntiles, qube, partials, outscale, s);
     case 14: return launch_simt_as<T, TP, 14, false>(mol, pm, ntiles, qube, partials, outscale, s);
@@ -263,13 +255,13 @@ static int max_smem() {
 static int simt_tile_rows(bool fp64, int npad, int s3) {
   const size_t lim = (size_t)max_smem() - 4096;
   if (!fp64) {
-    if (simt_smem<float, 64>(npad, simt_resident<float>(npad)) <= lim) return 64;
-    if (s3 <= 32 && simt_smem<float, 32>(npad, simt_resident<float>(npad)) <= lim) return 32;
-    if (s3 <= 16 && simt_smem<float, 16>(npad, simt_resident<float>(npad)) <= lim) return 16;
+    if (simt_smem<float, 64>(npad, simt_resident(npad)) <= lim) return 64;
+    if (s3 <= 32 && simt_smem<float, 32>(npad, simt_resident(npad)) <= lim) return 32;
+    if (s3 <= 16 && simt_smem<float, 16>(npad, simt_resident(npad)) <= lim) return 16;
   } else {
-    if (simt_smem<double, 64>(npad, simt_resident<double>(npad)) <= lim) return 64;
-    if (s3 <= 32 && simt_smem<double, 32>(npad, simt_resident<double>(npad)) <= lim) return 32;
-    if (s3 <= 16 && simt_smem<double, 16>(npad, simt_resident<double>(npad)) <= lim) return 16;
+    if (simt_smem<double, 64>(npad, simt_resident(npad)) <= lim) return 64;
+    if (s3 <= 32 && simt_smem<double, 32>(npad, simt_resident(npad)) <= lim) return 32;
+    if (s3 <= 16 && simt_smem<double, 16>(npad, simt_resident(npad)) <= lim) return 16;
   }
   return 0;
 }
