@@ -132,16 +132,6 @@ __device__ __forceinline__ const FactMol& fact_mol(const FactParams& p, int64_t 
   return p.mols[lo];
 }
 
-__device__ __forceinline__ uint64_t sw32_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)1u << 16;             // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(256u >> 4) << 32;    // stride byte offset: 8 rows x 32 B
-  d |= (uint64_t)1u << 46;             // descriptor version for sm_100
-  d |= (uint64_t)6u << 61;             // 32-byte swizzle
-  return d;
-}
-
 // ---- packed FP32 pairs (rows r and r + 64 of an item): one issue slot for both rows -------------
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 pk(float a, float b) {
@@ -496,11 +486,11 @@ __device__ __forceinline__ void issue_mma(const FactParams& p, FactBars& B, uint
 #pragma unroll
       for (int k = 0; k < GROUP; ++k) {
         if (u0 + k < nunits) {
-          const uint64_t ahi = sw32_desc(a), bhi = sw32_desc(b);
+          const uint64_t ahi = sw32_kmajor_desc(a), bhi = sw32_kmajor_desc(b);
           if (MAIN) {
             if (leader) mma_f16(d0 + ha * r16, ahi, bhi, idesc, acc);
           } else {
-            const uint64_t alo = sw32_desc(a + PIECE), blo = sw32_desc(b + half);
+            const uint64_t alo = sw32_kmajor_desc(a + PIECE), blo = sw32_kmajor_desc(b + half);
             if (leader) {
               mma_f16(S, ahi, blo, idesc, acc);
               mma_f16(S, alo, bhi, idesc, 1u);
@@ -974,25 +964,6 @@ struct PivotArgs {
   volatile unsigned long long* mail;
 };
 constexpr unsigned kMailPending = 1u << 30;   // there is a rank, the check is to come
-
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ double cluster_load_f64(const double* p, uint32_t rank) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
-  return v;
-}
 
 struct PivotCand {
   double d;

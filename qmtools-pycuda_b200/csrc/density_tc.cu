@@ -548,7 +548,6 @@ struct FusedMol {
   int natoms, norbs;
   int n16;                 // functions rounded up to 16: K of the MMAs; the K-steps beyond it
                            // only hold zero padding and are skipped
-  int nb;                  // N of the MMAs (rows of a K-step block of U): n16
   int ksteps, nchunks;     // n16 / 16 K-steps; ceil(n16 / 64) column chunks of A
   int tail0;               // n16 & ~63: first column of A's 32-byte swizzled tail blocks
   int u_rows;              // rows of one K-step block of U in HBM (kpad + 64)
@@ -621,16 +620,6 @@ __device__ __forceinline__ uint32_t a_offset(int row, int j, int tail0) {
                     (e & 7) * 2);
 }
 __device__ __forceinline__ uint32_t a_row64(int j, int tail0) { return j < tail0 ? 8192u : 2048u; }
-
-__device__ __forceinline__ uint64_t sw32_kmajor_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)1u << 16;             // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(256u >> 4) << 32;    // stride byte offset: 8 rows x 32 B
-  d |= (uint64_t)1u << 46;             // descriptor version for sm_100
-  d |= (uint64_t)6u << 61;             // 32-byte swizzle
-  return d;
-}
 
 template <int FMT>
 __device__ __forceinline__ void store_split16(uint8_t* hi, uint8_t* lo, uint32_t off, float x, bool two) {
@@ -1209,7 +1198,7 @@ __device__ __forceinline__ void fused_produce_u(const FusedParams* pp, uint8_t* 
     // the molecule's values in registers for the tile: read through a reference, they would be
     // reloaded after every barrier operation (each an asm statement that clobbers memory)
     const int ksteps = M.ksteps, u_rows = M.u_rows;
-    const uint32_t bytes = (uint32_t)M.nb * 32u;
+    const uint32_t bytes = (uint32_t)M.n16 * 32u;
     const uint8_t* const u_hi = M.u_hi;
     const uint8_t* const u_lo = M.u_lo;
     for (int ks = 0; ks < ksteps; ++ks, ++it) {
@@ -1249,7 +1238,7 @@ __device__ __forceinline__ void fused_issue_mma(const FusedParams* pp, uint32_t 
     int m;
     const FusedMol& M = fused_mol<MULTI>(p, t, m);
     // the molecule's values in registers for the tile (see the producer)
-    const int ksteps = M.ksteps, nb = M.nb, tail0 = M.tail0;
+    const int ksteps = M.ksteps, n16 = M.n16, tail0 = M.tail0;
     uint32_t need = 0;
 #pragma unroll
     for (int c = 0; c < MAX_FUSED_CHUNKS; ++c)
@@ -1285,8 +1274,8 @@ __device__ __forceinline__ void fused_issue_mma(const FusedParams* pp, uint32_t 
         alo = sw32_kmajor_desc(lbase + aoff);
       }
       const uint32_t bst = smem_u32(stages + (size_t)s * p.stage_bytes);
-      for (int c0 = 0; c0 < nb; c0 += 256) {
-        const int n = min(256, nb - c0);
+      for (int c0 = 0; c0 < n16; c0 += 256) {
+        const int n = min(256, n16 - c0);
         const uint32_t idesc = make_idesc(p.fmt, 128, (uint32_t)n);
         const uint32_t boff = (uint32_t)c0 * 32u;
         const uint32_t d = tmem + (uint32_t)c0;
@@ -1654,20 +1643,20 @@ static int fused_tab_bytes(const qmt_mol* m) {
 // and of one U piece slot in a stage.
 static int fused_n16(const qmt_mol* m) { return (m->norbs + 15) / 16 * 16; }
 static uint32_t fused_a_bytes(int n16) { return 128u * (uint32_t)n16 * 2u; }
-static uint32_t fused_b_slot(int nb) { return (uint32_t)nb * 32u; }
+static uint32_t fused_b_slot(int n16) { return (uint32_t)n16 * 32u; }
 
 // U pipeline stages that fit beside A and the tables (below 2: the fused path does not fit).
-// Bytes of one stage: a K-step of U (nb rows per piece).
-static long fused_stage_bytes(const TcShape& sh, int nb) { return (long)sh.nsplit * fused_b_slot(nb); }
+// Bytes of one stage: a K-step of U (n16 rows per piece).
+static long fused_stage_bytes(const TcShape& sh, int n16) { return (long)sh.nsplit * fused_b_slot(n16); }
 
 template <int FMT>
-static int fused_stages(const TcShape& sh, int n16, int nb, int tab_bytes) {
+static int fused_stages(const TcShape& sh, int n16, int tab_bytes) {
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaFuncAttributes fa;
   if (cudaFuncGetAttributes(&fa, density_fused_kernel<FMT, true>) != cudaSuccess) return 0;
-  const long a_bytes = fused_a_bytes(n16), stage_bytes = fused_stage_bytes(sh, nb);
+  const long a_bytes = fused_a_bytes(n16), stage_bytes = fused_stage_bytes(sh, n16);
   const long avail = (long)maxsm - (long)fa.sharedSizeBytes - 1024 - sh.nsplit * a_bytes - tab_bytes;
   return (int)std::max<long>(0, std::min<long>(MAX_STAGES, avail / stage_bytes));
 }
@@ -1688,7 +1677,6 @@ static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& 
   d.ksteps = n16 / 16;
   d.nchunks = (n16 + 63) / 64;
   d.tail0 = n16 & ~63;
-  d.nb = n16;
   d.u_rows = K + 64;
   d.u_hi = B;
   d.u_lo = B + piece;
@@ -1718,16 +1706,16 @@ static qmt_status fused_mol_desc(qmt_mol* m, const TcShape& sh, const PointMap& 
 // One persistent launch over every tile of the molecules in `p` (p.one, or the device array
 // p.mols); shared memory is sized for the largest operand, stage and table of the set.
 template <int FMT>
-static qmt_status launch_fused(FusedParams& p, const TcShape& sh_max, int n16_max, int nb_max, int tab_bytes_max,
+static qmt_status launch_fused(FusedParams& p, const TcShape& sh_max, int n16_max, int tab_bytes_max,
                                cudaStream_t s) {
   p.nsplit = sh_max.nsplit;
   p.a_bytes = fused_a_bytes(n16_max);
-  p.b_slot = fused_b_slot(nb_max);
-  p.stage_bytes = (uint32_t)fused_stage_bytes(sh_max, nb_max);
+  p.b_slot = fused_b_slot(n16_max);
+  p.stage_bytes = (uint32_t)fused_stage_bytes(sh_max, n16_max);
   p.fmt = (uint32_t)sh_max.fmt;
   p.wait_ns = wait_limit_ns();
   auto kern = p.nmol > 1 ? density_fused_kernel<FMT, true> : density_fused_kernel<FMT, false>;
-  const int stages = fused_stages<FMT>(sh_max, n16_max, nb_max, tab_bytes_max);
+  const int stages = fused_stages<FMT>(sh_max, n16_max, tab_bytes_max);
   if (stages < 2) return fail(QMT_BAD_ARG, "fused density tile does not fit in shared memory");
   p.stages = stages;
   const size_t dyn = (size_t)p.nsplit * p.a_bytes + (size_t)stages * p.stage_bytes + tab_bytes_max + 1024;
@@ -1751,7 +1739,7 @@ static qmt_status run_fused(qmt_mol* m, const TcShape& sh, const PointMap& pm, i
   p.nmol = 1;
   p.ntiles = ntiles;
   p.err = reinterpret_cast<int*>(m->d_scalars.as<double>() + 8);
-  return launch_fused<FMT>(p, sh, p.one.n16, p.one.nb, tab_bytes, s);
+  return launch_fused<FMT>(p, sh, p.one.n16, tab_bytes, s);
 }
 
 // Builds the scaled, split density matrix and the Phi column scales for `prec`.
@@ -1918,7 +1906,7 @@ static bool fused_fits(const qmt_mol* mol, const TcShape& sh) {
   if (sh.fmt == FMT_TF32 || sh.kpad > 320 || 2 * mol->natoms >= (int)CHUNK_COUNT) return false;
   const int tb = fused_tab_bytes(mol);
   const int n16 = fused_n16(mol);
-  return (sh.fmt == FMT_F16 ? fused_stages<FMT_F16>(sh, n16, n16, tb) : fused_stages<FMT_BF16>(sh, n16, n16, tb)) >= 2;
+  return (sh.fmt == FMT_F16 ? fused_stages<FMT_F16>(sh, n16, tb) : fused_stages<FMT_BF16>(sh, n16, tb)) >= 2;
 }
 
 qmt_status density_tc(qmt_mol* mol, int nx, int ny, int nz, float step, float ox, float oy, float oz,
@@ -2027,7 +2015,7 @@ struct BatchItem {
 struct qmt_batch_group {
   std::vector<qmt::FusedMol> fdesc;
   qmt::TcShape sh_max{};
-  int n16_max = 0, nb_max = 0, tab_bytes_max = 0;
+  int n16_max = 0, tab_bytes_max = 0;
   int64_t tiles = 0;
   qmt::DevBuf d_fdesc;
 };
@@ -2065,7 +2053,7 @@ static qmt_status batch_operands(const BatchItem& it, int prec, bool refresh, cu
 static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, int& stages, int& largest) {
   g.fdesc.clear();
   g.sh_max = TcShape{};
-  g.n16_max = g.nb_max = g.tab_bytes_max = 0;
+  g.n16_max = g.tab_bytes_max = 0;
   g.tiles = 0;
   largest = -1;
   stages = MAX_STAGES;
@@ -2080,14 +2068,13 @@ static qmt_status batch_group(qmt_batch* b, qmt_batch_group& g, int& stages, int
     g.fdesc.push_back(d);
     if (it.sh.kpad > g.sh_max.kpad) g.sh_max = it.sh;
     g.n16_max = std::max(g.n16_max, d.n16);
-    g.nb_max = std::max(g.nb_max, d.nb);
     g.tab_bytes_max = std::max(g.tab_bytes_max, tb);
     if (largest < 0 || it.sh.kpad + tb / 1024 > b->items[largest].sh.kpad + fused_tab_bytes(b->items[largest].mol) / 1024)
       largest = (int)i;
   }
   if (!g.fdesc.empty())
-    stages = b->fmt == FMT_F16 ? fused_stages<FMT_F16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max)
-                               : fused_stages<FMT_BF16>(g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max);
+    stages = b->fmt == FMT_F16 ? fused_stages<FMT_F16>(g.sh_max, g.n16_max, g.tab_bytes_max)
+                               : fused_stages<FMT_BF16>(g.sh_max, g.n16_max, g.tab_bytes_max);
   return QMT_OK;
 }
 
@@ -2100,7 +2087,7 @@ static qmt_status batch_launch(qmt_batch* b, const qmt_batch_group& g, cudaStrea
   p.mols = g.d_fdesc.as<FusedMol>();
   p.ntiles = g.tiles;
   p.err = b->d_err.as<int>();
-  return launch_fused<FMT>(p, g.sh_max, g.n16_max, g.nb_max, g.tab_bytes_max, s);
+  return launch_fused<FMT>(p, g.sh_max, g.n16_max, g.tab_bytes_max, s);
 }
 
 template <int FMT>

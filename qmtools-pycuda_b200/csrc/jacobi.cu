@@ -24,6 +24,7 @@
 #include "mol.cuh"
 #include "persistent.cuh"
 #include "reduce.cuh"
+#include "sm100.cuh"
 
 namespace qmt {
 
@@ -395,38 +396,6 @@ __global__ void __launch_bounds__(JAC_PLANE_THREADS, 1) jacobi_plane_kernel(Jaco
 constexpr int JAC_CLUSTER = 16;          // CTAs of the cluster (a non-portable size)
 constexpr int JAC_CLUSTER_THREADS = 1024;
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-// Address of the same shared-memory location in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t dsmem_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ float4 dsmem_ld4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
-}
-
-__device__ __forceinline__ double dsmem_ld_f64(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
-  return v;
-}
-
 // One cluster; CTA c owns planes [c P, c P + np) of the grid.  Thread t owns the four-point group
 // (xq, y) = (t % nxq, t / nxq) of every plane of the slab.  Shared memory: buf[2][P][ny][nxq]
 // float4 (the field before / after a sweep).  Launched only when nx % 4 == 0, nxq * ny <= 1024,
@@ -441,7 +410,7 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
   const int t = threadIdx.x, lane = t & 31;
   const bool act = t < nxq * ny;
   const int xq = act ? t % nxq : 0, y = act ? t / nxq : 0;
-  const uint32_t c = cluster_rank(), ncta = gridDim.x;
+  const uint32_t c = sm100::cluster_cta_rank(), ncta = gridDim.x;
   const int z0 = (int)c * P;
   const int np = max(0, min(P, nz - z0));
   const int pstride = nxq * ny;                 // float4 per plane
@@ -466,7 +435,7 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
   // shuffles give the x neighbours within a warp; at a warp's first / last lane the group beside
   // it (same row) belongs to another warp and is read from shared memory
   const bool left_smem = !xlo && lane == 0, right_smem = !xhi && lane == 31;
-  cluster_sync_all();
+  sm100::cluster_barrier();
   int sweeps = 0, pairs = 0, status = 0;
   double delta = INFINITY;
   while (sweeps + 2 <= a.max_sweeps) {
@@ -481,8 +450,8 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
       const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
       float4 below = zero, above = zero;
       if (act && np > 0) {
-        if (z0 > 0) below = dsmem_ld4(dsmem_addr(src + (P - 1) * pstride + own, c - 1));
-        if (z0 + np < nz) above = dsmem_ld4(dsmem_addr(src + own, c + 1));
+        if (z0 > 0) below = sm100::cluster_load_f4(src + (P - 1) * pstride + own, c - 1);
+        if (z0 + np < nz) above = sm100::cluster_load_f4(src + own, c + 1);
       }
       float4 prev = below;
 #pragma unroll
@@ -513,7 +482,7 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
           dst[k * pstride + own] = o;
         }
       }
-      cluster_sync_all();   // every read of src done, every write of dst visible cluster-wide
+      sm100::cluster_barrier();   // every read of src done, every write of dst visible cluster-wide
       if (resid) {
         // FP64 residual: warp tree, warps in order, CTAs in rank order -- every CTA adds the same
         // partials in the same order, so all take the same decision
@@ -525,10 +494,10 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
           for (int w = 0; w < JAC_CLUSTER_THREADS / 32; ++w) r += red[w];
           part = r;
         }
-        cluster_sync_all();
+        sm100::cluster_barrier();
         if (t == 0) {
           double r = 0.0;
-          for (uint32_t b = 0; b < ncta; ++b) r += dsmem_ld_f64(dsmem_addr(&part, b));
+          for (uint32_t b = 0; b < ncta; ++b) r += sm100::cluster_load_f64(&part, b);
           delta = r;
           stop_s = !isfinite(r) ? 2 : (r <= a.tol ? 1 : 0);
         }
@@ -542,7 +511,7 @@ __global__ void __launch_bounds__(JAC_CLUSTER_THREADS, 1) jacobi_cluster_kernel(
     }
   }
   // no CTA may leave while another can still read its shared memory
-  cluster_sync_all();
+  sm100::cluster_barrier();
 #pragma unroll
   for (int k = 0; k < P; ++k)
     if (act && k < np)

@@ -133,6 +133,35 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   }
 }
 
+// ---- thread-block clusters -----------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address of the same shared-memory location in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ double cluster_load_f64(const double* p, uint32_t rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 cluster_load_f4(const float4* p, uint32_t rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(cluster_addr(p, rank))
+               : "memory");
+  return v;
+}
+
 // One lane of a converged warp (always the same one).
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
@@ -288,6 +317,16 @@ __device__ __forceinline__ uint64_t sw128_kmajor_desc(uint32_t saddr) {
   d |= (uint64_t)(1024u >> 4) << 32;    // stride byte offset
   d |= (uint64_t)1u << 46;              // descriptor version for sm_100
   d |= (uint64_t)2u << 61;              // 128-byte swizzle
+  return d;
+}
+
+__device__ __forceinline__ uint64_t sw32_kmajor_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1u << 16;             // leading byte offset (unused for swizzled K-major)
+  d |= (uint64_t)(256u >> 4) << 32;    // stride byte offset: 8 rows x 32 B
+  d |= (uint64_t)1u << 46;             // descriptor version for sm_100
+  d |= (uint64_t)6u << 61;             // 32-byte swizzle
   return d;
 }
 
