@@ -959,6 +959,8 @@ struct PivotArgs {
   int ld0;                    // (at least rmax rounded up to 16)
   int* info;
   double* dmax;               // the first pivot
+  unsigned long long* zero;   // nzero words that the kernel clears first: column maxima, info, dmax, the check's flag
+  int nzero;
   int* usable;                // as fact_split_kernel leaves them, here where there is no factor; else the word's
   uint32_t number;            // kMailPending
   volatile unsigned long long* mail;
@@ -993,6 +995,8 @@ __global__ void __launch_bounds__(PIV_THREADS, 1) fact_pivot_kernel(PivotArgs a)
   double* lj = d + a.rows;                      // the pivot's row of L
   double* own = a.rows_in_smem ? lj + a.rmax : a.L + (size_t)r0 * a.rmax;
   const int ld = a.rows_in_smem ? a.ld : a.rmax;
+  if (c == 0)   // (info is written behind a barrier, the rest by later kernels)
+    for (int i = t; i < a.nzero; i += PIV_THREADS) a.zero[i] = 0ull;
   const PivotCand none{0.0, 0x7fffffff, 0u};
   PivotCand best = none;                        // of this thread's rows (lanes with sub == 0)
   for (int i = t >> 3; i < nr; i += PIV_THREADS / 8)
@@ -1264,11 +1268,9 @@ __global__ void __launch_bounds__(32 * SOLVE_WARPS) fact_solve_kernel(double* __
 }
 
 // Column scales: 2^h_q brings the column's largest scaled element near 2^14 (h in [-100, 100]); then
-// 2^-h_q in FP32 for the squares (0 for the padding columns).
-__global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax, const int* __restrict__ rank,
-                                  double* __restrict__ two_h, float* __restrict__ hscale) {
-  const int q = threadIdx.x, r = *rank;
-  if (r == 0 || q >= ceil16(r)) return;
+// 2^-h_q in FP32 for the squares (0 for the padding columns).  Thread q of one block, q < r16.
+__device__ __forceinline__ void column_scale(const unsigned long long* __restrict__ colmax, int q, int r,
+                                             double* __restrict__ two_h, float* __restrict__ hscale) {
   const double mx = __longlong_as_double((long long)colmax[q]);
   int h = mx > 0 ? (int)floor(log2(16000.0 / mx)) : 0;
   h = max(-100, min(100, h));
@@ -1277,15 +1279,18 @@ __global__ void fact_scale_kernel(const unsigned long long* __restrict__ colmax,
 }
 
 // Raises *bad when some |P_ij - sum_q L_iq L_jq| (i >= j) exceeds rel * dmax; L row i at L[i * r16].  One block per
-// 32 x 32 tile on or below the diagonal.
+// 32 x 32 tile on or below the diagonal.  The first block also forms the column scales.
 __global__ void __launch_bounds__(256) fact_residual_kernel(const double* __restrict__ P, int np,
                                                             const double* __restrict__ L, int n,
                                                             const int* __restrict__ rank, double rel,
-                                                            const double* __restrict__ dmax, int* bad) {
+                                                            const double* __restrict__ dmax, int* bad,
+                                                            const unsigned long long* __restrict__ colmax,
+                                                            double* __restrict__ two_h, float* __restrict__ hscale) {
   __shared__ double li[32][33], lj[32][33];
   const int r = *rank, ld = ceil16(r);
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   if (r == 0 || j0 > i0) return;
+  if (i0 == 0 && (int)threadIdx.x < ld) column_scale(colmax, threadIdx.x, r, two_h, hscale);
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int q0 = 0; q0 < r; q0 += 32) {
 #pragma unroll
@@ -1369,7 +1374,7 @@ constexpr double kFactorResid = 2e-7;
 }  // namespace
 
 static qmt_status launch_pivot(qmt_mol* m, int rmax, int limit, double* L, float* L0, int ld0, int* info, double* dmax,
-                               cudaStream_t s) {
+                               unsigned long long* zero, int nzero, cudaStream_t s) {
   const int n = m->norbs;
   int maxsm = 0, dev = 0;
   cudaGetDevice(&dev);
@@ -1390,6 +1395,8 @@ static qmt_status launch_pivot(qmt_mol* m, int rmax, int limit, double* L, float
     a.ld0 = ld0;
     a.info = info;
     a.dmax = dmax;
+    a.zero = zero;
+    a.nzero = nzero;
     a.usable = m->fact_usable();
     a.number = m->fact_number;
     a.mail = m->fact_mail;
@@ -1411,7 +1418,8 @@ static qmt_status launch_pivot(qmt_mol* m, int rmax, int limit, double* L, float
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, fact_pivot_kernel, &cfg) != cudaSuccess || nclusters < 1) {
+    if (ncta > 1 &&
+        (cudaOccupancyMaxActiveClusters(&nclusters, fact_pivot_kernel, &cfg) != cudaSuccess || nclusters < 1)) {
       cudaGetLastError();   // a smaller cluster
       continue;
     }
@@ -1519,9 +1527,8 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   double* two_h = m->d_fact_scale.as<double>();
   const double* P = m->d_P64.as<double>();
   const int r16max = (rmax + 15) / 16 * 16;   // <= rbuf
-  QMT_CUDA(cudaMemsetAsync(colmax, 0, (rbuf + 8) * sizeof(double), s));
   if (++m->fact_number == 0) m->fact_number = 1;
-  if ((st = launch_pivot(m, rmax, limit, Lp, L0, rbuf, info, dmax, s))) return st;
+  if ((st = launch_pivot(m, rmax, limit, Lp, L0, rbuf, info, dmax, colmax, rbuf + 8, s))) return st;
   if (wait) {   // the pivots alone may refuse the matrix, and the rest need not run
     unsigned word = 0;
     if ((st = read_mail(m, kMailPending, &word, s))) return st;
@@ -1547,9 +1554,8 @@ qmt_status ensure_factor(qmt_mol* m, int prec, int fmt, int nsplit, int kpad, bo
   fact_solve_kernel<<<(n + SOLVE_WARPS - 1) / SOLVE_WARPS, 32 * SOLVE_WARPS, ssm, s>>>(
       Y, CT, n, info, m->d_split_scale.as<double>(), colmax);
   QMT_CHECK_LAUNCH("fact_solve_kernel");
-  fact_scale_kernel<<<1, kFactorMaxR16, 0, s>>>(colmax, info, two_h, reinterpret_cast<float*>(two_h + kFactorMaxR16));
-  QMT_CHECK_LAUNCH("fact_scale_kernel");
-  fact_residual_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), 256, 0, s>>>(P, np, Y, n, info, kFactorResid, dmax, bad);
+  fact_residual_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), 256, 0, s>>>(
+      P, np, Y, n, info, kFactorResid, dmax, bad, colmax, two_h, reinterpret_cast<float*>(two_h + kFactorMaxR16));
   QMT_CHECK_LAUNCH("fact_residual_kernel");
   const int64_t tot = (int64_t)m->fact_units * 16 * r16max;
   const int blocks = (int)std::min<int64_t>((tot + 255) / 256, (int64_t)sm_count() * 4);
