@@ -1129,7 +1129,7 @@ def run_reference(args, world, rank, local, pg):
     cb = dict(samples[0])
     cb["value"] = v
     return {"metric": METRIC, "value": v, "unit": UNIT, "n_gpus": world, "steps": args.steps,
-            "warmup": 0, "ms_per_step": 1000.0 * (128 ** 3) / v, "higher_is_better": True,
+            "warmup": args.warmup, "ms_per_step": 1000.0 * (128 ** 3) / v, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "fp64", "data": "synthetic", "impl": "reference",
             "config": {"workload": WORKLOAD},
             "cpu_baseline": cb, "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},

@@ -2035,7 +2035,7 @@ struct qmt_batch {
 namespace qmt {
 
 // Re-derives (refresh) or checks the molecule's contraction operands for its path (a factored
-// molecule's factor comes from the host matrix at batch creation and is not re-derived).
+// molecule's factor is built and read back at batch creation and is not re-derived).
 static qmt_status batch_operands(const BatchItem& it, int prec, bool refresh, cudaStream_t s) {
   if (it.fact) {
     if (refresh) return fail(QMT_BAD_ARG, "a batch with factored molecules cannot re-derive their operands");

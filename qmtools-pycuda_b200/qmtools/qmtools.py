@@ -256,7 +256,7 @@ class Grid:
         if not numpy.array_equal(grd, blk * 8):
             raise ValueError("shape for xyz have to be multiple of 8")
         self.GPUblocks = tuple([x.item() for x in blk])
-        self.qube = numpy.zeros(self.shape, dtype=numpy.float32)   # (pages are touched only when used)
+        self.qube = numpy.zeros(self.shape, dtype=numpy.float32)
         self.npts = numpy.uint32(self.shape[1] * self.shape[2] * self.shape[3])
         self.nfields = numpy.uint32(self.shape[0])
         self.step = numpy.float32(step * ANG2BOR)
@@ -416,8 +416,9 @@ class Grid:
 def _new_like(g, nfields=None, written=False):
     """A grid like `g` with device storage, zero unless its one field is about to be `written` whole.
 
-    The storage is made on the device and the host array's pages stay untouched: making zeros on the host
-    and uploading them took 3.5 ms for 192^3 points."""
+    The storage is made on the device: making zeros on the host, converting them and uploading them took
+    3.5 ms for 192^3 points.  (The host array's own zeros are left: up to 0.8 ms of that size, where malloc
+    hands out a block that it has to clear.)"""
     out = Grid.emptyAs(g, nfields)
     N.ensure_device()
     new = _torch().empty if written and out.shape[0] == 1 else _torch().zeros

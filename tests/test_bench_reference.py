@@ -10,5 +10,5 @@ def test_cpu_port_arm(monkeypatch):
     monkeypatch.setattr(bench, "_ref_libs", lambda: None)
     monkeypatch.setattr(bench, "cpu_baseline_c1", lambda *a: ({"value": next(values), "kind": "port"}, None))
     out = bench.run_reference(argparse.Namespace(steps=3, warmup=2), 1, 0, 0, None)
-    assert out["value"] == 4.0 and out["impl"] == "reference"      # the median of the timed ones: 3, 4, 5
+    assert out["warmup"] == 2 and out["value"] == 4.0 and out["impl"] == "reference"      # the median of the timed ones: 3, 4, 5
     assert out["cpu_baseline"] == {"value": 4.0, "kind": "port"}
