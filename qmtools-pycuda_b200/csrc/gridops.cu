@@ -521,9 +521,9 @@ qmt_status qmt_vne_pseudo(qmt_mol* mol, int nx, int ny, int nz, float step, floa
       1, std::min<int64_t>((items + VNE_THREADS - 1) / VNE_THREADS, (int64_t)sm_count() * std::min(per_sm, 4)));
   // workspace: status and barrier words, two sets of CTA partials, the source term
   const size_t part_bytes = ((size_t)2 * grid * sizeof(double) + 255) / 256 * 256;
-  qmt_status st = mol->d_work.reserve(256 + part_bytes + (size_t)n * sizeof(float));
+  qmt_status st = mol->d_vne.reserve(256 + part_bytes + (size_t)n * sizeof(float));
   if (st) return st;
-  uint8_t* w = mol->d_work.as<uint8_t>();
+  uint8_t* w = mol->d_vne.as<uint8_t>();
   VneArgs a{};
   a.nx = nx;
   a.ny = ny;

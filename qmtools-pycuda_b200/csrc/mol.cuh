@@ -71,6 +71,7 @@ struct qmt_mol {
   qmt::DevBuf d_Phi_hi, d_Phi_lo;
   // scratch
   qmt::DevBuf d_partials, d_scalars, d_work;
+  qmt::DevBuf d_vne;            // pseudo-field (d_work, which a captured FFT solve reads, must not grow for it)
   // analytic potential: primitive-pair table (FP64), and the FP32 kernels' tables (gto.cu)
   bool gto_ready = false;
   int gto_npairs = 0;
